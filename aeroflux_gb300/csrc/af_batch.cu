@@ -99,9 +99,9 @@ struct InstDev {
     double* b;         // h^2 * Div, P-shaped
     float dt_invh;     // (DT/2)/H for the sweeps
     float lam;         // nu*(DT/2)/H^2
-    double div_scale;  // rho/(DT*H)
-    double h2;
-    double grad_scale;  // DT/(rho*H)
+    exact::MulC div_scale;   // rho/(DT*H)
+    exact::MulC h2;          // H^2
+    exact::MulC grad_scale;  // DT/(rho*H)
     double res_scale;   // DT/(rho*H^2): max|div| per unit residual
     double thresh;      // 0.5 * div_tol
     unsigned max_refine;
@@ -2801,9 +2801,9 @@ int batch_assign(Batch* b, const af_config& c, char* arena, std::string* err) {
     const double invH = 1.0 / c.h;
     I.dt_invh = (float)(half * invH);
     I.lam = (float)(c.viscosity * half * invH * invH);  // stencil.go:73
-    I.div_scale = c.density / (c.dt * c.h);             // project.go:49
-    I.h2 = c.h * c.h;                                   // project.go:107
-    I.grad_scale = c.dt / (c.density * c.h);            // project.go:179
+    I.div_scale = exact::mul_const(c.density / (c.dt * c.h));   // project.go:49
+    I.h2 = exact::mul_const(c.h * c.h);                         // project.go:107
+    I.grad_scale = exact::mul_const(c.dt / (c.density * c.h));  // project.go:179
     I.res_scale = c.dt / (c.density * c.h * c.h);
     I.thresh = 0.5 * c.div_tol;
     I.max_refine = (unsigned)c.max_refine;

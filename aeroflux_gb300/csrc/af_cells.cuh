@@ -4,6 +4,7 @@
 #pragma once
 
 #include "af_debug.cuh"
+#include "af_exact.cuh"
 #include "af_internal.h"
 
 #include <math.h>
@@ -26,7 +27,7 @@ __device__ __forceinline__ double flip(double a) {
 // GB300's FP64 pipe (about two operations per SM per clock) also executes
 // binary64 compares and conversions; the sweeps move the exact ones here.
 constexpr unsigned long long kFrac = 0xFFFFFFFFFFFFFull;
-__device__ __forceinline__ unsigned long long dbits(double x) { return (unsigned long long)__double_as_longlong(x); }
+__device__ __forceinline__ unsigned long long dbits(double x) { return exact::bits_of(x); }
 __device__ __forceinline__ double dfrom(unsigned long long b) { return __longlong_as_double((long long)b); }
 
 // (double)n for 0 <= n < 2^31.
@@ -60,7 +61,7 @@ __device__ __forceinline__ double frac_sub(double x, long long a0) {
     return dfrom(((unsigned long long)(1023 + e - 52 + p) << 52) | ((f << (52 - p)) & kFrac));
 }
 
-// RN(0.25 * x) and RN(2 * x): exact exponent shifts while the result stays
+// RN(0.25 * x), RN(2 * x) and RN(0.5 * x): exact exponent shifts while the result stays
 // normal (and for 0, Inf, NaN, which pass through); the FP64 multiply
 // otherwise, so every input rounds as the multiply would.
 __device__ __forceinline__ double quarter(double x) {
@@ -68,14 +69,21 @@ __device__ __forceinline__ double quarter(double x) {
     const unsigned e = (unsigned)((b >> 52) & 0x7FF);
     if (e >= 3u && e < 0x7FFu) return dfrom(b - (2ull << 52));
     if (e == 0x7FFu || (b & ~kSign) == 0ull) return x;
-    return dmul(0.25, x);
+    return exact::mul_native(0.25, x);
 }
 __device__ __forceinline__ double twice(double x) {
     const unsigned long long b = dbits(x);
     const unsigned e = (unsigned)((b >> 52) & 0x7FF);
     if (e >= 1u && e < 0x7FEu) return dfrom(b + (1ull << 52));
     if (e == 0x7FFu || (b & ~kSign) == 0ull) return x;
-    return dmul(2.0, x);
+    return exact::mul_native(2.0, x);
+}
+__device__ __forceinline__ double half(double x) {
+    const unsigned long long b = dbits(x);
+    const unsigned e = (unsigned)((b >> 52) & 0x7FF);
+    if (e >= 2u && e < 0x7FFu) return dfrom(b - (1ull << 52));
+    if (e == 0x7FFu || (b & ~kSign) == 0ull) return x;
+    return exact::mul_native(0.5, x);
 }
 
 // Correctly rounded x/6.  Because 6 = 3*2, x/6 is never within ulp/6 of a
@@ -317,11 +325,14 @@ __device__ __forceinline__ void pbc_cell(const Geom& g, AF_PTR(double) p, int se
 }
 
 // --- computeDivergence (project.go:42-62) + P zeroing + B = h2*Div ---------
-// (x, y, z) is any cell of the padded P extent.
+// (x, y, z) is any cell of the padded P extent.  The two products are integer
+// instructions (af_exact.cuh): the five additions left bound the kernel
+// (256^3, per launch: 260 us with the products on the binary64 pipe, 189 so).
 __device__ __forceinline__ void div_cell(const Geom& g, AF_PTR(const double) AF_RESTRICT u,
                                          AF_PTR(const double) AF_RESTRICT v, AF_PTR(const double) AF_RESTRICT w,
                                          AF_PTR(double) AF_RESTRICT p, AF_PTR(double) AF_RESTRICT dv,
-                                         AF_PTR(double) AF_RESTRICT bb, double scale, double h2, bool zero_p, int x,
+                                         AF_PTR(double) AF_RESTRICT bb, const exact::MulC& scale,
+                                         const exact::MulC& h2, bool zero_p, int x,
                                          int y, int z) {
     const long long i = x + y * g.p.sy + z * g.p.sz;
     if (zero_p) p[i] = 0.0;
@@ -333,9 +344,9 @@ __device__ __forceinline__ void div_cell(const Geom& g, AF_PTR(const double) AF_
     const double du = dsub(u[iu + 1], u[iu]);
     const double dvv = dsub(v[iv + g.v.sy], v[iv]);
     const double dw = dsub(w[iw + g.w.sz], w[iw]);
-    const double d = dmul(scale, dadd(dadd(du, dvv), dw));
+    const double d = exact::mulc(scale, dadd(dadd(du, dvv), dw));
     dv[i] = d;
-    bb[i] = dmul(h2, d);
+    bb[i] = exact::mulc(h2, d);
 }
 
 // --- subtractGradient, project.go:172-205 ----------------------------------
@@ -343,23 +354,23 @@ __device__ __forceinline__ void div_cell(const Geom& g, AF_PTR(const double) AF_
 // new value of the face of f (the component's field) is stored to out at the
 // same index -- f itself for the reference's in-place update.
 __device__ __forceinline__ void grad_face_to(const Geom& g, AF_PTR(const double) AF_RESTRICT p,
-                                             AF_PTR(const double) f, AF_PTR(double) out, double scale, int c, int x,
+                                             AF_PTR(const double) f, AF_PTR(double) out, const exact::MulC& scale, int c, int x,
                                              int y, int z) {
     const long long ip = x + y * g.p.sy + z * g.p.sz;
     if (c == 0) {
         const long long i = x + y * g.u.sy + z * g.u.sz;
-        out[i] = dsub(f[i], dmul(scale, dsub(p[ip], p[ip - 1])));
+        out[i] = dsub(f[i], exact::mulc(scale, dsub(p[ip], p[ip - 1])));
     } else if (c == 1) {
         const long long i = x + y * g.v.sy + z * g.v.sz;
-        out[i] = dsub(f[i], dmul(scale, dsub(p[ip], p[ip - g.p.sy])));
+        out[i] = dsub(f[i], exact::mulc(scale, dsub(p[ip], p[ip - g.p.sy])));
     } else {
         const long long i = x + y * g.w.sy + z * g.w.sz;
-        out[i] = dsub(f[i], dmul(scale, dsub(p[ip], p[ip - g.p.sz])));
+        out[i] = dsub(f[i], exact::mulc(scale, dsub(p[ip], p[ip - g.p.sz])));
     }
 }
 
 __device__ __forceinline__ void grad_face(const Geom& g, AF_PTR(const double) AF_RESTRICT p, AF_PTR(double) u,
-                                          AF_PTR(double) v, AF_PTR(double) w, double scale, int c, int x, int y,
+                                          AF_PTR(double) v, AF_PTR(double) w, const exact::MulC& scale, int c, int x, int y,
                                           int z) {
     AF_PTR(double) f = c == 0 ? u : (c == 1 ? v : w);
     grad_face_to(g, p, f, f, scale, c, x, y, z);

@@ -25,6 +25,8 @@ namespace {
 
 using namespace cells;
 
+inline unsigned cdiv(long long a, long long b) { return (unsigned)((a + b - 1) / b); }
+
 // applyVelocityBC, stencil.go:246-315: 3 components x 3 write sets, each cell
 // written once (see bc_cell).
 __global__ void k_velocity_bc(Geom g, double* u, double* v, double* w, Status* st, int gate) {
@@ -50,38 +52,41 @@ struct SweepArgs {
     AF_PTR(double) tw;
     Dims du, dv, dw;
     int NX, NY, NZ, G;
-    double dt, invH, lam;
+    exact::MulC dt, invH, lam;
+    int has_lam;
+    unsigned lim[3];  // per component: high word of binary64(its extent along the sweep axis - 1)
     Status* st;
     int phase;
+    void set_scheme(int axis, double dt_, double invH_, double lam_) {
+        dt = exact::mul_const(dt_);
+        invH = exact::mul_const(invH_);
+        lam = exact::mul_const(lam_);
+        has_lam = lam_ != 0;
+        const Dims* d[3] = {&du, &dv, &dw};
+        for (int c = 0; c < 3; ++c) {
+            const int n = axis == 0 ? d[c]->nx : (axis == 1 ? d[c]->ny : d[c]->nz);
+            lim[c] = (unsigned)(exact::bits_of((double)(n - 1)) >> 32);
+        }
+    }
 };
 
-// faceVelocity (stencil.go:128-155), only the component on the active axis:
-// the other two feed nothing and have no side effects.
-template <int AX>
-__device__ __forceinline__ double face_vel(const SweepArgs& a, int c, int x, int y, int z) {
-    AF_PTR(const double) u = a.u;
-    AF_PTR(const double) v = a.v;
-    AF_PTR(const double) w = a.w;
-    auto U = [&](int i, int j, int k) { return u[i + j * a.du.sy + k * a.du.sz]; };
-    auto V = [&](int i, int j, int k) { return v[i + j * a.dv.sy + k * a.dv.sz]; };
-    auto W = [&](int i, int j, int k) { return w[i + j * a.dw.sy + k * a.dw.sz]; };
-    if (c == 0) {
-        if (AX == 0) return U(x, y, z);
-        if (AX == 1)
-            return quarter(dadd(dadd(dadd(V(x - 1, y, z), V(x, y, z)), V(x - 1, y + 1, z)), V(x, y + 1, z)));
-        return quarter(dadd(dadd(dadd(W(x - 1, y, z), W(x, y, z)), W(x - 1, y, z + 1)), W(x, y, z + 1)));
-    } else if (c == 1) {
-        if (AX == 0)
-            return quarter(dadd(dadd(dadd(U(x, y - 1, z), U(x + 1, y - 1, z)), U(x, y, z)), U(x + 1, y, z)));
-        if (AX == 1) return V(x, y, z);
-        return quarter(dadd(dadd(dadd(W(x, y - 1, z), W(x, y, z)), W(x, y - 1, z + 1)), W(x, y, z + 1)));
-    } else {
-        if (AX == 0)
-            return quarter(dadd(dadd(dadd(U(x, y, z - 1), U(x + 1, y, z - 1)), U(x, y, z)), U(x + 1, y, z)));
-        if (AX == 1)
-            return quarter(dadd(dadd(dadd(V(x, y, z - 1), V(x, y + 1, z - 1)), V(x, y, z)), V(x, y + 1, z)));
-        return W(x, y, z);
-    }
+// faceVelocity (stencil.go:128-155) along the sweep axis at a face of
+// component C, only the component on the active axis: the other two feed
+// nothing and have no side effects.  Where four faces are averaged, the sum
+// is returned and *shift = -2: the caller folds the exact factor 1/4 in.
+template <int AX, int C>
+__device__ __forceinline__ double face_vel_sum(const SweepArgs& a, int x, int y, int z, int* shift) {
+    *shift = C == AX ? 0 : -2;
+    const Dims& d = AX == 0 ? a.du : (AX == 1 ? a.dv : a.dw);
+    AF_PTR(const double) f = AX == 0 ? a.u : (AX == 1 ? a.v : a.w);
+    const int sy = (int)d.sy, sz = (int)d.sz;
+    const int i = x + y * sy + z * sz;  // a field holds < 2^31 elements
+    if (C == AX) return f[i];
+    // The reference's tap order: before the sweep axis's own component
+    // (-e_C, 0, e_AX - e_C, e_AX), after it (-e_C, e_AX - e_C, 0, e_AX).
+    const int ec = C == 0 ? 1 : (C == 1 ? sy : sz), ea = AX == 0 ? 1 : (AX == 1 ? sy : sz);
+    if (AX > C) return dadd(dadd(dadd(f[i - ec], f[i]), f[i + ea - ec]), f[i + ea]);
+    return dadd(dadd(dadd(f[i - ec], f[i + ea - ec]), f[i]), f[i + ea]);
 }
 
 __device__ __forceinline__ double lerp(double a, double b, double t, double omt) {
@@ -103,39 +108,35 @@ __device__ __forceinline__ double lerp_t0(double a, double b) {
     return a;
 }
 
-// |v| < 2^1023 on the bit pattern: a lerp of two such values with weights in
+// |v| < 2^1023 on the high word: a lerp of two such values with weights in
 // [0, 1] is finite (the result is bounded by the larger magnitude times
 // (1-t) + t <= 1 + 2^-53), so it adds as an exact zero when its weight is +0.
 __device__ __forceinline__ bool below_2p1023(double v) {
-    return ((unsigned long long)__double_as_longlong(v) & 0x7FF0000000000000ull) < 0x7FE0000000000000ull;
-}
-// Finite and nonzero: x + (+-0) == x and x * 1 == x exactly.
-__device__ __forceinline__ bool finite_nonzero(double v) {
-    const unsigned long long m = (unsigned long long)__double_as_longlong(v) & ~kSign;
-    return m != 0ull && m < 0x7FF0000000000000ull;
+    return ((unsigned)(dbits(v) >> 32) & 0x7FF00000u) < 0x7FE00000u;
 }
 
+// v * dt * invH as the reference evaluates it, (dt*v)*invH; shift: v's exact
+// power-of-two factor (face_vel_sum).
+__device__ __forceinline__ double face_shift(const SweepArgs& a, double v, int shift) {
+    const unsigned long long b = dbits(v);
+    if (a.dt.ok && a.invH.ok) {
+        if (exact::mul_range(b)) return dfrom(exact::mulc_bits(a.invH, exact::mulc_bits(a.dt, b, shift)));
+        if (exact::is_zero(b)) return v;
+    }
+    return exact::mul_native(exact::mul_native(a.dt.v, shift ? quarter(v) : v), a.invH.v);
+}
+
+// sampleTrilinear (stencil.go:166-225) for any backtrace coordinate pa along
+// the sweep axis: the clamp, the amd64 truncation, the bounds check of a NaN
+// coordinate and the whole interpolation.  Taken by the faces the integer
+// form leaves out (zero or extreme taps, clamped or non-finite coordinates);
+// a call, so none of its binary64 operations run ahead of the branch.
+// False: a contained fault, recorded; the face is not written.
 template <int AX>
-__global__ void k_sweep_fp64(SweepArgs a) {
-    if (gated(a.st, a.phase)) return;
-    const int zr = a.NZ + 1;
-    const int c = blockIdx.z / zr;
-    const int z = a.G + (int)(blockIdx.z % zr);
-    const int x = a.G + (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    const int y = a.G + (int)(blockIdx.y * blockDim.y + threadIdx.y);
-    // Face-count extents of this component (stencil.go:53-68).
-    const int x1 = a.G + a.NX + (c == 0), y1 = a.G + a.NY + (c == 1), z1 = a.G + a.NZ + (c == 2);
-    if (x >= x1 || y >= y1 || z >= z1) return;
-
+__device__ __noinline__ bool sample_general(const SweepArgs& a, int c, int x, int y, int z, double pa, double* out) {
     const Dims& d = c == 0 ? a.du : (c == 1 ? a.dv : a.dw);
     AF_PTR(const double) sd = c == 0 ? a.u : (c == 1 ? a.v : a.w);
-    AF_PTR(double) dd = c == 0 ? a.tu : (c == 1 ? a.tv : a.tw);
-
-    const double vel = face_vel<AX>(a, c, x, y, z);
-    // Backtrace along the active axis only: p -= dt*v*invH.
-    const int ca = AX == 0 ? x : (AX == 1 ? y : z);
     const int na = AX == 0 ? d.nx : (AX == 1 ? d.ny : d.nz);
-    double pa = dsub(i2d_small(ca), dmul(dmul(a.dt, vel), a.invH));
     // Clamp to [0, na-1] (pa < 0 and pa > maxA on the bit patterns: -0 and
     // NaN pass through unchanged, as the comparisons leave them).
     const unsigned long long pab = dbits(pa);
@@ -144,18 +145,16 @@ __global__ void k_sweep_fp64(SweepArgs a) {
         if ((pab & kSign) && (pab & ~kSign)) pa = 0.0;
         else if (!(pab & kSign) && pab > dbits(i2d_small(na - 1))) pa = i2d_small(na - 1);
     }
-
     // Truncation toward zero as amd64 CVTTSD2SQ does (NaN -> INT64_MIN).  The
     // two other coordinates are integer faces strictly inside the padded
     // field, so their floor is the face itself and their weight is +0.
     long long a0 = pnan ? (long long)0x8000000000000000ull : d2i_trunc_small(pa);
     if (a0 >= na - 1) a0 = na - 2;
-    const double ta = pnan ? dsub(pa, (double)a0) : frac_sub(pa, a0);
+    const double t = pnan ? dsub(pa, (double)a0) : frac_sub(pa, a0);
     long long x0 = x, y0 = y, z0 = z;
-    double tx = 0.0, ty = 0.0, tz = 0.0;
-    if (AX == 0) { x0 = a0; tx = ta; }
-    if (AX == 1) { y0 = a0; ty = ta; }
-    if (AX == 2) { z0 = a0; tz = ta; }
+    if (AX == 0) x0 = a0;
+    if (AX == 1) y0 = a0;
+    if (AX == 2) z0 = a0;
     // Index arithmetic wraps modulo 2^64, as Go's int does.
     const unsigned long long i000 =
         (unsigned long long)x0 + (unsigned long long)y0 * (unsigned long long)d.sy +
@@ -172,61 +171,125 @@ __global__ void k_sweep_fp64(SweepArgs a) {
         if (oob) {
             atomicMin(&a.st->fault_gate, a.st->step * 8u + (unsigned)a.phase);
             atomicMin(&a.st->fault_key, fault_key(c, x, y, z));
-            return;  // the faulting face is not written, as the panic leaves it
+            return false;  // the faulting face is not written, as the panic leaves it
         }
     }
-    const long long sy = d.sy, sz = d.sz;
-    const long long b = (long long)i000;
+    const long long sy = d.sy, sz = d.sz, b = (long long)i000;
     // Only the active axis has a nonzero weight; the lerps along the other
     // two (weight exactly +0) run on the integer pipe with identical bits.
-    // The zero-weight lerps only matter when their operands are not finite
-    // (NaN propagates, Inf * 0 is NaN) or when the kept value is a zero
-    // (-0 + +0 = +0): otherwise the kept value passes through exactly, and
-    // the FP64 work of the discarded lerps is skipped.
-    double adv;
-    if (AX == 0) {
-        const double omt = dsub(1.0, tx);
-        const double c00 = lerp(sd[b], sd[b + 1], tx, omt);
-        const double t1 = sd[b + sy], t2 = sd[b + sy + 1], t3 = sd[b + sz], t4 = sd[b + sz + 1];
-        const double t5 = sd[b + sz + sy], t6 = sd[b + sz + sy + 1];
-        if (finite_nonzero(c00) && below_2p1023(t1) && below_2p1023(t2) && below_2p1023(t3) && below_2p1023(t4) &&
-            below_2p1023(t5) && below_2p1023(t6)) {
-            adv = c00;
-        } else {
-            const double c10 = lerp(t1, t2, tx, omt);
-            const double c01 = lerp(t3, t4, tx, omt);
-            const double c11 = lerp(t5, t6, tx, omt);
-            adv = lerp_t0(lerp_t0(c00, c10), lerp_t0(c01, c11));
-        }
-    } else if (AX == 1) {
-        const double omt = dsub(1.0, ty);
-        const double c00 = lerp_t0(sd[b], sd[b + 1]);
-        const double c10 = lerp_t0(sd[b + sy], sd[b + sy + 1]);
-        const double y0 = lerp(c00, c10, ty, omt);
-        const double t3 = sd[b + sz], t4 = sd[b + sz + 1], t5 = sd[b + sz + sy], t6 = sd[b + sz + sy + 1];
-        // lerp_t0 of values below 2^1023 is one of them or a zero: below too.
-        if (finite_nonzero(y0) && below_2p1023(t3) && below_2p1023(t4) && below_2p1023(t5) && below_2p1023(t6)) {
-            adv = y0;
-        } else {
-            const double c01 = lerp_t0(t3, t4);
-            const double c11 = lerp_t0(t5, t6);
-            adv = lerp_t0(y0, lerp(c01, c11, ty, omt));
-        }
-    } else {
-        const double c00 = lerp_t0(sd[b], sd[b + 1]);
-        const double c10 = lerp_t0(sd[b + sy], sd[b + sy + 1]);
-        const double c01 = lerp_t0(sd[b + sz], sd[b + sz + 1]);
-        const double c11 = lerp_t0(sd[b + sz + sy], sd[b + sz + sy + 1]);
-        adv = lerp(lerp_t0(c00, c10), lerp_t0(c01, c11), tz, dsub(1.0, tz));
-    }
+    const double t0 = sd[b], t1 = sd[b + 1], t2 = sd[b + sy], t3 = sd[b + sy + 1];
+    const double t4 = sd[b + sz], t5 = sd[b + sz + 1], t6 = sd[b + sz + sy], t7 = sd[b + sz + sy + 1];
+    const double omt = dsub(1.0, t);
+    if (AX == 0)
+        *out = lerp_t0(lerp_t0(lerp(t0, t1, t, omt), lerp(t2, t3, t, omt)),
+                       lerp_t0(lerp(t4, t5, t, omt), lerp(t6, t7, t, omt)));
+    else if (AX == 1)
+        *out = lerp_t0(lerp(lerp_t0(t0, t1), lerp_t0(t2, t3), t, omt), lerp(lerp_t0(t4, t5), lerp_t0(t6, t7), t, omt));
+    else
+        *out = lerp(lerp_t0(lerp_t0(t0, t1), lerp_t0(t2, t3)), lerp_t0(lerp_t0(t4, t5), lerp_t0(t6, t7)), t, omt);
+    return true;
+}
 
-    const long long i = (long long)x + (long long)y * sy + (long long)z * sz;
-    double lap = 0.0;
-    if (a.lam != 0) {
-        const long long s = AX == 0 ? 1 : (AX == 1 ? sy : sz);
-        lap = dmul(a.lam, dadd(dsub(sd[i - s], twice(sd[i])), sd[i + s]));
+// lam * ((m - 2*c) + p), the directional diffusion (stencil.go:73-119).
+__device__ __forceinline__ double diffusion(const SweepArgs& a, double m, double c, double p) {
+    return exact::mulc(a.lam, dadd(dsub(m, twice(c)), p));
+}
+
+// One face of component C.  The common face -- backtrace inside the field,
+// both interpolated taps zero or normal, none of the other six huge --
+// computes its six products (dt, 1/h, the two weights, the diffusion) and its
+// weights with integer instructions (af_exact.cuh), so only the additions
+// (eight, or five where the face's own component is the velocity) are left
+// to the binary64 pipe, which bounds the kernel.  The lerps along the two
+// other axes, whose weight is zero, then return their first operand (their
+// second ones are finite) unless it is -0.
+// Measured at 256^3 per launch: 2.28 / 2.45 / 2.71 ms (x, y, z) with the
+// products, weights and compares on the binary64 pipe (25-29 of its
+// instructions a face), 0.78 ms each so (7); block shapes from 32 x 4 to
+// 256 x 1 measure the same.
+template <int AX, int C>
+__device__ __forceinline__ void sweep_face(const SweepArgs& a, int x, int y, int z) {
+    const Dims& d = C == 0 ? a.du : (C == 1 ? a.dv : a.dw);
+    AF_PTR(const double) sd = C == 0 ? a.u : (C == 1 ? a.v : a.w);
+    AF_PTR(double) dd = C == 0 ? a.tu : (C == 1 ? a.tv : a.tw);
+    const int sy = (int)d.sy, sz = (int)d.sz;
+    const int i = x + y * sy + z * sz, st = AX == 0 ? 1 : (AX == 1 ? sy : sz);
+    int shift;
+    const double vel = face_vel_sum<AX, C>(a, x, y, z, &shift);
+    const int ca = AX == 0 ? x : (AX == 1 ? y : z);
+    // Backtrace along the active axis only: p -= dt*v*invH.
+    const double pa = dsub(i2d_small(ca), face_shift(a, vel, shift));
+    int a0;
+    exact::Weights w;
+    double adv;
+    bool done = false;
+    if (exact::foot_split(pa, a.lim[C], &a0, &w)) {
+        const int b = i + (a0 - ca) * st;
+        // The cell's taps: b and b + st interpolate along the axis, the
+        // other six carry a zero weight.
+        const int s1 = AX == 0 ? sy : 1, s2 = AX == 2 ? sy : sz;
+        const double d0 = sd[b], d1 = sd[b + st];
+        const double q[6] = {sd[b + s1], sd[b + s1 + st], sd[b + s2], sd[b + s2 + st], sd[b + s1 + s2],
+                             sd[b + s1 + s2 + st]};
+        unsigned any = 0;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) any |= (unsigned)(dbits(q[k]) >> 32);
+        bool ok = exact::weight_range(d0) && exact::weight_range(d1);
+        if (any & 0x40000000u) {  // some |tap| >= 2: look at each
+#pragma unroll
+            for (int k = 0; k < 6; ++k) ok = ok && below_2p1023(q[k]);
+        }
+        if (ok) {
+            // On a face: d0 * 1 + d1 * 0.
+            adv = w.t == 0 ? d0 : dadd(exact::weight_mul(w.o, w.oe, d0), exact::weight_mul(w.t, w.te, d1));
+            done = dbits(adv) != kSign;
+        }
     }
+    if (!done && !sample_general<AX>(a, C, x, y, z, pa, &adv)) return;
+    double lap = 0.0;
+    if (a.has_lam) lap = diffusion(a, sd[i - st], sd[i], sd[i + st]);
     dd[i] = dadd(adv, lap);
+}
+
+// The face of a thread: z layers of blocks per component, a warp to 32
+// consecutive x.  A U row holds NX + 1 faces; with NX a multiple of 32 its
+// last face would cost a whole warp, so those faces come in further z layers,
+// 32 rows to a warp.  False: no face.
+__device__ __forceinline__ bool block_face(const SweepArgs& a, int* c, int* x, int* y, int* z) {
+    const int zr = a.NZ + 1, layer = (int)blockIdx.z;
+    if (layer < 3 * zr) {
+        *c = layer < zr ? 0 : (layer < 2 * zr ? 1 : 2);
+        *z = a.G + layer - *c * zr;
+        *x = a.G + (int)(blockIdx.x * blockDim.x + threadIdx.x);
+        *y = a.G + (int)(blockIdx.y * blockDim.y + threadIdx.y);
+        // Face-count extents of the component (stencil.go:53-68).
+        return *x < a.G + a.NX + (*c == 0) && *y < a.G + a.NY + (*c == 1) && *z < a.G + a.NZ + (*c == 2);
+    }
+    const unsigned blk = ((unsigned)(layer - 3 * zr) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+    const unsigned k = (blk * blockDim.y + threadIdx.y) * blockDim.x + threadIdx.x;
+    if (k >= (unsigned)a.NY * (unsigned)a.NZ) return false;
+    *c = 0;
+    *x = a.G + a.NX;
+    *z = a.G + (int)(k / (unsigned)a.NY);
+    *y = a.G + (int)(k % (unsigned)a.NY);
+    return true;
+}
+dim3 face_grid(const Geom& g, dim3 block) {
+    const unsigned gx = cdiv(g.NX, block.x), gy = cdiv(g.NY + 1, block.y), gz = 3u * (unsigned)(g.NZ + 1);
+    if (g.NX % block.x) return dim3(gx, gy, gz);  // the last face shares its row's last warp
+    const unsigned last = cdiv((long long)g.NY * g.NZ, (long long)gx * gy * block.x * block.y);
+    if (gz + last > 65535u) return dim3(gx + 1, gy, gz);  // the z extent of a launch
+    return dim3(gx, gy, gz + last);
+}
+
+template <int AX>
+__global__ void k_sweep_fp64(const __grid_constant__ SweepArgs a) {
+    if (gated(a.st, a.phase)) return;
+    int c, x, y, z;
+    if (!block_face(a, &c, &x, &y, &z)) return;
+    if (c == 0) sweep_face<AX, 0>(a, x, y, z);
+    else if (c == 1) sweep_face<AX, 1>(a, x, y, z);
+    else sweep_face<AX, 2>(a, x, y, z);
 }
 
 // ---------------------------------------------------------------------------
@@ -243,40 +306,17 @@ __global__ void k_sweep_fp64(SweepArgs a) {
 // directional diffusion of phi.  Along the sweep axis only: the tangential
 // weights are zero, as in the forward step.  Taps of phi^ outside the faces
 // the sweep writes read phi (the boundary-conditioned field) instead.
+// The correction of one face for any operands (clamped or NaN feet, zero,
+// huge or non-finite taps); a call, as sample_general is.
 template <int AX>
-__global__ void k_maccormack_fp64(SweepArgs a, const double* fu, const double* fv, const double* fw) {
-    if (gated(a.st, a.phase)) return;
-    const int zr = a.NZ + 1;
-    const int c = blockIdx.z / zr;
-    const int z = a.G + (int)(blockIdx.z % zr);
-    const int x = a.G + (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    const int y = a.G + (int)(blockIdx.y * blockDim.y + threadIdx.y);
-    const int x1 = a.G + a.NX + (c == 0), y1 = a.G + a.NY + (c == 1), z1 = a.G + a.NZ + (c == 2);
-    if (x >= x1 || y >= y1 || z >= z1) return;
-
+__device__ __noinline__ double maccormack_general(const SweepArgs& a, AF_PTR(const double) fd, int c, int i, int ca,
+                                                  int lo, int hi, double pf, double pb, double fwd) {
     const Dims& d = c == 0 ? a.du : (c == 1 ? a.dv : a.dw);
     AF_PTR(const double) sd = c == 0 ? a.u : (c == 1 ? a.v : a.w);
-    AF_PTR(const double) fd = view(c == 0 ? fu : (c == 1 ? fv : fw), d.count, DK_F64_MACCORMACK, 0);
-    AF_PTR(double) dd = c == 0 ? a.tu : (c == 1 ? a.tv : a.tw);
-    const long long sy = d.sy, sz = d.sz;
-    const long long step = AX == 0 ? 1 : (AX == 1 ? sy : sz);
-    const long long i = (long long)x + (long long)y * sy + (long long)z * sz;
-    const int ca = AX == 0 ? x : (AX == 1 ? y : z);
     const int na = AX == 0 ? d.nx : (AX == 1 ? d.ny : d.nz);
-    const int lo = a.G, hi = AX == 0 ? x1 - 1 : (AX == 1 ? y1 - 1 : z1 - 1);  // written faces on the axis
-    const double fwd = fd[i];
-
-    double lap = 0.0;
-    if (a.lam != 0) lap = dmul(a.lam, dadd(dsub(sd[i - step], dmul(2.0, sd[i])), sd[i + step]));
-
-    const double shift = dmul(dmul(a.dt, face_vel<AX>(a, c, x, y, z)), a.invH);
+    const long long step = AX == 0 ? 1 : (AX == 1 ? d.sy : d.sz);
+    if (isnan(pf) || isnan(pb)) return fwd;  // the forward step has dealt with it
     const double maxA = (double)(na - 1);
-    // Forward foot (the one the forward step sampled) and backward foot.
-    double pf = dsub((double)ca, shift), pb = dadd((double)ca, shift);
-    if (isnan(pf) || isnan(pb)) {  // the forward step has dealt with it
-        dd[i] = dadd(fwd, lap);
-        return;
-    }
     pf = fmin(fmax(pf, 0.0), maxA);
     pb = fmin(fmax(pb, 0.0), maxA);
     long long f0 = (long long)pf, b0 = (long long)pb;
@@ -288,11 +328,75 @@ __global__ void k_maccormack_fp64(SweepArgs a, const double* fu, const double* f
     auto phi_hat = [&](long long k) { return (k >= lo && k <= hi) ? fd[base + k * step] : sd[base + k * step]; };
     const double tb = dsub(pb, (double)b0);
     const double back = dadd(dmul(phi_hat(b0), dsub(1.0, tb)), dmul(phi_hat(b0 + 1), tb));
-    double out = dadd(fwd, dmul(0.5, dsub(sd[i], back)));
-    if (!(out >= mn && out <= mx)) out = fwd;
+    const double out = dadd(fwd, dmul(0.5, dsub(sd[i], back)));
+    return out >= mn && out <= mx ? out : fwd;
+}
+
+// Finite doubles in their numeric order as integers, -0 equal to +0.
+__device__ __forceinline__ long long order_key(double v) {
+    const long long k = (long long)dbits(v);
+    return (k << 1) == 0 ? 0 : k ^ ((k >> 63) & 0x7FFFFFFFFFFFFFFFll);
+}
+__device__ __forceinline__ bool finite(double v) {
+    return ((unsigned)(dbits(v) >> 32) & 0x7FF00000u) != 0x7FF00000u;
+}
+
+// As sweep_face: the common face's products, weights, halving and limiter
+// comparisons are integer instructions, its additions (eleven, or eight where
+// the component is the velocity) the only work of the binary64 pipe.  With
+// the forward step, a sweep at 128^3 went from about 1.0 to 0.22 ms.
+template <int AX, int C>
+__device__ __forceinline__ void maccormack_face(const SweepArgs& a, const double* fwd_field, int x, int y, int z) {
+    const Dims& d = C == 0 ? a.du : (C == 1 ? a.dv : a.dw);
+    AF_PTR(const double) sd = C == 0 ? a.u : (C == 1 ? a.v : a.w);
+    AF_PTR(const double) fd = view(fwd_field, d.count, DK_F64_MACCORMACK, 0);
+    AF_PTR(double) dd = C == 0 ? a.tu : (C == 1 ? a.tv : a.tw);
+    const int sy = (int)d.sy, sz = (int)d.sz;
+    const int i = x + y * sy + z * sz, st = AX == 0 ? 1 : (AX == 1 ? sy : sz);
+    const int ca = AX == 0 ? x : (AX == 1 ? y : z);
+    // Written faces on the axis.
+    const int lo = a.G, hi = a.G + (AX == 0 ? a.NX : (AX == 1 ? a.NY : a.NZ)) - (C == AX ? 0 : 1);
+    const double fwd = fd[i], here = sd[i];
+    int shift;
+    const double vel = face_vel_sum<AX, C>(a, x, y, z, &shift);
+    const double cad = i2d_small(ca), s = face_shift(a, vel, shift);
+    // Forward foot (the one the forward step sampled) and backward foot.
+    const double pf = dsub(cad, s), pb = dadd(cad, s);
+    int f0, b0;
+    exact::Weights w;
+    double out;
+    bool done = false;
+    if (exact::foot_cell(pf, a.lim[C], &f0) && exact::foot_split(pb, a.lim[C], &b0, &w)) {
+        const int base = i - ca * st;
+        const double s0 = sd[base + f0 * st], s1 = sd[base + (f0 + 1) * st];
+        auto phi_hat = [&](int k) { return (k >= lo && k <= hi) ? fd[base + k * st] : sd[base + k * st]; };
+        const double e0 = phi_hat(b0), e1 = phi_hat(b0 + 1);
+        if (exact::weight_range(e0) && exact::weight_range(e1)) {
+            const double back = w.t == 0 ? e0 : dadd(exact::weight_mul(w.o, w.oe, e0), exact::weight_mul(w.t, w.te, e1));
+            out = dadd(fwd, half(dsub(here, back)));
+            if (dbits(back) != kSign && finite(s0) && finite(s1) && finite(out)) {
+                const long long k0 = order_key(s0), k1 = order_key(s1), k = order_key(out);
+                if (k < (k0 < k1 ? k0 : k1) || k > (k0 < k1 ? k1 : k0)) out = fwd;
+                done = true;
+            }
+        }
+    }
+    if (!done) out = maccormack_general<AX>(a, fd, C, i, ca, lo, hi, pf, pb, fwd);
+    double lap = 0.0;
+    if (a.has_lam) lap = diffusion(a, sd[i - st], here, sd[i + st]);
     dd[i] = dadd(out, lap);
 }
 
+template <int AX>
+__global__ void k_maccormack_fp64(const __grid_constant__ SweepArgs a, const double* fu, const double* fv,
+                                  const double* fw) {
+    if (gated(a.st, a.phase)) return;
+    int c, x, y, z;
+    if (!block_face(a, &c, &x, &y, &z)) return;
+    if (c == 0) maccormack_face<AX, 0>(a, fu, x, y, z);
+    else if (c == 1) maccormack_face<AX, 1>(a, fv, x, y, z);
+    else maccormack_face<AX, 2>(a, fw, x, y, z);
+}
 
 // ---------------------------------------------------------------------------
 // solvePressureRedBlack's zeroing (project.go:81-83) fused with
@@ -302,7 +406,8 @@ __global__ void k_maccormack_fp64(SweepArgs a, const double* fu, const double* f
 // ---------------------------------------------------------------------------
 __global__ void k_divergence_fp64(Geom g, const double* __restrict__ u, const double* __restrict__ v,
                                   const double* __restrict__ w, double* __restrict__ p, double* __restrict__ dv,
-                                  double* __restrict__ bb, double scale, double h2, int zero_p, Status* st,
+                                  double* __restrict__ bb, const __grid_constant__ exact::MulC scale,
+                                  const __grid_constant__ exact::MulC h2, int zero_p, Status* st,
                                   int gate) {
     if (gated(st, gate)) return;
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
@@ -372,12 +477,13 @@ __global__ void k_pressure_bc(Geom g, double* __restrict__ p, Status* st, int ga
 
 // subtractGradient, project.go:172-205.
 __global__ void k_gradient_fp64(Geom g, const double* __restrict__ p, double* __restrict__ u, double* __restrict__ v,
-                                double* __restrict__ w, double scale, Status* st, int gate) {
+                                double* __restrict__ w, const __grid_constant__ exact::MulC scale, Status* st,
+                                int gate) {
     if (gated(st, gate)) return;
     const int G = g.G;
-    const int zr = g.NZ + 1;
-    const int c = blockIdx.z / zr;
-    const int z = G + (int)(blockIdx.z % zr);
+    const int zr = g.NZ + 1, zc = (int)blockIdx.z;
+    const int c = zc < zr ? 0 : (zc < 2 * zr ? 1 : 2);
+    const int z = G + zc - c * zr;
     const int x = G + (int)(blockIdx.x * blockDim.x + threadIdx.x);
     const int y = G + (int)(blockIdx.y * blockDim.y + threadIdx.y);
     const int x1 = G + g.NX + (c == 0), y1 = G + g.NY + (c == 1), z1 = G + g.NZ + (c == 2);
@@ -531,8 +637,6 @@ __global__ void __launch_bounds__(kKeThreads) k_ke_final(const double* partials_
     s = block_sum_fixed(s);
     if (threadIdx.x == 0) *out = s;
 }
-
-inline unsigned cdiv(long long a, long long b) { return (unsigned)((a + b - 1) / b); }
 
 // Self-test of the exact /6 forms against IEEE division over PCG32-random
 // doubles: uniform significands, exponents spread over the whole range
@@ -697,10 +801,9 @@ void launch_sweep_fp64(const Geom& g, int axis, const Fields& f, double dt, doub
     a.tw = view(f.t2, g.w.count, DK_F64_SWEEP, 0);
     a.du = g.u; a.dv = g.v; a.dw = g.w;
     a.NX = g.NX; a.NY = g.NY; a.NZ = g.NZ; a.G = g.G;
-    a.dt = dt; a.invH = invH; a.lam = lam;
+    a.set_scheme(axis, dt, invH, lam);
     a.st = st; a.phase = phase;
-    dim3 block(64, 4);
-    dim3 grid(cdiv(g.NX + 1, 64), cdiv(g.NY + 1, 4), 3 * (g.NZ + 1));
+    const dim3 block(32, 8), grid = face_grid(g, block);
     if (axis == 0) k_sweep_fp64<0><<<grid, block, 0, s>>>(a);
     else if (axis == 1) k_sweep_fp64<1><<<grid, block, 0, s>>>(a);
     else k_sweep_fp64<2><<<grid, block, 0, s>>>(a);
@@ -719,10 +822,9 @@ void launch_maccormack_fp64(const Geom& g, int axis, const Fields& f, const Fiel
     a.tw = view(f.t2, g.w.count, DK_F64_SWEEP, 0);
     a.du = g.u; a.dv = g.v; a.dw = g.w;
     a.NX = g.NX; a.NY = g.NY; a.NZ = g.NZ; a.G = g.G;
-    a.dt = dt; a.invH = invH; a.lam = lam;
+    a.set_scheme(axis, dt, invH, lam);
     a.st = st; a.phase = phase;
-    dim3 block(64, 4);
-    dim3 grid(cdiv(g.NX + 1, 64), cdiv(g.NY + 1, 4), 3 * (g.NZ + 1));
+    const dim3 block(32, 8), grid = face_grid(g, block);
     if (axis == 0) k_maccormack_fp64<0><<<grid, block, 0, s>>>(a, fwd.t0, fwd.t1, fwd.t2);
     else if (axis == 1) k_maccormack_fp64<1><<<grid, block, 0, s>>>(a, fwd.t0, fwd.t1, fwd.t2);
     else k_maccormack_fp64<2><<<grid, block, 0, s>>>(a, fwd.t0, fwd.t1, fwd.t2);
@@ -732,7 +834,8 @@ void launch_divergence_fp64(const Geom& g, const Fields& f, double* b, double sc
                             Status* st, int gate, cudaStream_t s) {
     dim3 block(64, 4);
     dim3 grid(cdiv(g.p.nx, 64), cdiv(g.p.ny, 4), g.p.nz);
-    k_divergence_fp64<<<grid, block, 0, s>>>(g, f.u, f.v, f.w, f.p, f.div, b, scale, h2, zero_p ? 1 : 0, st, gate);
+    k_divergence_fp64<<<grid, block, 0, s>>>(g, f.u, f.v, f.w, f.p, f.div, b, exact::mul_const(scale),
+                                             exact::mul_const(h2), zero_p ? 1 : 0, st, gate);
 }
 
 // Integer-pipe share of the red-black chain: AEROFLUX_RBGS_EMU picks the
@@ -772,7 +875,7 @@ void launch_pressure_bc_fp64(const Geom& g, double* p, Status* st, int gate, cud
 void launch_gradient_fp64(const Geom& g, const Fields& f, double scale, Status* st, int gate, cudaStream_t s) {
     dim3 block(64, 4);
     dim3 grid(cdiv(g.NX + 1, 64), cdiv(g.NY + 1, 4), 3 * (g.NZ + 1));
-    k_gradient_fp64<<<grid, block, 0, s>>>(g, f.p, f.u, f.v, f.w, scale, st, gate);
+    k_gradient_fp64<<<grid, block, 0, s>>>(g, f.p, f.u, f.v, f.w, exact::mul_const(scale), st, gate);
 }
 
 void launch_step_tick(Status* st, cudaStream_t s) { k_step_tick<<<1, 1, 0, s>>>(st); }
