@@ -46,22 +46,6 @@ constexpr int kMaxLev = 16;
 constexpr int kCoarseThreads = 512;
 constexpr int kCoarseMax = 4096;
 
-// Unsigned 32-bit division by an invariant divisor with one multiply-high
-// (Granlund & Montgomery, "Division by invariant integers using
-// multiplication", 1994): l = ceil(log2 d), m = ceil(2^(32+l)/d) - 2^32,
-// n/d = (umulhi(n, m) + n) >> l for every n < 2^32.
-struct FastDiv {
-    unsigned d = 1, m = 0, l = 0;
-    FastDiv() = default;
-    __host__ explicit FastDiv(unsigned div) : d(div) {
-        while ((1ull << l) < d) ++l;
-        m = (unsigned)((((1ull << (32 + l)) + d - 1) / d) - (1ull << 32));
-    }
-    __device__ __forceinline__ unsigned div(unsigned n) const {
-        return (unsigned)(((unsigned long long)__umulhi(n, m) + n) >> l);
-    }
-};
-
 struct Lvl {
     int nx, ny, nz;
     float wx, wy, wz;   // (h0 / h_axis)^2

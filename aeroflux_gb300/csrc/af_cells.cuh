@@ -131,56 +131,15 @@ __device__ __forceinline__ double div6_int(double x) {
     return __longlong_as_double((long long)((b & kSign) | (e << 52) | (Q & 0xFFFFFFFFFFFFFull)));
 }
 
-// RN(a + b) in binary64 on the integer pipe.  Significands are aligned in
-// 64-bit integers with the leading bit at 62, leaving 10 guard bits; bits
-// shifted out of the smaller operand fold into a sticky bit.  Equal signs
-// add (one carry renormalisation), opposite signs subtract and renormalise
-// left (exact whenever more than the guard bits would be needed, i.e. for
-// exponent gaps of 0 or 1), then round to nearest, ties to even.  Zero and
-// subnormal operands, Inf, NaN and results that are subnormal or overflow
-// take the native add, so the result always equals __dadd_rn(a, b).
+// RN(a + b) with 32-bit instructions (exact::add_sum), the native addition --
+// a call, see exact::mul_native -- for the operands that leaves out: zero,
+// tiny, huge and non-finite ones, gaps of more than 31 binades and deep
+// cancellation.
+static __device__ __noinline__ double dadd_call(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double dadd_int(double a, double b) {
-    unsigned long long ua = (unsigned long long)__double_as_longlong(a);
-    unsigned long long ub = (unsigned long long)__double_as_longlong(b);
-    unsigned long long ma = ua & ~kSign, mb = ub & ~kSign;
-    if (ma < mb) {
-        const unsigned long long t = ua; ua = ub; ub = t;
-        const unsigned long long m = ma; ma = mb; mb = m;
-    }
-    const unsigned ea = (unsigned)(ma >> 52), eb = (unsigned)(mb >> 52);
-    if (eb == 0u || ea == 0x7FFu) return __dadd_rn(a, b);
-    const unsigned long long frac = 0xFFFFFFFFFFFFFull, one = 0x10000000000000ull;
-    const unsigned long long A = ((ma & frac) | one) << 10;
-    unsigned long long B = ((mb & frac) | one) << 10;
-    const unsigned d = ea - eb;
-    if (d >= 64u) B = 1ull;
-    else if (d) B = (B >> d) | ((B << (64u - d)) != 0ull ? 1ull : 0ull);
-    int e = (int)ea;
-    unsigned long long S;
-    if (((ua ^ ub) & kSign) == 0ull) {
-        S = A + B;
-        if (S >> 63) {
-            S = (S >> 1) | (S & 1ull);
-            e += 1;
-        }
-    } else {
-        S = A - B;
-        if (S == 0ull) return 0.0;  // x + (-x) = +0 under round to nearest
-        const int lz = __clzll((long long)S) - 1;
-        S <<= lz;
-        e -= lz;
-    }
-    unsigned long long M = S >> 10;
-    const unsigned long long R = S & 0x3FFull;
-    if (R > 0x200ull || (R == 0x200ull && (M & 1ull))) {
-        M += 1ull;
-        if (M >> 53) {
-            M >>= 1;
-            e += 1;
-        }
-    }
-    if (e <= 0 || e >= 0x7FF) return __dadd_rn(a, b);
-    return __longlong_as_double((long long)((ua & kSign) | ((unsigned long long)e << 52) | (M & frac)));
+    exact::Sum s;
+    if (exact::add_sum(dbits(a), dbits(b), &s)) return dfrom(exact::pack_sum(s));
+    return dadd_call(a, b);
 }
 
 // a - b through dadd_int (negation is exact).
@@ -324,27 +283,33 @@ __device__ __forceinline__ void pbc_cell(const Geom& g, AF_PTR(double) p, int se
     p[x + y * g.p.sy + z * g.p.sz] = p[cx + cy * g.p.sy + cz * g.p.sz];
 }
 
-// --- computeDivergence (project.go:42-62) + P zeroing + B = h2*Div ---------
-// (x, y, z) is any cell of the padded P extent.  The two products are integer
-// instructions (af_exact.cuh): the five additions left bound the kernel
-// (256^3, per launch: 260 us with the products on the binary64 pipe, 189 so).
+// --- computeDivergence (project.go:42-62) ----------------------------------
+// The products with the constants are integer instructions (af_exact.cuh):
+// the five additions left bound the kernels (256^3, per launch: 260 us with
+// the products on the binary64 pipe, 189 so).
+__device__ __forceinline__ double div_value(const Geom& g, AF_PTR(const double) AF_RESTRICT u,
+                                            AF_PTR(const double) AF_RESTRICT v, AF_PTR(const double) AF_RESTRICT w,
+                                            const exact::MulC& scale, int x, int y, int z) {
+    const int iu = x + y * (int)g.u.sy + z * (int)g.u.sz;  // a field holds < 2^31 elements
+    const int iv = x + y * (int)g.v.sy + z * (int)g.v.sz;
+    const int iw = x + y * (int)g.w.sy + z * (int)g.w.sz;
+    const double du = dsub(u[iu + 1], u[iu]);
+    const double dvv = dsub(v[iv + (int)g.v.sy], v[iv]);
+    const double dw = dsub(w[iw + (int)g.w.sz], w[iw]);
+    return exact::mulc(scale, dadd(dadd(du, dvv), dw));
+}
+// The batched form: with P zeroed and B = h2*Div, over any cell (x, y, z) of
+// the padded P extent.
 __device__ __forceinline__ void div_cell(const Geom& g, AF_PTR(const double) AF_RESTRICT u,
                                          AF_PTR(const double) AF_RESTRICT v, AF_PTR(const double) AF_RESTRICT w,
                                          AF_PTR(double) AF_RESTRICT p, AF_PTR(double) AF_RESTRICT dv,
                                          AF_PTR(double) AF_RESTRICT bb, const exact::MulC& scale,
-                                         const exact::MulC& h2, bool zero_p, int x,
-                                         int y, int z) {
-    const long long i = x + y * g.p.sy + z * g.p.sz;
+                                         const exact::MulC& h2, bool zero_p, int x, int y, int z) {
+    const int i = x + y * (int)g.p.sy + z * (int)g.p.sz;
     if (zero_p) p[i] = 0.0;
     const int G = g.G;
     if (x < G || x >= G + g.NX || y < G || y >= G + g.NY || z < G || z >= G + g.NZ) return;
-    const long long iu = x + y * g.u.sy + z * g.u.sz;
-    const long long iv = x + y * g.v.sy + z * g.v.sz;
-    const long long iw = x + y * g.w.sy + z * g.w.sz;
-    const double du = dsub(u[iu + 1], u[iu]);
-    const double dvv = dsub(v[iv + g.v.sy], v[iv]);
-    const double dw = dsub(w[iw + g.w.sz], w[iw]);
-    const double d = exact::mulc(scale, dadd(dadd(du, dvv), dw));
+    const double d = div_value(g, u, v, w, scale, x, y, z);
     dv[i] = d;
     bb[i] = exact::mulc(h2, d);
 }

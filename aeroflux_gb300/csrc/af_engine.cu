@@ -195,7 +195,8 @@ struct af_engine {
     int parity = 0;           // 1 when U/V/W live in the Tmp slots (after a faulted step)
     int64_t bytes = 0;
     char* arena = nullptr;
-    double* b = nullptr;      // h2*Div (P-shaped), FP64 form
+    char* split_mem = nullptr;  // FP64 form: the red-black sweeps' scratch
+    af::Split split{};
     Status* st = nullptr;
     double* partials = nullptr;
     double* sum = nullptr;
@@ -315,16 +316,16 @@ void enqueue_project_fp64(af_engine* e, const Fields& f, int gate) {
     af::launch_velocity_bc(g, f.u, f.v, f.w, e->st, gate, s);
     const double scale = c.density / (c.dt * c.h);  // project.go:49
     const double h2 = c.h * c.h;                    // project.go:107
-    af::launch_divergence_fp64(g, f, e->b, scale, h2, true, e->st, gate, s);
+    af::launch_divergence_fp64(g, f, &e->split, scale, h2, e->st, gate, s);
     rec(e, kEvRb + (gate == 3 ? 0 : 2));
     for (int64_t it = 0; it < c.gauss_seidel_iters; ++it) {
-        af::launch_rbgs_fp64(g, f.p, e->b, 0, e->st, gate, s);
-        af::launch_rbgs_fp64(g, f.p, e->b, 1, e->st, gate, s);
+        af::launch_rbgs_fp64(e->split, 0, s);
+        af::launch_rbgs_fp64(e->split, 1, s);
     }
     rec(e, kEvRb + (gate == 3 ? 1 : 3));
     e->launches_per_step += 5 + 2 * c.gauss_seidel_iters;
     e->rbgs_launches_per_step += 2 * c.gauss_seidel_iters;
-    af::launch_pressure_bc_fp64(g, f.p, e->st, gate, s);
+    af::launch_join_fp64(g, e->split, f.p, e->st, gate, s);
     af::launch_gradient_fp64(g, f, c.dt / (c.density * c.h), e->st, gate, s);  // project.go:179
     af::launch_velocity_bc(g, f.u, f.v, f.w, e->st, gate, s);
 }
@@ -442,13 +443,13 @@ int release(af_engine* e) {
     cudaFree(e->mc_scratch);
     e->mc_scratch = nullptr;
     cudaFree(e->arena);
-    cudaFree(e->b);
+    cudaFree(e->split_mem);
     cudaFree(e->st);
     cudaFree(e->partials);
     cudaFree(e->sum);
     cudaFree(e->mx);
     e->arena = nullptr;
-    e->b = nullptr;
+    e->split_mem = nullptr;
     e->st = nullptr;
     e->partials = e->sum = nullptr;
     e->mx = nullptr;
@@ -597,10 +598,12 @@ int af_create(const af_config* cin, af_engine** out, char* err, size_t errlen) {
         return fail(AF_ERR_NOMEM);
     }
     if (c.precision == AF_PRECISION_FP64) {
-        if ((cr = cudaMalloc(&e->b, (size_t)e->desc[AF_FIELD_P].count * 8)) != cudaSuccess) {
+        e->split = af::Split::of(g);
+        if ((cr = cudaMalloc(&e->split_mem, e->split.bytes())) != cudaSuccess) {
             e->err = sfmt("aeroflux: device scratch: %s", cudaGetErrorString(cr));
             return fail(AF_ERR_NOMEM);
         }
+        e->split.place(e->split_mem);
     }
     if ((cr = cudaMalloc(&e->st, sizeof(Status))) != cudaSuccess ||
         (cr = cudaMalloc(&e->partials, sizeof(double) * (size_t)std::max<int64_t>(c.nz, 1))) != cudaSuccess ||
@@ -763,7 +766,7 @@ int af_phase_divergence(af_engine* e) {
     }
     if (int rc = reset_status(e)) return rc;
     const af_config& c = e->cfg;
-    af::launch_divergence_fp64(e->geom, e->fields(), e->b, c.density / (c.dt * c.h), c.h * c.h, false, e->st, 0,
+    af::launch_divergence_fp64(e->geom, e->fields(), nullptr, c.density / (c.dt * c.h), c.h * c.h, e->st, 0,
                                e->stream);
     AF_CUDA(e, cudaGetLastError());
     return sync_and_check(e);
@@ -776,17 +779,15 @@ int af_phase_red_black(af_engine* e) {
         return AF_ERR_UNSUPPORTED;
     }
     if (int rc = reset_status(e)) return rc;
-    // solvePressureRedBlack zeroes P itself (project.go:81-83); the divergence
-    // kernel does that zeroing in the fused path, so do it here explicitly.
+    // solvePressureRedBlack zeroes P itself (project.go:81-83), and B = h2*Div
+    // as the divergence kernel would have left it.
     Fields f = e->fields();
-    AF_CUDA(e, cudaMemsetAsync(f.p, 0, (size_t)e->desc[AF_FIELD_P].count * 8, e->stream));
-    // B = h2*Div as the divergence kernel would have left it.
-    af::launch_b_from_div(e->geom, f.div, e->b, e->cfg.h * e->cfg.h, e->stream);
+    af::launch_split_from_div(e->geom, f.div, e->split, e->cfg.h * e->cfg.h, e->stream);
     for (int64_t it = 0; it < e->cfg.gauss_seidel_iters; ++it) {
-        af::launch_rbgs_fp64(e->geom, f.p, e->b, 0, e->st, 0, e->stream);
-        af::launch_rbgs_fp64(e->geom, f.p, e->b, 1, e->st, 0, e->stream);
+        af::launch_rbgs_fp64(e->split, 0, e->stream);
+        af::launch_rbgs_fp64(e->split, 1, e->stream);
     }
-    af::launch_pressure_bc_fp64(e->geom, f.p, e->st, 0, e->stream);
+    af::launch_join_fp64(e->geom, e->split, f.p, e->st, 0, e->stream);
     AF_CUDA(e, cudaGetLastError());
     return sync_and_check(e);
 }

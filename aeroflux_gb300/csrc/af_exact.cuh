@@ -209,5 +209,114 @@ AF_HD double weight_mul(u64 w, int we, double d) {
                      (b & kSignBit));
 }
 
+// ---------------------------------------------------------------------------
+// RN(a + b) and RN(RN(a - b) / 6) with 32-bit instructions
+// ---------------------------------------------------------------------------
+// 32 bits of hi:lo starting s bits up (fsr) or s bits down from the top (fsl); 0 <= s < 32.
+AF_HD unsigned fsr(unsigned lo, unsigned hi, int s) {
+#if defined(__CUDA_ARCH__)
+    return __funnelshift_r(lo, hi, s);
+#else
+    return (unsigned)((((u64)hi << 32) | lo) >> s);
+#endif
+}
+AF_HD unsigned fsl(unsigned lo, unsigned hi, int s) {
+#if defined(__CUDA_ARCH__)
+    return __funnelshift_l(lo, hi, s);
+#else
+    return (unsigned)(((((u64)hi << 32) | lo) << s) >> 32);
+#endif
+}
+AF_HD int clz32(unsigned v) {
+#if defined(__CUDA_ARCH__)
+    return __clz((int)v);
+#else
+    return v ? __builtin_clz(v) : 32;
+#endif
+}
+// h:l:r += carry-in and b:bl:0, 96 bits.
+AF_HD void add96(unsigned& h, unsigned& l, unsigned& r, unsigned bh, unsigned bl, unsigned cin) {
+#if defined(__CUDA_ARCH__)
+    asm("add.cc.u32 %0, %0, %5;\n\taddc.cc.u32 %1, %1, %4;\n\taddc.u32 %2, %2, %3;"
+        : "+r"(r), "+r"(l), "+r"(h)
+        : "r"(bh), "r"(bl), "r"(cin));
+#else
+    const unsigned __int128 t = (((unsigned __int128)h << 64) | ((unsigned __int128)l << 32) | r) +
+                                (((unsigned __int128)bh << 64) | ((unsigned __int128)bl << 32)) + cin;
+    h = (unsigned)(t >> 64), l = (unsigned)(t >> 32), r = (unsigned)t;
+#endif
+}
+// h:l += v; the carry out.
+AF_HD unsigned add64_carry(unsigned& h, unsigned& l, unsigned v) {
+#if defined(__CUDA_ARCH__)
+    unsigned c;
+    asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, 0;\n\taddc.u32 %2, 0, 0;" : "+r"(l), "+r"(h), "=r"(c) : "r"(v));
+    return c;
+#else
+    const unsigned __int128 t = (((unsigned __int128)h << 32) | l) + v;
+    h = (unsigned)(t >> 32), l = (unsigned)t;
+    return (unsigned)(t >> 64);
+#endif
+}
+
+// A rounded sum before packing: its 53-bit significand at the top of c:h:l
+// (c = 1, h = 0 when it rounded up to the next power of two), the low 11
+// bits of l unspecified; e the exponent field for c = 0; sign in bit 31.
+struct Sum {
+    unsigned c, h, l, sign;
+    int e;
+};
+
+// RN(a + b) for normal operands (fields 64 .. 2044) at most 31 binades
+// apart whose sum keeps at least one of the larger one's upper 21 bits;
+// false otherwise (*s is then unspecified).  The smaller significand is
+// aligned to the larger over 96 bits, which hold every bit of both, so the
+// sum is exact before it is rounded once.  The logic and shift pipe bounds
+// this form: the complement of a subtraction is a multiply-add.
+AF_HD bool add_sum(u64 a, u64 b, Sum* s) {
+    const unsigned ah = (unsigned)(a >> 32), al = (unsigned)a, bh = (unsigned)(b >> 32), bl = (unsigned)b;
+    const unsigned ma = ah & 0x7FFFFFFFu, mb = bh & 0x7FFFFFFFu;
+    const bool sw = ma < mb;
+    const unsigned big = ma > mb ? ma : mb, small = ma < mb ? ma : mb;
+    const unsigned bigl = sw ? bl : al, smalll = sw ? al : bl;
+    const int eb = (int)(big >> 20), d = eb - (int)(small >> 20);
+    const unsigned B = (big & 0xFFFFFu) | 0x100000u, S = (small & 0xFFFFFu) | 0x100000u;
+    const unsigned m = (unsigned)((int)(ah ^ bh) >> 31), f = m | 1u;  // -1 - v = v * -1 + -1 to subtract
+    const int dd = d & 31;
+    unsigned r = fsr(0u, smalll, dd) * f + m, l = fsr(smalll, S, dd) * f + m, h = (S >> dd) * f + m;
+    add96(h, l, r, B, bigl, m & 1u);
+    // h = 0: deep cancellation; h negative: equal high words.
+    const bool ok = small >= (64u << 20) && big < (2045u << 20) && d <= 31 && h - 1u < 0x3FFFFFu;
+    const int z = clz32(h) & 31;  // 10 .. 31
+    s->h = fsl(l, h, z);
+    s->l = fsl(r, l, z);
+    // Round to nearest even at bit 11 of l; what lies below l is sticky.
+    const unsigned q = ((s->l >> 11) & 1u) | ((r << z) != 0u ? 1u : 0u);
+    s->c = add64_carry(s->h, s->l, 0x3FFu + q);
+    s->e = eb + 11 - z;
+    s->sign = (sw ? bh : ah) & 0x80000000u;
+    return ok;
+}
+AF_HD u64 pack_sum(const Sum& s) {
+    const unsigned hi = (((unsigned)(s.e - 1) << 20) + fsr(s.h, s.c, 11)) | s.sign;
+    return ((u64)hi << 32) | fsr(s.l, s.h, 11);
+}
+
+// RN(x / 6) of a rounded sum with c = 0, as div6_int divides: x / 6 =
+// 2^-1 x / 3, the significand division by 3 exact integer work (a
+// multiply-high by ceil(2^64 / 3) is the exact quotient below 2^63).
+AF_HD u64 div6_sum(const Sum& s) {
+    const unsigned t = s.h >= 0xC0000000u ? 1u : 2u;
+    const int up = 11 - (int)t;
+    const u64 n = ((u64)(s.h >> up) << 32) | fsr(s.l & ~0x7FFu, s.h, up);
+#if defined(__CUDA_ARCH__)
+    u64 q = __umul64hi(n, 0x5555555555555556ull);
+#else
+    u64 q = n / 3;
+#endif
+    if ((unsigned)n - 3u * (unsigned)q == 2u) q += 1ull;  // remainder 2/3: up; 1/3: down; never a tie
+    return (q + ((u64)(unsigned)(s.e - 2 - (int)t) << 52)) | ((u64)s.sign << 32);
+}
+
 }  // namespace exact
 }  // namespace af

@@ -399,71 +399,138 @@ __global__ void k_maccormack_fp64(const __grid_constant__ SweepArgs a, const dou
 }
 
 // ---------------------------------------------------------------------------
-// solvePressureRedBlack's zeroing (project.go:81-83) fused with
-// computeDivergence (project.go:42-62).  Also stores B = h2*Div, the product
-// every red-black update recomputes (project.go:126), so the sweeps read it
-// instead of multiplying again: same bits, one FP64 multiply fewer per update.
+// computeDivergence (project.go:42-62).  For the red-black sweeps it also
+// stores B = h2*Div, the product every update recomputes (project.go:126),
+// split by colour -- same bits, one multiply fewer per update -- and zeroes
+// their P (project.go:81-83).
 // ---------------------------------------------------------------------------
-__global__ void k_divergence_fp64(Geom g, const double* __restrict__ u, const double* __restrict__ v,
-                                  const double* __restrict__ w, double* __restrict__ p, double* __restrict__ dv,
-                                  double* __restrict__ bb, const __grid_constant__ exact::MulC scale,
-                                  const __grid_constant__ exact::MulC h2, int zero_p, Status* st,
-                                  int gate) {
+__device__ __forceinline__ void split_store(const Split& S, const exact::MulC& h2, int xi, int yi, int zi, double d) {
+    AF_PTR(double) b = view(S.b, 2 * S.bn, DK_F64_DIV, 0);
+    const int c = (xi + yi + zi + S.G) & 1;
+    b[c * S.bn + ((xi >> 1) + S.hx * (yi + S.NY * zi))] = exact::mulc(h2, d);
+}
+__device__ __forceinline__ void split_zero(const Split& S) {
+    AF_PTR(double) p = view(S.p, 2 * S.pn, DK_F64_DIV, 0);
+    const long long block = ((long long)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+    const int n = blockDim.x * blockDim.y, t = threadIdx.y * blockDim.x + threadIdx.x;
+    const long long stride = (long long)gridDim.x * gridDim.y * gridDim.z * n;
+    for (long long k = block * n + t; k < 2 * S.pn; k += stride) p[k] = 0.0;
+}
+
+__global__ void k_divergence_fp64(const __grid_constant__ Geom g, const double* __restrict__ u,
+                                  const double* __restrict__ v, const double* __restrict__ w, double* __restrict__ dv,
+                                  const __grid_constant__ Split S, int with_b,
+                                  const __grid_constant__ exact::MulC scale, const __grid_constant__ exact::MulC h2,
+                                  Status* st, int gate) {
     if (gated(st, gate)) return;
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = blockIdx.y * blockDim.y + threadIdx.y;
-    const int z = blockIdx.z;
-    if (x >= g.p.nx || y >= g.p.ny) return;
-    div_cell(g, view(u, g.u.count, DK_F64_DIV, 0), view(v, g.v.count, DK_F64_DIV, 0),
-             view(w, g.w.count, DK_F64_DIV, 0), view(p, g.p.count, DK_F64_DIV, 0),
-             view(dv, g.p.count, DK_F64_DIV, 0), view(bb, g.p.count, DK_F64_DIV, 0), scale, h2, zero_p != 0, x,
-             y, z);
+    if (with_b) split_zero(S);
+    const int xi = blockIdx.x * blockDim.x + threadIdx.x;
+    const int yi = blockIdx.y * blockDim.y + threadIdx.y;
+    const int zi = blockIdx.z;
+    if (xi >= g.NX || yi >= g.NY) return;
+    const int x = g.G + xi, y = g.G + yi, z = g.G + zi;
+    const double d = div_value(g, view(u, g.u.count, DK_F64_DIV, 0), view(v, g.v.count, DK_F64_DIV, 0),
+                               view(w, g.w.count, DK_F64_DIV, 0), scale, x, y, z);
+    view(dv, g.p.count, DK_F64_DIV, 0)[x + y * g.p.sy + z * g.p.sz] = d;
+    if (with_b) split_store(S, h2, xi, yi, zi, d);
+}
+
+// The same split arrays for the red-black phase hook, when Div was supplied
+// directly instead of by the divergence kernel.
+__global__ void k_split_from_div(const __grid_constant__ Geom g, const double* __restrict__ dv,
+                                 const __grid_constant__ Split S, const __grid_constant__ exact::MulC h2) {
+    split_zero(S);
+    const int xi = blockIdx.x * blockDim.x + threadIdx.x;
+    const int yi = blockIdx.y * blockDim.y + threadIdx.y;
+    const int zi = blockIdx.z;
+    if (xi >= g.NX || yi >= g.NY) return;
+    const int i = (g.G + xi) + (g.G + yi) * (int)g.p.sy + (g.G + zi) * (int)g.p.sz;
+    split_store(S, h2, xi, yi, zi, view(dv, g.p.count, DK_F64_B, 0)[i]);
 }
 
 // ---------------------------------------------------------------------------
-// gaussSeidelSweep, project.go:103-130, with applyPressureBC folded in.
-// Before each colour the reference mirrors the interior into the ghosts
-// (project.go:89,93); a face ghost of a cell being updated then holds that
-// cell's own pre-update value, so the sweep reads the centre instead and the
-// ghosts are materialised once, after the last sweep (k_pressure_bc).
+// gaussSeidelSweep, project.go:103-130, with applyPressureBC folded in: the
+// split arrays' ghosts (see Split) always hold what the reference's mirror
+// before each colour would put there.
 // ---------------------------------------------------------------------------
-// EMU selects which of the update's six binary64 add/subtracts run on the
-// integer pipe (bit k: operation k of the chain, the subtraction last); the
-// others issue on the FP64 pipe.  Every choice computes the same bits.
-template <int EMU>
-__device__ __forceinline__ double chain_add(int k, double a, double b) {
-    return ((EMU >> k) & 1) ? dadd_int(a, b) : dadd(a, b);
-}
+// EMU selects which of the update's six binary64 additions (five, and the
+// subtraction last) run on the integer pipe (bit k: operation k of the
+// chain); the others issue on the binary64 pipe.  Every choice computes the
+// same bits.
+static __device__ __noinline__ double sub_div6_call(double a, double b) { return div6_int(dsub(a, b)); }
 
 template <int EMU>
-__global__ void k_rbgs_fp64(Geom g, double* __restrict__ p_, const double* __restrict__ bb_, int color,
-                            Status* st, int gate) {
+__device__ __forceinline__ double rb_update(double xm, double xp, double ym, double yp, double zm, double zp,
+                                            double b) {
+    const double v[5] = {xp, ym, yp, zm, zp};
+    double sum = xm;
+#pragma unroll
+    for (int k = 0; k < 5; ++k) sum = ((EMU >> k) & 1) ? dadd_int(sum, v[k]) : dadd(sum, v[k]);
+    if ((EMU >> 5) & 1) {
+        // The subtraction feeds the division unpacked.
+        exact::Sum s;
+        if (exact::add_sum(dbits(sum), dbits(b) ^ kSign, &s) && s.c == 0) return dfrom(exact::div6_sum(s));
+        return sub_div6_call(sum, b);
+    }
+    return div6_int(dsub(sum, b));
+}
+
+// A thread per cell of the colour, a plane's cells dealt out in order, which
+// keeps the warps of short and ragged rows full (a block per row measured the
+// same on long rows, blocks of 256 slower; several cells a thread along z,
+// unrolled or marching, are slower on every grid or on the small ones).  An
+// odd row's last slot of the colour it has one cell less of computes its
+// in-bounds neighbours too and drops the result, so warps do not diverge.
+// The sweeps touch scratch only, so they do not look at the fault gate: the
+// join does, before P is written.
+template <int EMU>
+__global__ void __launch_bounds__(128) k_rbgs_fp64(const __grid_constant__ Split S, int color) {
+    const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (t >= S.hx * S.NY) return;
+    const int y = (int)S.fhx.div((unsigned)t), j = t - y * S.hx, z = (int)blockIdx.y;
+    const int q = (color + S.G + y + z) & 1, x = 2 * j + q;
+    AF_PTR(double) own = view(S.p, 2 * S.pn, DK_F64_RBGS, 0) + (color ? S.pn : 0);
+    AF_PTR(double) opp = view(S.p, 2 * S.pn, DK_F64_RBGS, 0) + (color ? 0 : S.pn);
+    AF_PTR(const double) b = view((const double*)S.b, 2 * S.bn, DK_F64_RBGS, 0) + (color ? S.bn : 0);
+    const int i = (j + 1) + S.px * (y + 1) + S.plane * (z + 1);
+    pdl_wait();
+    // Of the two x neighbours one has the cell's own half index, the other
+    // the next (odd x) or the previous one; their sum does not depend on
+    // which is which.
+    const double r = rb_update<EMU>(opp[i], opp[q ? i + 1 : i - 1], opp[i - S.px], opp[i + S.px], opp[i - S.plane],
+                                    opp[i + S.plane], b[t + S.hx * S.NY * z]);
+    pdl_trigger();  // the next sweep's blocks get ready while this one's last ones finish
+    if (x >= S.NX) return;
+    own[i] = r;
+    if ((unsigned)(x - 1) >= (unsigned)(S.NX - 2) || (unsigned)(y - 1) >= (unsigned)(S.NY - 2) ||
+        (unsigned)(z - 1) >= (unsigned)(S.NZ - 2)) {  // a wall cell: its ghosts
+        if (x == 0) opp[i - 1] = r;
+        if (x == S.NX - 1) opp[q ? i + 1 : i] = r;
+        if (y == 0) opp[i - S.px] = r;
+        if (y == S.NY - 1) opp[i + S.px] = r;
+        if (z == 0) opp[i - S.plane] = r;
+        if (z == S.NZ - 1) opp[i + S.plane] = r;
+    }
+}
+
+// The split P into P: a ghost of the first layer holds the interior cell at
+// the clamped coordinates (applyPressureBC, project.go:139-163, composed),
+// the layers past it stay zero (project.go:81-83).
+__global__ void k_join_fp64(const __grid_constant__ Geom g, const __grid_constant__ Split S, double* p_, Status* st,
+                            int gate) {
     if (gated(st, gate)) return;
-    AF_PTR(double) AF_RESTRICT p = view(p_, g.p.count, DK_F64_RBGS, 0);
-    AF_PTR(const double) AF_RESTRICT bb = view(bb_, g.p.count, DK_F64_RBGS, 0);
-    const int G = g.G;
-    const int y = G + (int)(blockIdx.y * blockDim.y + threadIdx.y);
-    const int z = G + (int)blockIdx.z;
-    if (y >= G + g.NY) return;
-    const int start = (((G + y + z) & 1) != color) ? G + 1 : G;
-    const int x = start + 2 * (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    if (x >= G + g.NX) return;
-    const long long sy = g.p.sy, sz = g.p.sz;
-    const long long i = x + y * sy + z * sz;
-    const double pc = p[i];
-    const double xm = x > G ? p[i - 1] : pc;
-    const double xp = x < G + g.NX - 1 ? p[i + 1] : pc;
-    const double ym = y > G ? p[i - sy] : pc;
-    const double yp = y < G + g.NY - 1 ? p[i + sy] : pc;
-    const double zm = z > G ? p[i - sz] : pc;
-    const double zp = z < G + g.NZ - 1 ? p[i + sz] : pc;
-    double sum = chain_add<EMU>(0, xm, xp);
-    sum = chain_add<EMU>(1, sum, ym);
-    sum = chain_add<EMU>(2, sum, yp);
-    sum = chain_add<EMU>(3, sum, zm);
-    sum = chain_add<EMU>(4, sum, zp);
-    const double r = ((EMU >> 5) & 1) ? dsub_int(sum, bb[i]) : dsub(sum, bb[i]);
-    p[i] = div6_int(r);
+    const int x = blockIdx.x * blockDim.x + threadIdx.x - g.G;
+    const int y = blockIdx.y * blockDim.y + threadIdx.y - g.G;
+    const int z = (int)blockIdx.z - g.G;
+    if (x >= g.NX + g.G || y >= g.NY + g.G) return;
+    AF_PTR(double) p = view(p_, g.p.count, DK_F64_PBC, 0);
+    AF_PTR(const double) s = view((const double*)S.p, 2 * S.pn, DK_F64_PBC, 0);
+    double v = 0.0;
+    if (x >= -1 && x <= g.NX && y >= -1 && y <= g.NY && z >= -1 && z <= g.NZ) {
+        const int cx = min(max(x, 0), g.NX - 1), cy = min(max(y, 0), g.NY - 1), cz = min(max(z, 0), g.NZ - 1);
+        v = s[((cx + cy + cz + g.G) & 1 ? S.pn : 0) + ((cx >> 1) + 1 + S.px * (cy + 1) + S.plane * (cz + 1))];
+    }
+    p[(x + g.G) + (y + g.G) * (int)g.p.sy + (z + g.G) * (int)g.p.sz] = v;
 }
 
 // applyPressureBC, project.go:139-163 (see pbc_cell).
@@ -493,20 +560,6 @@ __global__ void k_gradient_fp64(Geom g, const double* __restrict__ p, double* __
 }
 
 __global__ void k_step_tick(Status* st) { st->step += 1; }
-
-// B = h2*Div over the interior, for the red-black phase hook when Div was
-// supplied directly instead of by the divergence kernel.
-__global__ void k_b_from_div(Geom g, const double* __restrict__ dv_, double* __restrict__ bb_, double h2) {
-    const int G = g.G;
-    AF_PTR(const double) AF_RESTRICT dv = view(dv_, g.p.count, DK_F64_B, 0);
-    AF_PTR(double) AF_RESTRICT bb = view(bb_, g.p.count, DK_F64_B, 0);
-    const int x = G + (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    const int y = G + (int)(blockIdx.y * blockDim.y + threadIdx.y);
-    const int z = G + (int)blockIdx.z;
-    if (x >= G + g.NX || y >= G + g.NY) return;
-    const long long i = x + y * g.p.sy + z * g.p.sz;
-    bb[i] = dmul(h2, dv[i]);
-}
 
 // ---------------------------------------------------------------------------
 // Diagnostics.  A max is exact in any order; NaN is skipped as the
@@ -830,40 +883,48 @@ void launch_maccormack_fp64(const Geom& g, int axis, const Fields& f, const Fiel
     else k_maccormack_fp64<2><<<grid, block, 0, s>>>(a, fwd.t0, fwd.t1, fwd.t2);
 }
 
-void launch_divergence_fp64(const Geom& g, const Fields& f, double* b, double scale, double h2, bool zero_p,
-                            Status* st, int gate, cudaStream_t s) {
-    dim3 block(64, 4);
-    dim3 grid(cdiv(g.p.nx, 64), cdiv(g.p.ny, 4), g.p.nz);
-    k_divergence_fp64<<<grid, block, 0, s>>>(g, f.u, f.v, f.w, f.p, f.div, b, exact::mul_const(scale),
-                                             exact::mul_const(h2), zero_p ? 1 : 0, st, gate);
+void launch_divergence_fp64(const Geom& g, const Fields& f, const Split* split, double scale, double h2, Status* st,
+                            int gate, cudaStream_t s) {
+    const dim3 block(32, 8), grid(cdiv(g.NX, 32), cdiv(g.NY, 8), g.NZ);
+    k_divergence_fp64<<<grid, block, 0, s>>>(g, f.u, f.v, f.w, f.div, split ? *split : Split{}, split ? 1 : 0,
+                                             exact::mul_const(scale), exact::mul_const(h2), st, gate);
 }
 
-// Integer-pipe share of the red-black chain: AEROFLUX_RBGS_EMU picks the
-// mask.  Measured on GB300 at 256^3, every emulated add slows the update
-// (all six native: 41 ms per 200-pair projection; all six emulated: 146 ms),
-// so the default keeps the adds on the FP64 pipe; the exact /6 stays on the
-// integer pipe, where it wins over its three-operation FP64 sequence.
+void launch_split_from_div(const Geom& g, const double* div, const Split& split, double h2, cudaStream_t s) {
+    const dim3 block(32, 8), grid(cdiv(g.NX, 32), cdiv(g.NY, 8), g.NZ);
+    k_split_from_div<<<grid, block, 0, s>>>(g, div, split, exact::mul_const(h2));
+}
+
+// Integer-pipe share of the red-black chain.  Of the update's six additions
+// the first and the last (the subtraction, which feeds the division unpacked)
+// run there: at 256^3 a launch takes 101 us with none, 86 with either, 77
+// with both -- both pipes then about 70 % busy -- 88 with a third and 140
+// with all six (the logic pipe bounds).  AEROFLUX_RBGS_EMU picks another mask
+// for measurements.
 static int rbgs_emu_mask() {
-    static int m = -1;
-    if (m < 0) {
+    static const int m = [] {
         const char* v = getenv("AEROFLUX_RBGS_EMU");
-        m = v ? atoi(v) : 0x00;
-    }
+        return v ? atoi(v) : 0x21;
+    }();
     return m;
 }
 
-void launch_rbgs_fp64(const Geom& g, double* p, const double* b, int color, Status* st, int gate, cudaStream_t s) {
-    dim3 block(32, 4);
-    dim3 grid(cdiv((g.NX + 1) / 2, 32), cdiv(g.NY, 4), g.NZ);
+void launch_rbgs_fp64(const Split& split, int color, cudaStream_t s) {
+    const dim3 grid(cdiv((long long)split.hx * split.NY, 128), split.NZ);
+    void (*k)(const Split, int) = k_rbgs_fp64<0x3F>;
     switch (rbgs_emu_mask()) {
-    case 0x00: k_rbgs_fp64<0x00><<<grid, block, 0, s>>>(g, p, b, color, st, gate); break;
-    case 0x01: k_rbgs_fp64<0x01><<<grid, block, 0, s>>>(g, p, b, color, st, gate); break;
-    case 0x05: k_rbgs_fp64<0x05><<<grid, block, 0, s>>>(g, p, b, color, st, gate); break;
-    case 0x15: k_rbgs_fp64<0x15><<<grid, block, 0, s>>>(g, p, b, color, st, gate); break;
-    case 0x2A: k_rbgs_fp64<0x2A><<<grid, block, 0, s>>>(g, p, b, color, st, gate); break;
-    case 0x35: k_rbgs_fp64<0x35><<<grid, block, 0, s>>>(g, p, b, color, st, gate); break;
-    default: k_rbgs_fp64<0x3F><<<grid, block, 0, s>>>(g, p, b, color, st, gate); break;
+    case 0x00: k = k_rbgs_fp64<0x00>; break;
+    case 0x01: k = k_rbgs_fp64<0x01>; break;
+    case 0x20: k = k_rbgs_fp64<0x20>; break;
+    case 0x21: k = k_rbgs_fp64<0x21>; break;
+    case 0x23: k = k_rbgs_fp64<0x23>; break;
     }
+    launch_pdl(k, grid, dim3(128), 0, s, split, color);
+}
+
+void launch_join_fp64(const Geom& g, const Split& split, double* p, Status* st, int gate, cudaStream_t s) {
+    const dim3 block(64, 4), grid(cdiv(g.p.nx, 64), cdiv(g.p.ny, 4), g.p.nz);
+    k_join_fp64<<<grid, block, 0, s>>>(g, split, p, st, gate);
 }
 
 void launch_pressure_bc_fp64(const Geom& g, double* p, Status* st, int gate, cudaStream_t s) {
@@ -879,12 +940,6 @@ void launch_gradient_fp64(const Geom& g, const Fields& f, double scale, Status* 
 }
 
 void launch_step_tick(Status* st, cudaStream_t s) { k_step_tick<<<1, 1, 0, s>>>(st); }
-
-void launch_b_from_div(const Geom& g, const double* div, double* b, double h2, cudaStream_t s) {
-    dim3 block(64, 4);
-    dim3 grid(cdiv(g.NX, 64), cdiv(g.NY, 4), g.NZ);
-    k_b_from_div<<<grid, block, 0, s>>>(g, div, b, h2);
-}
 
 void launch_max_divergence(const Geom& g, const double* u, const double* v, const double* w, double invH,
                            unsigned long long* out, cudaStream_t s) {

@@ -23,6 +23,56 @@ struct Geom {
     Dims p, u, v, w;     // P (= Div shape), U (= Tmp0), V (= Tmp1), W (= Tmp2)
 };
 
+// Unsigned 32-bit division by an invariant divisor with one multiply-high
+// (Granlund & Montgomery, "Division by invariant integers using
+// multiplication", 1994): l = ceil(log2 d), m = ceil(2^(32+l)/d) - 2^32,
+// n/d = (umulhi(n, m) + n) >> l for every n < 2^32.
+struct FastDiv {
+    unsigned d = 1, m = 0, l = 0;
+    FastDiv() = default;
+    __host__ explicit FastDiv(unsigned div) : d(div) {
+        while ((1ull << l) < d) ++l;
+        m = (unsigned)((((1ull << (32 + l)) + d - 1) / d) - (1ull << 32));
+    }
+    __device__ __forceinline__ unsigned div(unsigned n) const {
+        return (unsigned)(((unsigned long long)__umulhi(n, m) + n) >> l);
+    }
+};
+
+// Scratch of the red-black solver: P and B = h^2 Div split by colour, so a
+// colour's update reads and writes contiguous cells and touches no cell it
+// does not need.  Colour c holds the interior cells (x, y, z) with
+// x + y + z + G = c (mod 2), at half index x >> 1.  P rows carry one ghost
+// cell on every side (pitch px = hx + 2, NY + 2 rows, NZ + 2 planes per
+// colour); a wall cell's ghost lies in the other colour's array, where its
+// update writes its new value too (applyPressureBC, project.go:139-163:
+// before a cell is updated its face ghosts hold the cell's own value).
+// B holds the interior only (pitch hx).
+struct Split {
+    int NX, NY, NZ, G;
+    int hx, px, plane;      // (NX+1)/2, hx + 2, px * (NY + 2)
+    long long pn, bn;       // elements per colour of p and b
+    double* p;
+    double* b;
+    FastDiv fhx;
+    static Split of(const Geom& g) {
+        Split s{};
+        s.NX = g.NX, s.NY = g.NY, s.NZ = g.NZ, s.G = g.G;
+        s.hx = (g.NX + 1) / 2;
+        s.px = s.hx + 2;
+        s.plane = s.px * (g.NY + 2);
+        s.pn = (long long)s.plane * (g.NZ + 2);
+        s.bn = (long long)s.hx * g.NY * g.NZ;
+        s.fhx = FastDiv((unsigned)s.hx);
+        return s;
+    }
+    size_t bytes() const { return (size_t)(2 * pn + 2 * bn) * sizeof(double); }
+    void place(void* mem) {
+        p = (double*)mem;
+        b = p + 2 * pn;
+    }
+};
+
 // Device status block of one engine.
 //  fault_gate: step*8 + sweep phase (0..5) of the first contained fault,
 //              0xFFFFFFFF when none.  Every kernel of a later phase returns at
@@ -56,6 +106,34 @@ struct Fields {
     double* t2;
 };
 
+// Launches a kernel that may be scheduled while its predecessor in the stream
+// still runs (programmatic dependent launch): the kernel waits for it with
+// pdl_wait() before it touches anything an earlier kernel wrote or reads.
+// Every kernel launched so calls pdl_wait() in every block that does work;
+// then a kernel that follows finds all earlier ones finished too.  Measured
+// for the red-black sweeps, us per launch: 16^3 2.01 -> 1.76, 64^3 3.26 ->
+// 2.79, 128^3 11.5 -> 11.0, 256^3 79.1 -> 77.8; with the trigger at the
+// kernel's start, where the early blocks take residency from the running
+// ones, 64^3 3.54.
+template <class... P, class... A>
+void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+#if defined(__CUDACC__)
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+#endif
+
 // --- FP64 plain-form stage launchers (af_fp64.cu) ---------------------------
 // `gate` is the step-relative phase index a kernel belongs to: it returns at
 // entry when a fault was recorded at an earlier (step, phase).
@@ -67,15 +145,20 @@ void launch_sweep_fp64(const Geom& g, int axis, const Fields& f, double dt, doub
 // directional diffusion into f.t0..t2.  Two launches.
 void launch_maccormack_fp64(const Geom& g, int axis, const Fields& f, const Fields& fwd, double dt, double invH,
                             double lam, Status* st, int phase, cudaStream_t s);
-// zero_p also zeroes all of P, as solvePressureRedBlack does first (project.go:81-83).
-void launch_divergence_fp64(const Geom& g, const Fields& f, double* b, double scale, double h2, bool zero_p,
-                            Status* st, int gate, cudaStream_t s);
-void launch_rbgs_fp64(const Geom& g, double* p, const double* b, int color, Status* st, int gate,
-                      cudaStream_t s);
+// computeDivergence into Div (project.go:42-62); with split, also B into it
+// and its P zeroed for the red-black sweeps (project.go:81-83).
+void launch_divergence_fp64(const Geom& g, const Fields& f, const Split* split, double scale, double h2, Status* st,
+                            int gate, cudaStream_t s);
+// B and zero P of the red-black sweeps from a Div supplied directly.
+void launch_split_from_div(const Geom& g, const double* div, const Split& split, double h2, cudaStream_t s);
+// One colour sweep over the split arrays (scratch only: not gated).
+void launch_rbgs_fp64(const Split& split, int color, cudaStream_t s);
+// The split P back into P, with applyPressureBC's ghosts; cells no one
+// writes (ghost layers past the first) are zero.
+void launch_join_fp64(const Geom& g, const Split& split, double* p, Status* st, int gate, cudaStream_t s);
 void launch_pressure_bc_fp64(const Geom& g, double* p, Status* st, int gate, cudaStream_t s);
 void launch_gradient_fp64(const Geom& g, const Fields& f, double scale, Status* st, int gate, cudaStream_t s);
 void launch_step_tick(Status* st, cudaStream_t s);
-void launch_b_from_div(const Geom& g, const double* div, double* b, double h2, cudaStream_t s);
 
 // Diagnostics (af_fp64.cu).  `out` receives the bit pattern of a
 // non-negative double (max) or the fixed-order sum; `scratch` holds one

@@ -1,4 +1,4 @@
-"""The integer forms of binary64 products and interpolation weights
+"""The integer forms of binary64 products, sums and interpolation weights
 (csrc/af_exact.cuh) against the native operations, bit for bit, on the CPU:
 the header compiles as plain C++ there."""
 import os
@@ -36,7 +36,7 @@ static double draw(int lo, int hi) {
 
 int main(int argc, char** argv) {
     const long n = atol(argv[1]);
-    long bad = 0, products = 0, feet = 0, cells = 0;
+    long bad = 0, products = 0, feet = 0, cells = 0, sums = 0;
     for (long i = 0; i < n; ++i) {  // constant times anything, extremes, zero and NaN included
         const double c = fabs(draw(1, 2046)), x = i % 64 ? draw(0, 2047) : (i % 128 ? 0.0 : -0.0);
         const double got = mulc(mul_const(c), x), want = c * x;
@@ -75,12 +75,34 @@ int main(int argc, char** argv) {
         if (t != 0.0) bad += bits_of(weight_mul(w.t, w.te, d)) != bits_of(d * t);
         bad += bits_of(weight_mul(w.o, w.oe, d)) != bits_of(d * o);
     }
-    printf("%ld %ld %ld %ld\n", bad, products, feet, cells);
+    for (long i = 0; i < n; ++i) {  // sums: any exponents, near ones, near cancellation, ties, zero, extremes
+        const double a = draw(i % 4 ? 40 : 0, i % 4 ? 2046 : 2047);
+        const u64 ab = bits_of(a), ea = exp_field(ab);
+        double b;
+        switch (rng() % 6) {
+        case 0: b = draw(0, 2047); break;
+        case 1: b = draw(ea > 40 ? (int)ea - 40 : 0, ea < 2007 ? (int)ea + 40 : 2047); break;
+        case 2: b = from_bits((ab ^ ((rng() & 1) << 63)) + (rng() & 0xFFF) - 0x800); break;
+        case 3: b = from_bits((ab ^ ((rng() & 1) << 63)) + ((rng() & 0xFFF) << 30) - (0x800ull << 30)); break;
+        case 4: b = from_bits(((rng() & 1) << 63) | ((ea > 60 ? ea - 50 - rng() % 6 : ea) << 52) | (rng() & 0xF)); break;
+        default: b = rng() % 2 ? -a : (rng() % 2 ? 0.0 : -0.0);
+        }
+        Sum s;
+        if (add_sum(ab, bits_of(b), &s)) {
+            ++sums;
+            bad += pack_sum(s) != bits_of(a + b);
+        }
+        if (add_sum(ab, bits_of(b) ^ kSignBit, &s)) {
+            bad += pack_sum(s) != bits_of(a - b);
+            if (s.c == 0) bad += div6_sum(s) != bits_of((a - b) / 6.0);
+        }
+    }
+    printf("%ld %ld %ld %ld %ld\n", bad, products, feet, cells, sums);
 }
 """
 
 
-def test_integer_products_and_weights_equal_the_native_ones(tmp_path):
+def test_integer_forms_equal_the_native_operations(tmp_path):
     cxx = shutil.which("g++") or shutil.which("c++")
     if not cxx:
         pytest.skip("no C++ compiler")
@@ -88,7 +110,7 @@ def test_integer_products_and_weights_equal_the_native_ones(tmp_path):
     src.write_text(MAIN)
     subprocess.run([cxx, "-O2", "-ffp-contract=off", "-I", CSRC, str(src), "-o", str(exe)], check=True)
     n = 3_000_000
-    bad, products, feet, cells = (int(v) for v in subprocess.run([str(exe), str(n)], check=True, capture_output=True,
+    bad, products, feet, cells, sums = (int(v) for v in subprocess.run([str(exe), str(n)], check=True, capture_output=True,
                                                                  text=True).stdout.split())
     assert bad == 0
-    assert products == n and feet > n // 4 and cells > n // 4  # the integer forms took them
+    assert products == n and feet > n // 4 and cells > n // 4 and sums > n // 3  # the integer forms took them
