@@ -57,7 +57,13 @@ struct Lvl {
     FastDiv ftx;            // fused-pair wide tiles along x
     FastDiv fty[3];         // fused-pair tiles along y, per tile variant (kPairVarTY)
     int nxw;                // 64 x the wide pair tiles along x; a narrow tile column covers nxw .. nx-1
-    int tma;                // 1: the level's e, e2, r have tensor maps (the TMA-staged pair may run on it)
+    // Marching pair (kb_smooth_march), per block size (kMarchT): the quads of
+    // a tile column (0 when the level cannot run it) and of its loaded rows,
+    // the output rows of a tile, the tile columns and the tiles along y.
+    struct March {
+        int w, q, rows;
+        FastDiv fq, fcol, fty;
+    } march[3];
 };
 
 struct Ctl {
@@ -102,7 +108,6 @@ struct InstDev {
     int shp[3];              // row pitch of each shadow (floats): its padded x extent rounded up to 4
     int shq[4];              // shadow conversion: prefix of the components' (row, quad) counts
     FastDiv fsq[3];          // quads per shadow row
-    const CUtensorMap* pmap; // 3 tensor maps per level for the TMA-staged pair: e, e2 and r
     const CUtensorMap* tmap; // 12 tensor maps over the shadows: [component][role], role 0-2 the staged
                              // tile of a sweep along axis 0-2, role 3 the axis-velocity tile
     int sw_tiles;            // staged sweep: work items (3 components x the spatial tiles)
@@ -123,7 +128,8 @@ enum {
     S_PAIR = S_BIGCOARSE + kMaxLev,
     S_PAIRN = S_PAIR + kMaxLev,
     S_SWEEPT = S_PAIRN + kMaxLev,
-    S_COUNT = S_SWEEPT + 1
+    S_MARCH = S_SWEEPT + 1,
+    S_COUNT = S_MARCH + kMaxLev
 };
 
 struct Shape {
@@ -874,7 +880,11 @@ __device__ __forceinline__ long long lidx(int x, int y, int z, int nx, int ny) {
 // to max|div| <= 1e-10 per projection at 256^3: 8 at omega = 1, 6 at 1.3,
 // 5 at 1.5, 7 at 1.6).
 constexpr float kMgOmega = 1.5f;
-__device__ __forceinline__ float mg_relax(const Lvl& L, float sx, float sy, float sz, float r, float inv, float c) {
+struct MgW {  // a level's weights
+    float wx, wy, wz;
+};
+template <class LevelOrWeights>
+__device__ __forceinline__ float mg_relax(const LevelOrWeights& L, float sx, float sy, float sz, float r, float inv, float c) {
     const float v = __fmul_rn(__fsub_rn(__fmaf_rn(L.wz, sz, __fmaf_rn(L.wy, sy, __fmul_rn(L.wx, sx))), r), inv);
     return __fmaf_rn(kMgOmega, __fsub_rn(v, c), c);
 }
@@ -1171,11 +1181,12 @@ __device__ float block_sum(float v, float* red) {
 // red cells at 16 x 8 rows and planes, 1.9x at 8 x 4, 2.3x at 4 x 4) against
 // parallelism: a 64^3 level holds 32 of the largest tiles for 152 SMs.  The
 // autotuner picks a variant per level; untuned, the level's size does.
-// Variant 3 is the TMA-staged z-marching pair (kb_smooth_pair_zm): 64 x 16
-// columns of 16 planes.
+// Variant 3 is the marching pair (kb_smooth_march) on the slots whose level
+// allows it.
 // Variant 4: 64 x 16 x 16 tiles, the red halo recomputed over 1.27x the
 // tile's red cells.
-constexpr int kPairVarTY[5] = {16, 8, 4, 16, 16}, kPairVarTZ[5] = {8, 4, 4, 16, 16};
+constexpr int kPairVarTY[5] = {16, 8, 4, 0, 16}, kPairVarTZ[5] = {8, 4, 4, 0, 16};
+constexpr int kPairTileVars[4] = {0, 1, 2, 4};
 constexpr int kPairWideX = 64;
 
 template <int LANES, int V>
@@ -1274,298 +1285,187 @@ __global__ void __launch_bounds__(PairTile<LANES, V>::THREADS, PairTile<LANES, V
     }
 }
 
-// --- TMA-staged, z-marching fused pair -----------------------------------------
-// The red-black pair of kb_smooth_pair on 64 x 16 columns of ZC planes,
-// marching along z with its inputs in shared-memory rings filled by TMA
-// plane loads (e_in planes of the column plus a two-cell ring, r planes plus
-// a one-cell ring).  Step k computes the red cells of halo plane z0-1+k (the
-// tile's rows plus one on each side) into a ring of red planes, then the
-// black cells of plane z0-2+k from the three red planes around it.  The red
-// halo is recomputed only across the column's sides and the chunk's two end
-// planes (1.3x the tile's red cells at ZC = 16), not around every 3-D tile.
+// --- marching fused pair -----------------------------------------------------
+// The red-black pair of kb_smooth_pair with each thread owning a quad (four
+// consecutive cells of a row, two red and two black on every plane) and
+// marching along z with its column of e, r and red values in registers: a
+// plane costs a quad 16-byte loads of e two planes ahead, of r one plane
+// ahead and of the two rows beside it, one scalar across the quad's end, and
+// one 16-byte store.  Red values of a plane are exchanged with the rows and
+// quads beside it through a two-plane ring in shared memory, so there is one
+// barrier a plane: while a block computes the red cells of plane z, it
+// computes the black ones of plane z - 1, whose neighbours' red cells the
+// last barrier published.
 //
-// Walls cost no per-cell work.  The e ring holds, for the planes z0-2+p, the
-// plane clamped into the level (the plane beyond a z wall is the wall plane
-// loaded again), and once a plane lands, the cells just beyond an x or y wall
-// are overwritten with the wall cell they face.  So every neighbour of an
-// in-level red cell is read at a fixed offset and is exactly the value
-// kb_smooth_pair uses (at a wall: the cell's own).  A red position just
-// outside the level takes the old value stored there, i.e. the wall cell it
-// faces, which is the value the black cell beside it uses for its wall
-// neighbour: the black pass needs no selects either.  Arithmetic and operand
-// order are those of kb_smooth_pair: the same bits.
+// A tile is a column of at most kMarchQ quads by March::rows rows; its block
+// also computes the red cells of the row on either side, of the quad on
+// either side where the level has several columns, and of the plane on
+// either side of its z chunk.  Walls cost no selects: a row or plane outside
+// the level stands in with the row or plane of the wall cells it faces, and
+// its "red" values are their old ones, which is what the black cells beside
+// it use.  Operands and their order are those of kb_smooth_pair: the same
+// bits.
 //
-// Every thread keeps its rows for the whole column: warp w of 18 computes
-// the red cells of halo row w (warp 16 also the rows' 33rd cells) and warps
-// 0-15 the black cells of tile row w.  Plane loads run five steps ahead; a
-// plane's loads are waited one step before it is first read, so its wall
-// fix-up is published by the step's one block barrier.
+// A plane's operands load into the registers that the plane before has just
+// used, between its red and its black cells: no copy waits for a load, and
+// the loads have the black cells, the barrier and the other warps to land.
 //
-// A level runs it only when its rows and arrays are 16-byte aligned (nx a
-// multiple of 4; InstDev::pmap, Lvl::tma).  Boxes start at x0 - 4, a 16-byte
-// boundary; box cells outside the level load as zeros and are never read.
-constexpr int kZmTX = 64, kZmTY = 16, kZmZC = 16, kZmBX = 72;
-static_assert(kPairVarTY[3] == kZmTY && kPairVarTZ[3] == kZmZC, "work-list tiles of pair variant 3");
-constexpr int kZmEY = kZmTY + 4, kZmRY = kZmTY + 2;     // e rows: tile + 2 each side; r and red rows: + 1
-constexpr int kZmNE = 8, kZmNR = 8, kZmNRed = 4, kZmLead = 5, kZmNB = 8;
-constexpr int kZmEBox = kZmBX * kZmEY, kZmRBox = kZmBX * kZmRY;  // floats one plane load delivers
-// Ring slots of e and r planes start on 128-byte boundaries (the rule for a
-// TMA tensor load's shared-memory destination): plane pitches round up to 32 floats.
-constexpr int kZmEPlane = (kZmEBox + 31) / 32 * 32, kZmRPlane = (kZmRBox + 31) / 32 * 32;
-constexpr int kZmRedPlane = kZmRY * 33;
-constexpr int kZmROff = kZmNE * kZmEPlane, kZmRedOff = kZmROff + kZmNR * kZmRPlane;  // ring offsets (floats)
-constexpr int kZmFloats = kZmRedOff + kZmNRed * kZmRedPlane;
-// 18 warps: warp w computes red halo row w, warps 0-15 also the black cells
-// of tile row w and warp 16 the rows' 33rd red cells, so no warp does more
-// than two row passes between the march's barriers.  Two blocks per SM keep
-// every per-thread offset of the column in registers (with fewer, the
-// compiler re-derives them from the thread index at every step).
-constexpr int kZmWarps = kZmRY;
-constexpr int kZmThreads = kZmWarps * 32;
-constexpr int kZmBlocks = 2;
-constexpr size_t kZmSmem = (size_t)kZmFloats * sizeof(float);
-// Ring sizes for a lead of kZmLead groups with each group waited one step
-// before its first read (a slot is rewritten only after its last reader).
-static_assert(kZmNE >= kZmLead + 3 && kZmNR >= kZmLead + 2 && kZmNB > kZmLead, "ring sizes of the z-march");
-// The march is unrolled by 8 steps, so every ring slot, red plane and
-// barrier of a step is a compile-time constant.
-static_assert(kZmNE == 8 && kZmNR == 8 && kZmNB == 8 && kZmNRed == 4, "ring sizes of the unrolled march");
-static_assert(kZmEPlane % 32 == 0 && kZmRPlane % 32 == 0 && kZmROff % 32 == 0,
-              "TMA destinations of the z-march rings on 128-byte boundaries");
+// A warp waits for the other warps' red cells of the last plane, not of this
+// one, on a barrier that splits arriving from waiting (a block-wide barrier a
+// plane left the block idle half the time: 57 us instead of 41 at 256^3).
+//
+// A level runs it when rows and arrays are 16-byte aligned (nx a multiple
+// of 4).  Measured per pair against the best tiles, us: finest levels of
+// 512^3 541 -> 323 and 256^3 69 -> 41 (39 of them on the device, 200 MB at
+// 5 TB/s, issue 60 % active), 128^3 14.7 -> 12.6, the 256-grid batch 504 ->
+// 250.  Block sizes: 1024 threads on 64 quads (one block an SM) for long
+// rows, two of 576 on 32 quads for many middling ones, four of 256 for small
+// levels; prefetching further planes to L2 gained nothing.
+constexpr int kMarchT[3] = {256, 576, 1024}, kMarchQ[3] = {16, 32, 64}, kMarchBlocks[3] = {4, 2, 1};
+// Launch shapes the autotuner tries: block size (index into kMarchT) and
+// planes of a z chunk.
+struct MarchShape {
+    int k, zc;
+};
+constexpr MarchShape kMarchShapes[] = {{0, 4}, {0, 8}, {0, 16}, {1, 8}, {1, 16}, {1, 32}, {2, 16}, {2, 32}};
+constexpr int kMarchShapeCount = sizeof kMarchShapes / sizeof kMarchShapes[0];
 
-// Shared-memory access of the z-march: byte addresses with compile-time
-// offsets ([addr + imm]), so a neighbour costs no address arithmetic.  The
-// bounds-checking build indexes the checked ring view instead.
-#if AEROFLUX_DEBUG_BOUNDS
-using ZmAddr = int;  // float index into the rings
-#define ZM_A(i) (i)
-#define ZM_LD(a, off) S[(a) + (off)]
-#define ZM_ST(a, v) (S[(a)] = (v))
-constexpr int kZmB = 1;  // address units per float
-#else
-using ZmAddr = unsigned;  // shared-window byte address
-template <int OFF>
-__device__ __forceinline__ float zm_lds(unsigned a) {
-    float v;
-    asm volatile("ld.shared.f32 %0, [%1+%2];" : "=f"(v) : "r"(a), "n"(OFF) : "memory");
-    return v;
+__device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
-__device__ __forceinline__ void zm_sts(unsigned a, float v) {
-    asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
-}
-#define ZM_A(i) (sb + 4u * (unsigned)(i))
-#define ZM_LD(a, off) zm_lds<4 * (off)>(a)
-#define ZM_ST(a, v) zm_sts((a), (v))
-constexpr int kZmB = 4;
-#endif
-
-template <int ZC>
-__global__ void __launch_bounds__(kZmThreads, kZmBlocks)
-    kb_smooth_pair_zm(const InstDev* inst, const Ctl* ctl, Tab tab, int l, int dir, int vc, unsigned* diag) {
-    if (vc_idle(ctl, tab.n, vc)) return;
-    extern __shared__ __align__(128) float zsm[];
-    __shared__ __align__(8) unsigned long long bar[kZmNB];
-    __shared__ unsigned stop;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const unsigned sb = smem_addr(zsm);
-    if (sb & 127u) {  // the rings' TMA destinations need a 128-byte aligned base
-        if (tid == 0) atomicOr(diag, 4u);
-        return;
+// Waits for the block's own warps only, all resident and none of them waiting
+// for anything else; bounded all the same.
+__device__ __forceinline__ void march_wait(unsigned long long* bar, unsigned parity) {
+    for (unsigned it = 0; it < kSwSpinLimit && !mbar_try_wait(bar, parity); ++it) {
     }
+}
+
+template <int K>
+__global__ void __launch_bounds__(kMarchT[K], kMarchBlocks[K])
+    kb_smooth_march(const InstDev* inst, const Ctl* ctl, Tab tab, int l, int dir, int vc, int zc) {
+    if (vc_idle(ctl, tab.n, vc)) return;
+    constexpr int T = kMarchT[K];
+    __shared__ float2 ring[4][T];
+    __shared__ __align__(8) unsigned long long bar[2];
+    const int tid = threadIdx.x;
     if (tid == 0) {
-        for (int i = 0; i < kZmNB; ++i) mbar_init(&bar[i], 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        stop = diag_set(diag) ? 1u : 0u;
+        mbar_init(&bar[0], T / 32);
+        mbar_init(&bar[1], T / 32);
     }
     __syncthreads();
-    if (stop) return;
-    // Group k of a column completes on barrier k % 8; bit b of `phase` is
-    // the parity barrier b completes next (every thread waits every group).
-    unsigned phase = 0;
+    unsigned n = 0;  // planes this block has marched over
     for (int item = blockIdx.x, total = tab.prefix[tab.n]; item < total; item += gridDim.x) {
         const int s = find_slot(tab.prefix, tab.n, item);
         if (mg_off(ctl[s], vc)) continue;
-        const Lvl L = inst[s].lev[l];
-        if (!L.tma) {  // the host switches the stage off this variant first; never stage through an unset map
-            if (tid == 0) atomicOr(diag, 2u);
-            continue;
-        }
-        AF_PTR(float) S = view(zsm, (long long)kZmFloats, DK_PAIR, s);  // the three rings
-        (void)S;
+        const Lvl& L = inst[s].lev[l];
+        AF_PTR(const float) AF_RESTRICT ein = view((const float*)(dir ? L.e2 : L.e), lvl_cells(L), DK_PAIR, s);
         AF_PTR(float) AF_RESTRICT eout = view(dir ? L.e : L.e2, lvl_cells(L), DK_PAIR, s);
-        const int nx = L.nx, ny = L.ny, nz = L.nz;
-        const unsigned local = (unsigned)(item - tab.prefix[s]);
-        const unsigned q1 = L.ftx.div(local), q2 = L.fty[0].div(q1);
-        const int x0 = (int)(local - q1 * L.ftx.d) * kZmTX;
-        const int y0 = (int)(q1 - q2 * L.fty[0].d) * kZmTY;
-        const int z0 = (int)q2 * ZC;
-        const int K = min(ZC, nz - z0);  // black planes z0 .. z0+K-1; steps 0 .. K+1
-        // Group k: e plane z0+k into ring plane p = k+2 and r plane z0-1+k
-        // into r slot k % kZmNR, when needed; group 0 also brings ring
-        // planes 0 and 1 (z0-2, z0-1).  A plane just beyond a z wall loads
-        // the wall plane; one further out is never read and not loaded.
-        auto issue = [&](int k) {
-            unsigned long long* b = &bar[k & 7];
-            const int pa = k == 0 ? 0 : k + 2, pb = k + 2;
-            int ne = 0;
-            for (int p = pa; p <= pb; ++p) ne += (z0 - 2 + p >= -1 && z0 - 2 + p <= nz) ? 1 : 0;
-            const int rz = z0 - 1 + k;
-            const bool rr = rz >= 0 && rz < nz;
-            mbar_expect_tx(b, (unsigned)((ne * kZmEBox + (rr ? kZmRBox : 0)) * sizeof(float)));
-            const CUtensorMap* em = inst[s].pmap + 3 * l + dir;
-            for (int p = pa; p <= pb; ++p) {
-                const int z = z0 - 2 + p;
-                if (z >= -1 && z <= nz)
-                    tma_load_3d(zsm + (p & 7) * kZmEPlane, em, x0 - 4, y0 - 2, min(max(z, 0), nz - 1), b);
-            }
-            if (rr) tma_load_3d(zsm + kZmROff + (k & 7) * kZmRPlane, inst[s].pmap + 3 * l + 2, x0 - 4, y0 - 1, rz, b);
-        };
-        // Wall fix-up of a landed e plane: the cell beyond an x or y wall
-        // takes the wall cell's value (box column 4 is x = x0, box row 2 is
-        // y = y0).  Only cells beside an in-level cell matter; the corners
-        // two walls share are never read.
-        const int wx0 = x0 == 0, wx1 = x0 + kZmTX >= nx, wy0 = y0 == 0, wy1 = y0 + kZmRY - 1 >= ny;
-        const bool walls = wx0 | wx1 | wy0 | wy1;
-        const int gx = nx - x0 + 4, gy = ny - y0 + 2;  // box column of x = nx, box row of y = ny
-        auto fill = [&](int slot) {
-            const int P = slot * kZmEPlane;
-            if (tid < kZmEY) {
-                const ZmAddr r = ZM_A(P + tid * kZmBX);
-                if (wx0) ZM_ST(r + 3 * kZmB, ZM_LD(r, 4));
-                if (wx1) ZM_ST(r + gx * kZmB, ZM_LD(r + (gx - 1) * kZmB, 0));
-            } else if (tid >= 32 && tid < 32 + kZmBX) {
-                const ZmAddr c = ZM_A(P + tid - 32);
-                if (wy0) ZM_ST(c + kZmBX * kZmB, ZM_LD(c, 2 * kZmBX));
-                if (wy1) ZM_ST(c + gy * kZmBX * kZmB, ZM_LD(c + (gy - 1) * kZmBX * kZmB, 0));
-            }
-        };
+        AF_PTR(const float) AF_RESTRICT r = view((const float*)L.r, lvl_cells(L), DK_PAIR, s);
+        const int nx = L.nx, ny = L.ny, nz = L.nz, nxy = nx * ny, mq = L.march[K].q, mw = L.march[K].w;
+        const int mrows = L.march[K].rows;
+        const MgW W{L.wx, L.wy, L.wz};
         const float inv = 1.0f / (2.0f * (L.wx + L.wy + L.wz));
-        // Red cells of this thread: cell `lane` of halo row `warp`, and for
-        // warp 16 also cell 32 of halo row lane % 18 (lanes 18-31 repeat
-        // lanes 0-13: the same value to the same place).  Per cell: e offset
-        // for parity 0, red offset, level row + 1, level x for parity 0.
-        const bool xe = warp == kZmTY;
-        const int hyB = lane % kZmRY, jB = 32;
-        const int eA = (warp + 1) * kZmBX + 3 + 2 * lane, eB = (hyB + 1) * kZmBX + 3 + 2 * jB;
-        const int dA = warp * 33 + lane, dB = hyB * 33 + jB;
-        const int yA = y0 + warp, yB = y0 + hyB;  // level row + 1
-        const int xA = x0 - 1 + 2 * lane, xB = x0 - 1 + 2 * jB;
-        // Black cells of this thread (warps 0-15): tile row `warp`, pair
-        // x0 + 2 lane, +1; computed by every lane, stored where in the level.
-        const bool bw = warp < kZmTY;
-        const int by = y0 + warp;
-        const bool bok = by < ny && x0 + 2 * lane < nx;
-        const int ebk = (warp + 2) * kZmBX + 2 * lane + 5;  // e offset of the black cell when the pair starts red
-        const int rbk = (warp + 1) * 33 + lane;              // red offset of cell lane in halo row warp+1
-        const long long nxy = (long long)nx * ny;
-        AF_PTR(float) gp = eout + ((long long)(x0 + 2 * lane) + (long long)nx * by + nxy * z0);
-        if (tid == 0) {
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            for (int k = 0; k < kZmLead && k <= K + 1; ++k) issue(k);
+        const unsigned local = (unsigned)(item - tab.prefix[s]);
+        const unsigned t1 = L.march[K].fcol.div(local), t2 = L.march[K].fty.div(t1);
+        const int q0 = (int)(local - t1 * L.march[K].fcol.d) * mw;  // first output quad
+        const int y0 = (int)(t1 - t2 * L.march[K].fty.d) * mrows;
+        const int z0 = (int)t2 * zc, zl = min(z0 + zc, nz);  // output planes z0 .. zl-1
+        const int row = (int)L.march[K].fq.div((unsigned)tid), rows = min(mrows, ny - y0);
+        const int xq = q0 - (q0 > 0 ? 1 : 0) + tid - row * mq, x = 4 * xq;
+        const int y = y0 - 1 + row, yc = min(max(y, 0), ny - 1);
+        const bool in_y = y == yc;
+        const bool active = row < rows + 2 && x < nx && xq < q0 + mw + 1;
+        const bool out = active && row >= 1 && row <= rows && xq >= q0 && xq < q0 + mw;
+        const int i0 = x + nx * yc;                    // the quad in its (wall-clamped) row
+        const int on = in_y && y > 0 ? -nx : 0, os = in_y && y < ny - 1 ? nx : 0;
+        // The cell across the quad's end that a red cell needs: left of it
+        // when the red cells are 0 and 2, right when they are 1 and 3 (the
+        // quad's own end cell at an x wall).
+        const int xl = x > 0 ? -1 : 0, xr = x + 4 < nx ? 4 : 3;
+        auto quad = [&](AF_PTR(const float) p) { return AF_VEC(const float4, p, 0, 4); };
+        float4 ec{}, ep{}, rc{}, N{}, S{};
+        float xs = 0.0f;
+        float2 em{}, rb{}, red1{}, red2{};  // e (plane z-1) and r (z-1) at plane z's red positions; red of z-1, z-2
+        int pr = (y + z0 - 1) & 1;          // the red cells of plane z are pr and pr + 2
+        // The quad at plane z (e) and z + 1 (e), at z (r) and at z - 1 (out);
+        // planes outside the level are the wall plane.
+        const int zf = max(z0 - 1, 0);
+        AF_PTR(const float) pe = ein + (i0 + zf * nxy);
+        AF_PTR(const float) pn = ein + (i0 + z0 * nxy);
+        AF_PTR(const float) pv = r + (i0 + zf * nxy);
+        AF_PTR(float) po = eout + (i0 + z0 * nxy);
+        if (active) {
+            const float4 e0 = quad(ein + (i0 + max(z0 - 2, 0) * nxy));
+            ec = quad(pe);
+            ep = quad(pn);
+            rc = quad(pv);
+            N = quad(pe + on);
+            S = quad(pe + os);
+            xs = pe[pr ? xr : xl];
+            em = pr ? make_float2(e0.y, e0.w) : make_float2(e0.x, e0.z);
         }
-        bool failed = !mbar_wait_bounded(&bar[0], phase & 1u);
-        if (!failed) phase ^= 1u;
-        if (walls && !failed) {
-            fill(0);
-            fill(1);
-            fill(2);
-        }
-        if (__syncthreads_or(failed ? 1 : 0)) {
-            if (tid == 0) {
-                atomicOr(diag, 1u);
-                for (int j = 0; j < kZmLead && j <= K + 1; ++j) mbar_wait_bounded(&bar[j], (phase >> j) & 1u);
-            }
-            __syncthreads();
-            return;
-        }
-        // Step k (k = kb + J, J the compile-time step within a block of 8):
-        // e ring slots of planes k .. k+3 are J .. J+3 (mod 8), r slots of
-        // planes z0-1+k and z0-2+k are J and J-1, the red plane is J & 3 and
-        // group k+1's barrier is J+1.
-        auto step = [&](auto Jc, int kb) -> bool {  // false: a wait gave up (the block has returned its transfers)
-            constexpr int J = decltype(Jc)::value;
-            constexpr int s0 = J & 7, s1 = (J + 1) & 7, s2 = (J + 2) & 7, s3 = (J + 3) & 7;
-            constexpr int sr = J & 7, srp = (J + 7) & 7, b1 = (J + 1) & 7;
-            const int k = kb + J;
-            if (k + 1 <= K + 1) {  // group k+1, first read at step k+1
-                if (!failed) {
-                    if (mbar_wait_bounded(&bar[b1], (phase >> b1) & 1u)) phase ^= 1u << b1;
-                    else failed = true;
+        for (int z = z0 - 1; z <= zl; ++z, ++n) {
+            float2 red{}, eb{}, rv{};
+            if (active) {
+                const bool in = in_y && (unsigned)z < (unsigned)nz;
+                const float c0 = pr ? ec.y : ec.x, c1 = pr ? ec.w : ec.z;
+                const float sx0 = (pr ? ec.x : xs) + (pr ? ec.z : ec.y), sx1 = (pr ? ec.z : ec.y) + (pr ? xs : ec.w);
+                const float sy0 = (pr ? N.y : N.x) + (pr ? S.y : S.x), sy1 = (pr ? N.w : N.z) + (pr ? S.w : S.z);
+                const float v0 = mg_relax(W, sx0, sy0, em.x + (pr ? ep.y : ep.x), pr ? rc.y : rc.x, inv, c0);
+                const float v1 = mg_relax(W, sx1, sy1, em.y + (pr ? ep.w : ep.z), pr ? rc.w : rc.z, inv, c1);
+                red = in ? make_float2(v0, v1) : make_float2(c0, c1);
+                ring[n & 3u][tid] = red;
+                // Plane z + 1's red positions are plane z's black ones.
+                eb = em, rv = rb;
+                em = pr ? make_float2(ec.x, ec.z) : make_float2(ec.y, ec.w);
+                rb = pr ? make_float2(rc.x, rc.z) : make_float2(rc.y, rc.w);
+                ec = ep;
+                if (z < zl) {  // the next plane's operands
+                    pe = pn;
+                    if (z >= 0 && z + 1 < nz) pv += nxy;  // r's plane z + 1, e's plane z + 2
+                    if (z + 2 < nz) pn += nxy;
+                    ep = quad(pn);
+                    rc = quad(pv);
+                    N = quad(pe + on);
+                    S = quad(pe + os);
+                    xs = pe[pr ? xl : xr];
                 }
-                if (walls && !failed) fill(s3);
             }
-            const int zr = z0 - 1 + k;
-            const bool zin = (unsigned)zr < (unsigned)nz;
-            const ZmAddr ec = ZM_A(s1 * kZmEPlane);
-            constexpr int dzm = (s0 - s1) * kZmEPlane * kZmB, dzp = (s2 - s1) * kZmEPlane * kZmB;
-            constexpr int drr = (kZmROff + sr * kZmRPlane - s1 * kZmEPlane - kZmBX) * kZmB;
-            const ZmAddr rs = ZM_A(kZmRedOff + (J & 3) * kZmRedPlane);
-            if (!failed) {
-                auto red_cell = [&](int e0, int d0, int y1, int x) {
-                    const int par = (y1 + zr) & 1;
-                    const ZmAddr a = ec + (e0 + par) * kZmB;
-                    const bool in = zin && (unsigned)(y1 - 1) < (unsigned)ny && (unsigned)(x + par) < (unsigned)nx;
-                    const float c = ZM_LD(a, 0);
-                    const float v = mg_relax(L, ZM_LD(a, -1) + ZM_LD(a, 1), ZM_LD(a, -kZmBX) + ZM_LD(a, kZmBX),
-                                             ZM_LD(a + (ZmAddr)dzm, 0) + ZM_LD(a + (ZmAddr)dzp, 0), ZM_LD(a + (ZmAddr)drr, 0), inv, c);
-                    ZM_ST(rs + d0 * kZmB, in ? v : c);
-                };
-                red_cell(eA, dA, yA, xA);
-                if (xe) red_cell(eB, dB, yB, xB);
-            }
-            if (__syncthreads_or(failed ? 1 : 0)) {
-                if (tid == 0) {
-                    atomicOr(diag, 1u);
-                    for (int j = k + 1; j <= k + kZmLead - 1 && j <= K + 1; ++j)  // groups issued, not yet waited
-                        mbar_wait_bounded(&bar[j & 7], (phase >> (j & 7)) & 1u);
+            // Publish this plane's red cells; then wait for the last one's.
+            // A warp runs at most a plane ahead of the others: its ring slot
+            // was last read three planes ago.
+            __syncwarp();
+            if ((tid & 31) == 0) mbar_arrive(&bar[n & 1u]);
+            if (n > 0) march_wait(&bar[(n - 1u) & 1u], ((n - 1u) >> 1) & 1u);
+            if (active) {
+                if (z > z0) {
+                    if (out) {
+                        // Black cells of plane z - 1, at plane z's red
+                        // positions: their old values are eb, their r rv, the
+                        // red cells below and above red2 and red, beside them
+                        // red1.
+                        const float2* rg = ring[(n - 1u) & 3u];
+                        const float2 n = rg[tid - mq], u = rg[tid + mq];
+                        // Across the quad's end: the next quad's first red
+                        // cell (black 1 and 3) or the previous one's last.
+                        float e;
+                        if (pr) e = x + 4 < nx ? rg[tid + 1].x : eb.y;
+                        else e = x > 0 ? rg[tid - 1].y : eb.x;
+                        const float mid = red1.x + red1.y;
+                        const float sb0 = pr ? mid : e + red1.x, sb1 = pr ? red1.y + e : mid;
+                        const float b0 = mg_relax(W, sb0, n.x + u.x, red2.x + red.x, rv.x, inv, eb.x);
+                        const float b1 = mg_relax(W, sb1, n.y + u.y, red2.y + red.y, rv.y, inv, eb.y);
+                        AF_VEC(float4, po, 0, 4) =
+                            pr ? make_float4(red1.x, b0, red1.y, b1) : make_float4(b0, red1.x, b1, red1.y);
+                    }
+                    po += nxy;
                 }
-                __syncthreads();
-                return false;
+                red2 = red1, red1 = red;
+                pr ^= 1;
             }
-            if (tid == 0 && k + kZmLead <= K + 1) {
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                issue(k + kZmLead);
-            }
-            if (k >= 2 && bw) {
-                // Black cells of plane zr - 1: e ring plane k, r plane k-1,
-                // red planes k-2, k-1, k.
-                const int pr = (by + zr - 1) & 1;
-                const ZmAddr eb = ZM_A(s0 * kZmEPlane + ebk - pr);
-                const float c = ZM_LD(eb, 0);
-                constexpr int drv = (kZmROff + srp * kZmRPlane - s0 * kZmEPlane - kZmBX) * kZmB;
-                const float rv = ZM_LD(eb + (ZmAddr)drv, 0);
-                const ZmAddr r1 = ZM_A(kZmRedOff + ((J + 3) & 3) * kZmRedPlane + rbk);
-                const ZmAddr h1 = r1 + (1 - pr) * kZmB;
-                constexpr int dz0 = (((J + 2) & 3) - ((J + 3) & 3)) * kZmRedPlane * kZmB;
-                constexpr int dz2 = ((J & 3) - ((J + 3) & 3)) * kZmRedPlane * kZmB;
-                const float sx = ZM_LD(r1, 0) + ZM_LD(r1, 1);
-                const float sy = ZM_LD(h1, -33) + ZM_LD(h1, 33);
-                const float sz = ZM_LD(h1 + (ZmAddr)dz0, 0) + ZM_LD(h1 + (ZmAddr)dz2, 0);
-                const float bv = mg_relax(L, sx, sy, sz, rv, inv, c);
-                const float red_v = ZM_LD(r1 + pr * kZmB, 0);
-                if (bok) AF_VEC(float2, gp, 0, 2) = pr ? make_float2(bv, red_v) : make_float2(red_v, bv);
-            }
-            if (k >= 2) gp += nxy;
-            return true;
-        };
-        bool ok = true;
-        for (int kb = 0; ok && kb <= K + 1; kb += 8) {
-            ok = step(std::integral_constant<int, 0>{}, kb);
-            if (ok && kb + 1 <= K + 1) ok = step(std::integral_constant<int, 1>{}, kb);
-            if (ok && kb + 2 <= K + 1) ok = step(std::integral_constant<int, 2>{}, kb);
-            if (ok && kb + 3 <= K + 1) ok = step(std::integral_constant<int, 3>{}, kb);
-            if (ok && kb + 4 <= K + 1) ok = step(std::integral_constant<int, 4>{}, kb);
-            if (ok && kb + 5 <= K + 1) ok = step(std::integral_constant<int, 5>{}, kb);
-            if (ok && kb + 6 <= K + 1) ok = step(std::integral_constant<int, 6>{}, kb);
-            if (ok && kb + 7 <= K + 1) ok = step(std::integral_constant<int, 7>{}, kb);
         }
-        if (!ok) return;
-        __syncthreads();  // every thread is done with the rings before the next column's loads
     }
 }
-#undef ZM_A
-#undef ZM_LD
-#undef ZM_ST
 
 // --- tail V-cycle: every level from the slot's tail down, in one block -------
 // Levels of at most kCoarseMax cells live in shared memory: pre-smoothing and
@@ -1844,6 +1744,7 @@ struct Batch {
     unsigned graph_big = 0;          // levels whose large-coarsest smoothing the graph carries
     unsigned graph_pair = 0;         // levels with wide fused-pair tiles in the graph
     unsigned graph_pairn = 0;        // levels with narrow fused-pair tiles in the graph
+    unsigned graph_march = 0;        // levels with marching pairs in the graph
     unsigned graph_single = 0;       // levels with in-place colour sweeps in the graph
     size_t tail_smem = 0;            // dynamic shared memory of the tail V-cycle
     int graph_nu = 0;                // smoothing sweeps the captured graph carries
@@ -1864,8 +1765,7 @@ struct Batch {
     CUtensorMap* d_tmaps = nullptr;    // 12 per slot, see InstDev::tmap
     std::vector<CUtensorMap> h_tmaps;
     bool tmaps_dirty = true;
-    CUtensorMap* d_pmaps = nullptr;    // 3 per level and slot, see InstDev::pmap
-    std::vector<CUtensorMap> h_pmaps;
+    unsigned march = ~0u;              // levels whose fused pairs march where a slot's level allows it
     int force_pair_var = -1;           // AEROFLUX_PAIR_VARIANT: every fused pair stage's variant (-1: tuned)
     bool pair_chosen = false;          // the fused pairs' tile variants are set (tuned or by level size)
     unsigned* d_diag = nullptr;        // nonzero: a kernel gave up waiting on a transfer
@@ -1901,6 +1801,21 @@ unsigned single_levels(const Batch* b) {
     return m;
 }
 
+// Whether a slot's fused pairs of level l march.
+bool marches(const Batch* b, const SlotHost& S, int l) { return (b->march & (1u << l)) && S.d.lev[l].march[0].w > 0; }
+
+// Levels with marching pairs.
+unsigned march_levels(const Batch* b) {
+    unsigned m = 0;
+    for (const auto& s : b->slots) {
+        if (!s.used) continue;
+        const int lim = s.d.tail >= 0 ? s.d.tail : s.d.nlev - 1;
+        for (int l = 0; l < lim; ++l)
+            if (s.d.lev[l].e2 && marches(b, s, l)) m |= 1u << l;
+    }
+    return m;
+}
+
 // Levels whose fused pairs need the narrow tile column (wide: the others).
 unsigned pair_levels(const Batch* b, bool narrow) {
     unsigned m = 0;
@@ -1909,7 +1824,7 @@ unsigned pair_levels(const Batch* b, bool narrow) {
         const int lim = s.d.tail >= 0 ? s.d.tail : s.d.nlev - 1;
         for (int l = 0; l < lim; ++l) {
             const Lvl& L = s.d.lev[l];
-            if (L.e2 && (narrow ? L.nxw < L.nx : L.nxw > 0)) m |= 1u << l;
+            if (L.e2 && !marches(b, s, l) && (narrow ? L.nxw < L.nx : L.nxw > 0)) m |= 1u << l;
         }
     }
     return m;
@@ -1923,7 +1838,7 @@ size_t tail_smem_bytes(const Batch* b) {
 }
 
 // Items of stage `st` for slot `s` under shape sh.
-long long stage_items(const SlotHost& S, int st, const Shape& sh) {
+long long stage_items(const Batch* b, const SlotHost& S, int st, const Shape& sh) {
     if (!S.used || !S.active) return 0;
     const InstDev& I = S.d;
     const long long per = (long long)sh.tpb * sh.ept;
@@ -1953,10 +1868,16 @@ long long stage_items(const SlotHost& S, int st, const Shape& sh) {
     } else if (st >= S_BIGCOARSE && st < S_PAIR) {
         const int l = st - S_BIGCOARSE;
         n = (l == I.nlev - 1 && I.tail < 0) ? row_box(I.lev[l]) : 0;
-    } else if (st >= S_PAIR && st < S_COUNT) {
+    } else if (st >= S_MARCH) {
+        const int l = st - S_MARCH;
+        if (l >= lim || !I.lev[l].e2 || !marches(b, S, l)) return 0;
+        const MarchShape& m = kMarchShapes[sh.var];
+        const Lvl::March& M = I.lev[l].march[m.k];
+        return (long long)M.fcol.d * M.fty.d * cdivl(I.lev[l].nz, m.zc);
+    } else if (st >= S_PAIR) {
         const bool wide = st < S_PAIRN;
         const int l = st - (wide ? S_PAIR : S_PAIRN);
-        if (l >= lim || !I.lev[l].e2) return 0;
+        if (l >= lim || !I.lev[l].e2 || marches(b, S, l)) return 0;
         const Lvl& L = I.lev[l];
         const long long cols = wide ? L.nxw / kPairWideX : (L.nxw < L.nx ? 1 : 0);
         return cols * cdivl(L.ny, kPairVarTY[sh.var]) * cdivl(L.nz, kPairVarTZ[sh.var]);
@@ -1964,18 +1885,28 @@ long long stage_items(const SlotHost& S, int st, const Shape& sh) {
     return cdivl(n, per);
 }
 
+// A stage's prefix of tiles per slot under its present shape.
+void fill_tab(Batch* b, int st) {
+    int* pre = &b->h_tab[(size_t)st * (b->cap + 1)];
+    long long acc = 0;
+    for (int s = 0; s < b->cap; ++s) {
+        pre[s] = (int)acc;
+        acc += stage_items(b, b->slots[s], st, b->shape[st]);
+    }
+    pre[b->cap] = (int)acc;
+}
+
+// One stage's work list alone, when only its shape changed.
+cudaError_t upload_stage(Batch* b, int st) {
+    const size_t w = (size_t)b->cap + 1;
+    fill_tab(b, st);
+    return cudaMemcpyAsync(b->d_tab + st * w, &b->h_tab[st * w], w * sizeof(int), cudaMemcpyHostToDevice, b->stream);
+}
+
 cudaError_t upload_tables(Batch* b) {
     const int w = b->cap + 1;
     b->h_tab.assign((size_t)S_COUNT * w, 0);
-    for (int st = 0; st < S_COUNT; ++st) {
-        int* pre = &b->h_tab[(size_t)st * w];
-        long long acc = 0;
-        for (int s = 0; s < b->cap; ++s) {
-            pre[s] = (int)acc;
-            acc += stage_items(b->slots[s], st, b->shape[st]);
-        }
-        pre[b->cap] = (int)acc;
-    }
+    for (int st = 0; st < S_COUNT; ++st) fill_tab(b, st);
     std::vector<InstDev> inst(b->cap);
     for (int s = 0; s < b->cap; ++s) {
         inst[s] = b->slots[s].d;
@@ -1990,8 +1921,6 @@ cudaError_t upload_tables(Batch* b) {
         return rc;
     if (b->tmaps_dirty) {
         if ((rc = cudaMemcpyAsync(b->d_tmaps, b->h_tmaps.data(), b->h_tmaps.size() * sizeof(CUtensorMap),
-                                  cudaMemcpyHostToDevice, b->stream)) != cudaSuccess ||
-            (rc = cudaMemcpyAsync(b->d_pmaps, b->h_pmaps.data(), b->h_pmaps.size() * sizeof(CUtensorMap),
                                   cudaMemcpyHostToDevice, b->stream)) != cudaSuccess)
             return rc;
         b->tmaps_dirty = false;
@@ -2062,12 +1991,6 @@ void launch_pair_v(Batch* b, int st, int l, int dir, int vc, cudaStream_t s) {
 
 void launch_pair(Batch* b, int st, int l, int dir, int vc, cudaStream_t s) {
     const bool wide = st < S_PAIRN;
-    if (wide && b->shape[st].var == 3) {
-        kb_smooth_pair_zm<kZmZC><<<grid(b, st), kZmThreads, kZmSmem, s>>>(b->d_inst, b->d_ctl, tab(b, st), l, dir,
-                                                                         vc, b->d_diag);
-        ++b->launches;
-        return;
-    }
     switch (b->shape[st].var) {
         case 0: wide ? launch_pair_v<32, 0>(b, st, l, dir, vc, s) : launch_pair_v<16, 0>(b, st, l, dir, vc, s); break;
         case 1: wide ? launch_pair_v<32, 1>(b, st, l, dir, vc, s) : launch_pair_v<16, 1>(b, st, l, dir, vc, s); break;
@@ -2077,31 +2000,22 @@ void launch_pair(Batch* b, int st, int l, int dir, int vc, cudaStream_t s) {
 }
 
 Shape pair_shape(bool wide, int var) {
-    if (var == 3) return Shape{kZmThreads, 1, kZmBlocks, 3};
     const int threads = kPairVarTY[var] * (wide ? 32 : 16);
     return Shape{threads, 1, (var == 0 || var == 4 ? 2048 : 1536) / threads, var};
 }
 
-// Whether a used slot has wide pair tiles at level l without the staged
-// pair's maps.
-bool pair_tma_missing(const Batch* b, int l) {
-    for (const auto& S : b->slots)
-        if (S.used && l < S.d.nlev && S.d.lev[l].e2 && S.d.lev[l].nxw > 0 && !S.d.lev[l].tma) return true;
-    return false;
+Shape march_shape(int m) {
+    const int t = kMarchT[kMarchShapes[m].k];
+    return Shape{t, 1, kMarchBlocks[kMarchShapes[m].k], m};
 }
 
-// Whether every used slot whose level l has wide pair tiles can run the
-// TMA-staged pair there (and at least one has them).
-bool pair_tma_ok(const Batch* b, int l) {
-    bool any = false;
-    for (const auto& S : b->slots) {
-        if (!S.used || l >= S.d.nlev) continue;
-        const Lvl& L = S.d.lev[l];
-        if (!L.e2 || L.nxw == 0) continue;
-        if (!L.tma) return false;
-        any = true;
-    }
-    return any;
+void launch_march(Batch* b, int l, int dir, int vc, cudaStream_t s) {
+    const int st = S_MARCH + l, g = grid(b, st);
+    const MarchShape m = kMarchShapes[b->shape[st].var];
+    if (m.k == 0) kb_smooth_march<0><<<g, kMarchT[0], 0, s>>>(b->d_inst, b->d_ctl, tab(b, st), l, dir, vc, m.zc);
+    else if (m.k == 1) kb_smooth_march<1><<<g, kMarchT[1], 0, s>>>(b->d_inst, b->d_ctl, tab(b, st), l, dir, vc, m.zc);
+    else kb_smooth_march<2><<<g, kMarchT[2], 0, s>>>(b->d_inst, b->d_ctl, tab(b, st), l, dir, vc, m.zc);
+    ++b->launches;
 }
 
 // Pre- or post-smoothing of level l: fused pairs ping-ponging through e2
@@ -2113,6 +2027,7 @@ void enq_level_smooth(Batch* b, int l, int vc, cudaStream_t s) {
     for (int k = 0; k < b->nu; ++k) {
         if (b->graph_pair & (1u << l)) launch_pair(b, S_PAIR + l, l, k & 1, vc, s);
         if (b->graph_pairn & (1u << l)) launch_pair(b, S_PAIRN + l, l, k & 1, vc, s);
+        if (b->graph_march & (1u << l)) launch_march(b, l, k & 1, vc, s);
     }
     if (b->graph_single & (1u << l)) enq_smooth(b, S_SMOOTH + l, l, b->nu, vc, s);
 }
@@ -2246,32 +2161,23 @@ cudaError_t capture(Batch* b, F body, cudaGraphExec_t* out) {
     return rc;
 }
 
-// Untuned tile variants of the fused pairs, by the largest level each pair
-// stage serves: the largest tiles from 4 Mi cells, the middle ones from
-// 256 Ki, the smallest below.  Set once, before the first capture (the
-// captured kernels and the work lists must agree); the autotuner may replace
-// them.
+// Untuned tile variants and march shapes of the fused pairs, by the largest
+// level each pair stage serves: the largest tiles from 4 Mi cells, the middle
+// ones from 256 Ki, the smallest below.  Set once, before the first capture
+// (the captured kernels and the work lists must agree); the autotuner may
+// replace them.
 void default_pair_variants(Batch* b) {
-    // A slot assigned after the choice may lack the staged pair's maps at a
-    // level that runs it: that level goes back to the plain variant 1 tiles.
-    for (int l = 0; l < kMaxLev; ++l)
-        if (b->shape[S_PAIR + l].var == 3 && pair_tma_missing(b, l)) {
-            b->shape[S_PAIR + l] = pair_shape(true, 1);
-            b->tables_dirty = true;
-            if (b->graph) {
-                cudaGraphExecDestroy(b->graph);
-                b->graph = nullptr;
-            }
-        }
     if (b->pair_chosen || b->graph) return;
+    if (b->force_pair_var >= 0) b->march = b->force_pair_var == 3 ? ~0u : 0u;
     for (int l = 0; l < kMaxLev; ++l) {
         long long most = 0;
         for (const auto& S : b->slots)
             if (S.used && l < S.d.nlev) most = std::max(most, lvl_cells(S.d.lev[l]));
         int var = most >= (4ll << 20) ? 0 : (most >= (256ll << 10) ? 1 : 2);
-        if (b->force_pair_var >= 0) var = b->force_pair_var;
-        b->shape[S_PAIR + l] = pair_shape(true, var == 3 && !pair_tma_ok(b, l) ? 1 : var);
-        b->shape[S_PAIRN + l] = pair_shape(false, var == 3 ? 1 : var);
+        b->shape[S_MARCH + l] = march_shape(most >= (4ll << 20) ? 7 : (most >= (256ll << 10) ? 1 : 0));
+        if (b->force_pair_var >= 0 && b->force_pair_var != 3) var = b->force_pair_var;
+        b->shape[S_PAIR + l] = pair_shape(true, var);
+        b->shape[S_PAIRN + l] = pair_shape(false, var);
     }
     b->pair_chosen = true;
     b->tables_dirty = true;
@@ -2283,10 +2189,10 @@ cudaError_t prepare(Batch* b) {
     if (b->tables_dirty && (rc = upload_tables(b)) != cudaSuccess) return rc;
     const int L = max_levels(b);
     const unsigned big = big_coarse_levels(b), pair = pair_levels(b, false), pairn = pair_levels(b, true),
-                   single = single_levels(b);
+                   single = single_levels(b), march = march_levels(b);
     const size_t tsm = tail_smem_bytes(b);
     if (b->graph && (L > b->graph_levels || (big & ~b->graph_big) || (pair & ~b->graph_pair) ||
-                     (pairn & ~b->graph_pairn) || (single & ~b->graph_single) || tsm > b->tail_smem ||
+                     (pairn & ~b->graph_pairn) || (march & ~b->graph_march) || (single & ~b->graph_single) || tsm > b->tail_smem ||
                      b->graph_nu != b->nu)) {
         cudaGraphExecDestroy(b->graph);
         b->graph = nullptr;
@@ -2296,6 +2202,7 @@ cudaError_t prepare(Batch* b) {
         b->graph_big |= big;
         b->graph_pair |= pair;
         b->graph_pairn |= pairn;
+        b->graph_march |= march;
         b->graph_single |= single;
         b->tail_smem = std::max(b->tail_smem, tsm);
         b->graph_nu = b->nu;
@@ -2372,29 +2279,27 @@ bool encode_slot_maps(const InstDev& I, CUtensorMap* maps) {
     return true;
 }
 
-// The three tensor maps of the z-marching pair per level (e, e2, r: one
-// plane of a 64 x 16 column plus a two-cell ring for e and e2, a one-cell
-// ring for r) for every level with wide pair tiles whose rows and arrays are
-// 16-byte aligned; sets Lvl::tma on those levels.
-void encode_pair_maps(InstDev& I, CUtensorMap* maps) {
-    auto enc = tensor_map_encoder();
+// The tiles of the marching pair on every level with e2 whose rows and arrays
+// are 16-byte aligned.
+void plan_march(InstDev& I) {
     for (int l = 0; l < I.nlev; ++l) {
         Lvl& L = I.lev[l];
-        L.tma = 0;
-        if (!enc || !L.e2 || L.nxw == 0 || L.nx % 4 != 0) continue;
         auto aligned = [](const void* q) { return ((uintptr_t)q & 15u) == 0; };
-        if (!aligned(L.e) || !aligned(L.e2) || !aligned(L.r)) continue;
-        const cuuint64_t dims[3] = {(cuuint64_t)L.nx, (cuuint64_t)L.ny, (cuuint64_t)L.nz};
-        const cuuint64_t strides[2] = {(cuuint64_t)L.nx * 4u, (cuuint64_t)L.nx * L.ny * 4u};
-        const cuuint32_t estr[3] = {1, 1, 1};
-        const cuuint32_t ebox[3] = {kZmBX, kZmEY, 1}, rbox[3] = {kZmBX, kZmRY, 1};
-        float* arr[3] = {L.e, L.e2, L.r};
-        bool ok = true;
-        for (int k = 0; k < 3 && ok; ++k)
-            ok = enc(&maps[3 * l + k], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, arr[k], dims, strides, k < 2 ? ebox : rbox,
-                     estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                     CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-        L.tma = ok ? 1 : 0;
+        const bool ok = L.e2 && L.nx % 4 == 0 && aligned(L.e) && aligned(L.e2) && aligned(L.r);
+        const int quads = L.nx / 4;
+        for (int k = 0; k < 3; ++k) {
+            Lvl::March& M = L.march[k];
+            M = Lvl::March{};
+            if (!ok) continue;
+            const int cols = (quads + kMarchQ[k] - 1) / kMarchQ[k];
+            M.w = (quads + cols - 1) / cols;
+            M.q = cols > 1 ? M.w + 2 : M.w;
+            const int most = kMarchT[k] / M.q - 2, ty = (L.ny + most - 1) / most;  // most >= 12
+            M.rows = (L.ny + ty - 1) / ty;
+            M.fq = FastDiv((unsigned)M.q);
+            M.fcol = FastDiv((unsigned)((quads + M.w - 1) / M.w));
+            M.fty = FastDiv((unsigned)((L.ny + M.rows - 1) / M.rows));
+        }
     }
 }
 
@@ -2433,6 +2338,7 @@ Batch* batch_create(int capacity, size_t pool_bytes, std::string* err) {
     for (int l = 0; l < kMaxLev; ++l) {
         b->shape[S_PAIR + l] = pair_shape(true, 0);
         b->shape[S_PAIRN + l] = pair_shape(false, 0);
+        b->shape[S_MARCH + l] = march_shape(0);
     }
     cudaError_t rc;
     if ((rc = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking)) != cudaSuccess ||
@@ -2442,7 +2348,6 @@ Batch* batch_create(int capacity, size_t pool_bytes, std::string* err) {
         (rc = cudaMalloc(&b->d_ctl, sizeof(Ctl) * (capacity + 1))) != cudaSuccess ||
         (rc = cudaMalloc(&b->d_tab, sizeof(int) * (size_t)S_COUNT * (capacity + 1))) != cudaSuccess ||
         (rc = cudaMalloc(&b->d_tmaps, sizeof(CUtensorMap) * 12 * (size_t)capacity)) != cudaSuccess ||
-        (rc = cudaMalloc(&b->d_pmaps, sizeof(CUtensorMap) * 3 * kMaxLev * (size_t)capacity)) != cudaSuccess ||
         (rc = cudaMalloc(&b->d_diag, sizeof(unsigned))) != cudaSuccess) {
         *err = std::string("aeroflux: batch tables: ") + cudaGetErrorString(rc);
         batch_destroy(b);
@@ -2451,10 +2356,8 @@ Batch* batch_create(int capacity, size_t pool_bytes, std::string* err) {
     cudaMemsetAsync(b->d_ctl, 0, sizeof(Ctl) * (capacity + 1), b->stream);
     cudaMemsetAsync(b->d_diag, 0, sizeof(unsigned), b->stream);
     b->h_tmaps.assign(12 * (size_t)capacity, CUtensorMap{});
-    b->h_pmaps.assign(3 * kMaxLev * (size_t)capacity, CUtensorMap{});
-    cudaFuncSetAttribute(kb_smooth_pair_zm<kZmZC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kZmSmem);
-    // The fused pairs' tile variant for every level (0-2 and 4; 3: TMA-staged
-    // where the levels allow it), instead of the tuned or size-based choice.
+    // The fused pairs' tile variant for every level (0-2 and 4; 3: marching
+    // where a slot's level allows it), instead of the tuned or size-based choice.
     if (const char* pv = getenv("AEROFLUX_PAIR_VARIANT")) b->force_pair_var = std::min(4, std::max(0, atoi(pv)));
     if (pool_bytes) {
         if (!b->pool.init(pool_bytes)) {
@@ -2486,7 +2389,6 @@ void batch_destroy(Batch* b) {
     cudaFree(b->d_ctl);
     cudaFree(b->d_tab);
     cudaFree(b->d_tmaps);
-    cudaFree(b->d_pmaps);
     cudaFree(b->d_diag);
     if (b->body) cudaStreamDestroy(b->body);
     if (b->stream) cudaStreamDestroy(b->stream);
@@ -2779,8 +2681,7 @@ int batch_assign(Batch* b, const af_config& c, char* arena, std::string* err) {
         }
     }
     cudaMemsetAsync(p, 0, mg, b->stream);
-    I.pmap = b->d_pmaps + 3 * kMaxLev * (size_t)s;
-    encode_pair_maps(I, &b->h_pmaps[3 * kMaxLev * (size_t)s]);
+    plan_march(I);
     const double half = c.dt * 0.5;  // aeroflux.go:353
     const double invH = 1.0 / c.h;
     I.dt_invh = (float)(half * invH);
@@ -2858,6 +2759,7 @@ cudaError_t batch_prepare_capture(Batch* b) {
     b->graph_big |= big_coarse_levels(b);
     b->graph_pair |= pair_levels(b, false);
     b->graph_pairn |= pair_levels(b, true);
+    b->graph_march |= march_levels(b);
     b->graph_single |= single_levels(b);
     b->tail_smem = std::max(b->tail_smem, tail_smem_bytes(b));
     if ((rc = cudaFuncSetAttribute(kb_vtail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->tail_smem)) !=
@@ -3015,10 +2917,8 @@ bool batch_device_error(Batch* b, std::string* msg) {
     cudaMemcpy(&v, b->d_diag, sizeof v, cudaMemcpyDeviceToHost);
     if (!v) return false;
     cudaMemset(b->d_diag, 0, sizeof v);
-    *msg = (v & 4u)   ? "aeroflux: cuda: the staged pair's shared-memory rings are not 128-byte aligned; the step's "
+    *msg = (v & 4u)   ? "aeroflux: cuda: a staged kernel's shared-memory buffers are not 128-byte aligned; the step's "
                         "results are invalid"
-           : (v & 2u) ? "aeroflux: cuda: the TMA-staged pair ran on a level without tensor maps; the step's results "
-                        "are invalid"
                       : "aeroflux: cuda: a staged kernel gave up waiting for its tile transfer; the step's results "
                         "are invalid";
     return true;
@@ -3114,6 +3014,7 @@ std::string batch_tune(Batch* b, int reps) {
             kb_prolong<<<gsz, tpb, 0, s>>>(b->d_inst, b->d_ctl, t, st - S_PROLONG, 0);
         else if (st >= S_PAIR && st < S_PAIRN) launch_pair(b, st, st - S_PAIR, 0, 0, s);
         else if (st >= S_PAIRN && st < S_PAIRN + kMaxLev) launch_pair(b, st, st - S_PAIRN, 0, 0, s);
+        else if (st >= S_MARCH) launch_march(b, st - S_MARCH, 0, 0, s);
     };
     std::vector<int> stages = {S_BC, S_SHADOW, S_DIV, S_INT, S_PBC, S_GRAD};
     if (!b->tma_sweep) stages.push_back(S_SWEEP);  // the staged sweep keeps its fixed tile shape
@@ -3122,66 +3023,129 @@ std::string batch_tune(Batch* b, int reps) {
         stages.push_back(S_RESTRICT + l);
         stages.push_back(S_PROLONG + l);
     }
-    bool first = true;
-    // Fused pairs: one of three tile variants per level and tile column.
-    for (int l = 0; l < L; ++l) {
-        stages.push_back(S_PAIR + l);
-        stages.push_back(S_PAIRN + l);
-    }
     default_pair_variants(b);
     b->pair_chosen = true;
-    const Shape pair_cands[2][4] = {{pair_shape(true, 0), pair_shape(true, 1), pair_shape(true, 2), pair_shape(true, 4)},
-                                    {pair_shape(false, 0), pair_shape(false, 1), pair_shape(false, 2), pair_shape(false, 4)}};
-    for (int st : stages) {
-        long long items = 0;
-        for (auto& S : b->slots) items += stage_items(S, st, b->shape[st]);
-        if (!items) continue;
-        Shape best = b->shape[st];
-        float best_ms = 1e30f;
-        const bool pair_st = st >= S_PAIR && st < S_PAIRN + kMaxLev;
-        if (pair_st && b->force_pair_var >= 0) continue;
-        std::vector<Shape> cs(cands, cands + sizeof cands / sizeof cands[0]);
-        if (pair_st) {
-            cs.assign(pair_cands[st >= S_PAIRN], pair_cands[st >= S_PAIRN] + 4);
-            if (st < S_PAIRN && pair_tma_ok(b, st - S_PAIR)) cs.push_back(pair_shape(true, 3));
+    // Per-launch median of stage st under its present shape, microseconds (each
+    // repetition timed on its own: one disturbed launch does not decide);
+    // negative when a launch failed.  Events resolve about 2 us, so a
+    // repetition of a short stage is two or four launches (decided by the first
+    // candidate's warm-up, *launches = 0).
+    auto timed = [&](int st, int* launches) {
+        upload_stage(b, st);
+        if (*launches == 0) cudaEventRecord(rev[0], s);
+        run(st);  // warm-up
+        if (*launches == 0) {
+            cudaEventRecord(rev[1], s);
+            cudaEventSynchronize(rev[1]);
+            float once = 0.0f;
+            cudaEventElapsedTime(&once, rev[0], rev[1]);
+            *launches = once < 0.015f ? 4 : (once < 0.03f ? 2 : 1);
         }
-        std::string tried;  // fused-pair stages: every tile variant's time
-        for (const Shape& c : cs) {
-            b->shape[st] = c;
-            upload_tables(b);
-            run(st);  // warm-up
-            // Each repetition timed on its own; the median of them stands
-            // for the candidate (one disturbed launch does not decide).
-            for (int r = 0; r < reps; ++r) {
-                cudaEventRecord(rev[2 * r], s);
-                run(st);
-                cudaEventRecord(rev[2 * r + 1], s);
-            }
-            cudaEventSynchronize(rev[2 * reps - 1]);
-            std::vector<float> t(reps);
-            for (int r = 0; r < reps; ++r) cudaEventElapsedTime(&t[r], rev[2 * r], rev[2 * r + 1]);
-            std::nth_element(t.begin(), t.begin() + reps / 2, t.end());
-            const float ms = t[reps / 2] * reps;  // per-launch median, scaled like the report's sum
-            const bool ok = cudaGetLastError() == cudaSuccess;
-            if (ok && ms < best_ms) {
-                best_ms = ms;
-                best = c;
-            }
-            if (pair_st) {
-                char t[48];
-                snprintf(t, sizeof t, "%s\"%d\": %.2f", tried.empty() ? "" : ", ", c.var, ok ? 1e3 * ms / reps : -1.0);
-                tried += t;
-            }
+        for (int r = 0; r < reps; ++r) {
+            cudaEventRecord(rev[2 * r], s);
+            for (int k = 0; k < *launches; ++k) run(st);
+            cudaEventRecord(rev[2 * r + 1], s);
         }
-        b->shape[st] = best;
+        cudaEventSynchronize(rev[2 * reps - 1]);
+        std::vector<float> t(reps);
+        for (int r = 0; r < reps; ++r) cudaEventElapsedTime(&t[r], rev[2 * r], rev[2 * r + 1]);
+        std::nth_element(t.begin(), t.begin() + reps / 2, t.end());
+        return cudaGetLastError() == cudaSuccess ? 1e3f * t[reps / 2] / *launches : -1.0f;
+    };
+    auto has_items = [&](int st) {
+        for (auto& S : b->slots)
+            if (stage_items(b, S, st, b->shape[st])) return true;
+        return false;
+    };
+    auto report_stage = [&](int st, const Shape& sh, int var, float us, const std::string& variants) {
         char buf[160];
         snprintf(buf, sizeof buf,
                  "%s\"stage_%d\": {\"tpb\": %d, \"ept\": %d, \"blocks_per_sm\": %d, \"variant\": %d, \"us\": %.2f",
-                 first ? "" : ", ", st, best.tpb, best.ept, best.bpsm, best.var, 1e3 * best_ms / reps);
+                 report.size() > 1 ? ", " : "", st, sh.tpb, sh.ept, sh.bpsm, var, us);
         report += buf;
-        if (pair_st) report += ", \"variants_us\": {" + tried + "}";
+        if (!variants.empty()) report += ", \"variants_us\": {" + variants + "}";
         report += "}";
-        first = false;
+    };
+    // Gives a stage the fastest of the candidate shapes: of the first `brief`
+    // only when the first one takes less than 10 us, most of it the launch.
+    auto fastest = [&](int st, const std::vector<Shape>& cs, std::vector<float>* times, size_t brief) {
+        Shape best = b->shape[st];
+        float best_us = 1e30f, first_us = 1e30f;
+        int launches = 0;
+        for (size_t i = 0; i < cs.size() && (i < brief || first_us >= 10.0f); ++i) {
+            const Shape& c = cs[i];
+            b->shape[st] = c;
+            const float us = timed(st, &launches);
+            if (i == 0) first_us = us;
+            if (times) times->push_back(us);
+            if (us >= 0.0f && us < best_us) best_us = us, best = c;
+        }
+        b->shape[st] = best;
+        return best_us;
+    };
+    for (int st : stages) {
+        if (!has_items(st)) continue;
+        const float us = fastest(st, std::vector<Shape>(cands, cands + sizeof cands / sizeof cands[0]), nullptr, 3);
+        report_stage(st, b->shape[st], b->shape[st].var, us, "");
+    }
+    // Fused pairs, per level: the tile variants of both tile columns with no
+    // slot marching, then the march shapes; a level marches (variant 3 of its
+    // first pair stage) when that and what cannot march take less time than
+    // the tiles do.
+    for (int l = 0; l < L && b->force_pair_var < 0; ++l) {
+        const unsigned bit = 1u << l;
+        b->march &= ~bit;
+        const int stages2[2] = {S_PAIR + l, S_PAIRN + l};
+        std::vector<float> t[2];
+        float tile_us[2] = {0.0f, 0.0f};
+        bool has[2];
+        for (int w = 0; w < 2; ++w) {
+            has[w] = has_items(stages2[w]);
+            if (!has[w]) continue;
+            std::vector<Shape> cs;
+            for (int v : kPairTileVars) cs.push_back(pair_shape(w == 0, v));
+            tile_us[w] = fastest(stages2[w], cs, &t[w], cs.size());
+        }
+        if (!has[0] && !has[1]) continue;
+        const float tiles = tile_us[0] + tile_us[1];
+        float march_us = -1.0f;
+        b->march |= bit;
+        if (has_items(S_MARCH + l)) {
+            std::vector<Shape> cs;
+            long long most = 0;  // the largest level's cells: small ones have no use for long chunks of large blocks
+            for (auto& S : b->slots)
+                if (S.used && S.active && l < S.d.nlev) most = std::max(most, lvl_cells(S.d.lev[l]));
+            for (int m = 0; m < kMarchShapeCount; ++m)
+                if (most >= (1ll << 20) ? kMarchShapes[m].zc >= 8 : kMarchShapes[m].k == 0)
+                    cs.push_back(march_shape(m));
+            march_us = fastest(S_MARCH + l, cs, nullptr, cs.size());
+            for (int st : stages2)
+                if (has_items(st)) {  // slots that cannot march
+                    int launches = 0;
+                    march_us += std::max(0.0f, timed(st, &launches));
+                }
+        }
+        const bool march = march_us >= 0.0f && march_us < tiles;
+        if (!march) b->march &= ~bit;
+        const int lead = has[0] ? 0 : 1;  // the stage whose report carries the level's choice
+        for (int w = 0; w < 2; ++w) {
+            if (!has[w]) continue;
+            const float other = w == lead ? tiles - tile_us[w] : 0.0f;
+            std::string variants;
+            char buf[64];
+            for (size_t v = 0; v < t[w].size(); ++v) {
+                snprintf(buf, sizeof buf, "%s\"%d\": %.2f", v ? ", " : "", kPairTileVars[v],
+                         t[w][v] < 0.0f ? -1.0f : t[w][v] + other);
+                variants += buf;
+            }
+            if (w == lead && march_us >= 0.0f) {
+                snprintf(buf, sizeof buf, ", \"3\": %.2f", march_us);
+                variants += buf;
+            }
+            const bool m = w == lead && march;
+            report_stage(stages2[w], m ? b->shape[S_MARCH + l] : b->shape[stages2[w]],
+                         m ? 3 : b->shape[stages2[w]].var, m ? march_us : tile_us[w] + other, variants);
+        }
     }
     report += "}";
     for (auto& ev : rev) cudaEventDestroy(ev);
