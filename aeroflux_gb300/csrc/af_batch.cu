@@ -29,6 +29,7 @@
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdio.h>
+#include <stddef.h>
 #include <stdlib.h>
 #include <string.h>
 
@@ -161,6 +162,37 @@ __device__ __forceinline__ int find_slot(const int* prefix, int n, int item) {
     return __shfl_sync(0xffffffffu, lo, 0);
 }
 
+// The start of every batched kernel.  Its launch may overlap the end of the
+// kernel before it (launch_pdl): the block waits before it reads anything a
+// kernel wrote.  What no kernel writes -- with one slot, its record (`bytes`
+// from `off`) and work list -- it fetches into its L1 before it waits (with
+// many slots the search for the block's own costs as much as it saves).
+// Measured per Step with the passes before the WHILE node: 16^3 789 -> 722
+// us, 48x32x64 1.62 -> 1.48 ms, 128^3 3.25 -> 3.18, the 256-grid batch
+// unchanged.
+__device__ __forceinline__ void touch(const void* p) {
+    unsigned v;
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+}
+__device__ __forceinline__ void begin(const InstDev* inst, const Tab& tab, size_t off, size_t bytes) {
+    if (tab.n == 1) {
+        const char* p = (const char*)inst + off;
+        if (threadIdx.x * 128u < bytes) touch(p + threadIdx.x * 128u);
+        if (threadIdx.x == 0) touch(tab.prefix);
+    }
+    pdl_wait();
+    // A grid that takes at most a quarter of the SMs' threads leaves the next
+    // kernel's blocks room to get this far while it runs.
+    if (gridDim.x * blockDim.x <= 152u * 512u) pdl_trigger();
+}
+// The record up to its levels, or level l (and the next).
+__device__ __forceinline__ void begin_slot(const InstDev* inst, const Tab& tab) {
+    begin(inst, tab, 0, offsetof(InstDev, lev) + sizeof(Lvl));
+}
+__device__ __forceinline__ void begin_level(const InstDev* inst, const Tab& tab, int l, int levels) {
+    begin(inst, tab, offsetof(InstDev, lev) + l * sizeof(Lvl), levels * sizeof(Lvl));
+}
+
 // Loop over this block's tiles; `s` is the slot, `first` the first element
 // of the tile; body sees element index `el` (< the slot's count, checked by
 // the body).
@@ -197,6 +229,7 @@ __host__ __device__ inline long long lvl_cells(const Lvl& L) { return (long long
 
 // --- binary64 stages (bit-identical to the FP64 form's cells) -------------
 __global__ void kb_bc(const InstDev* inst, Status* st, Tab tab, int parity, int gate) {
+    begin_slot(inst, tab);
     FOR_TILES(tab)
     const InstDev& I = inst[s];
     if (gated(&st[s], gate)) continue;
@@ -225,6 +258,7 @@ __global__ void kb_bc(const InstDev* inst, Status* st, Tab tab, int parity, int 
 }
 
 __global__ void kb_div(const InstDev* inst, Status* st, Tab tab, int parity, int gate) {
+    begin_slot(inst, tab);
     FOR_TILES(tab)
     const InstDev& I = inst[s];
     if (gated(&st[s], gate)) continue;
@@ -243,6 +277,7 @@ __global__ void kb_div(const InstDev* inst, Status* st, Tab tab, int parity, int
 }
 
 __global__ void kb_pbc(const InstDev* inst, Status* st, Tab tab, int gate) {
+    begin_slot(inst, tab);
     FOR_TILES(tab)
     const InstDev& I = inst[s];
     if (gated(&st[s], gate)) continue;
@@ -262,6 +297,7 @@ __global__ void kb_pbc(const InstDev* inst, Status* st, Tab tab, int gate) {
 // scratch = 1 (the autotuner's timing runs) stores the new values into the
 // Tmp fields instead, so timing leaves the slots' velocities untouched.
 __global__ void kb_grad(const InstDev* inst, Status* st, Tab tab, int parity, int gate, int scratch) {
+    begin_slot(inst, tab);
     FOR_TILES(tab)
     const InstDev& I = inst[s];
     if (gated(&st[s], gate)) continue;
@@ -295,6 +331,7 @@ __global__ void kb_grad(const InstDev* inst, Status* st, Tab tab, int parity, in
 // describe the shadow.  A thread converts four consecutive elements of one
 // row and stores them with one 16-byte store (padding: zeros).
 __global__ void kb_shadow(const InstDev* inst, Tab tab, int parity) {
+    begin_slot(inst, tab);
     FOR_TILES(tab)
     const InstDev& I = inst[s];
     const long long n = I.shq[3];
@@ -382,6 +419,7 @@ __host__ __device__ inline long long sweep_box(const Geom& g) {
 
 template <int AX>
 __global__ void kb_sweep(const InstDev* inst, Status* st, Tab tab, int parity, int phase) {
+    begin_slot(inst, tab);
     FOR_TILES(tab)
     const InstDev& I = inst[s];
     if (gated(&st[s], phase)) continue;
@@ -648,6 +686,7 @@ __device__ __forceinline__ void sw_issue(const InstDev& I, const SwTile& t, floa
 template <int AX>
 __global__ void __launch_bounds__(kSwThreads, 4)
     kb_sweep_tma(const InstDev* inst, Status* st, Tab tab, int parity, int phase, unsigned* diag) {
+    begin_slot(inst, tab);
     extern __shared__ __align__(128) float swsm[];
     // Buffer pair k: own-component box and axis box.
     auto own = [&](int k) { return swsm + k * kSwOwnMax; };
@@ -705,12 +744,14 @@ __global__ void __launch_bounds__(kSwThreads, 4)
 }
 
 __global__ void kb_tick(const InstDev* inst, Status* st, int n) {
+    pdl_wait();
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x)
         if (inst[s].active) st[s].step += 1;
 }
 
 // --- refinement control ---------------------------------------------------
 __global__ void kb_init(const InstDev* inst, Ctl* ctl, int n) {
+    pdl_wait();
     if (blockIdx.x == 0 && threadIdx.x == 0) ctl[n].nv = 0xFFFFFFFFu;  // until a check counts them
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
         ctl[s].maxr_bits = 0;
@@ -741,6 +782,7 @@ __device__ __forceinline__ void warp_max_commit(unsigned long long m, unsigned l
 // atomics are per block, not per warp-sized tile.  In the loop a converged
 // slot is skipped.
 __global__ void kb_residual(const InstDev* inst, Status* st, Ctl* ctl, Tab tab, int gate, int in_loop) {
+    begin_slot(inst, tab);
     int held = -1;
     unsigned long long m = 0;
     for (int item = blockIdx.x, total = tab.prefix[tab.n]; item < total; item += gridDim.x) {
@@ -789,6 +831,7 @@ __global__ void kb_residual(const InstDev* inst, Status* st, Ctl* ctl, Tab tab, 
 
 // p += e over the interior, a warp per (y, z) row (32 lanes per row).
 __global__ void kb_correct(const InstDev* inst, Ctl* ctl, Tab tab) {
+    begin_slot(inst, tab);
     FOR_TILES(tab)
     const InstDev& I = inst[s];
     if (ctl[s].stopped) continue;
@@ -813,6 +856,7 @@ __global__ void kb_correct(const InstDev* inst, Ctl* ctl, Tab tab) {
 // condition is "any slot continues".  Bounded by each slot's max_refine.
 __global__ void kb_check(const InstDev* inst, Status* st, Ctl* ctl, int n, cudaGraphConditionalHandle h, int use_cond,
                          int count_pass, int gate, int vcycles, double pass_floor) {
+    pdl_wait();
     __shared__ unsigned most;  // V-cycles of the next pass, most over the slots
     if (threadIdx.x == 0) most = 0u;
     __syncthreads();
@@ -912,6 +956,7 @@ __device__ __forceinline__ float mg_interp(float ax, float ay, float az, float e
 __host__ __device__ inline long long row_box(const Lvl& L) { return 32ll * L.ny * L.nz; }
 
 __global__ void kb_smooth(const InstDev* inst, const Ctl* ctl, Tab tab, int l, int color, int vc) {
+    begin_level(inst, tab, l, 1);
     if (vc_idle(ctl, tab.n, vc)) return;
     FOR_TILES(tab)
     if (mg_off(ctl[s], vc)) continue;
@@ -964,6 +1009,7 @@ __device__ __forceinline__ float mg_residual(const Lvl& L, int x, int y, int z, 
 // the compiler's 56 registers.  (The prolongation spills at 32 and measured
 // slower at 32 and 40.)
 __global__ void __launch_bounds__(1024, 2) kb_restrict(const InstDev* inst, const Ctl* ctl, Tab tab, int l, int vc) {
+    begin_level(inst, tab, l, 2);
     if (vc_idle(ctl, tab.n, vc)) return;
     FOR_TILES(tab)
     if (mg_off(ctl[s], vc)) continue;
@@ -1050,6 +1096,7 @@ __host__ __device__ inline long long prolong_box(const Lvl& F, const Lvl& C) {
 }
 
 __global__ void kb_prolong(const InstDev* inst, const Ctl* ctl, Tab tab, int l, int vc) {
+    begin_level(inst, tab, l, 2);
     if (vc_idle(ctl, tab.n, vc)) return;
     FOR_TILES(tab)
     if (mg_off(ctl[s], vc)) continue;
@@ -1208,6 +1255,7 @@ struct PairTile {
 template <int LANES, int V>
 __global__ void __launch_bounds__(PairTile<LANES, V>::THREADS, PairTile<LANES, V>::RESIDENT / PairTile<LANES, V>::THREADS)
     kb_smooth_pair(const InstDev* inst, const Ctl* ctl, Tab tab, int l, int dir, int vc) {
+    begin_level(inst, tab, l, 1);
     if (vc_idle(ctl, tab.n, vc)) return;
     using T = PairTile<LANES, V>;
     __shared__ float red[T::HZ][T::HY][T::RX];
@@ -1343,6 +1391,7 @@ __device__ __forceinline__ void march_wait(unsigned long long* bar, unsigned par
 template <int K>
 __global__ void __launch_bounds__(kMarchT[K], kMarchBlocks[K])
     kb_smooth_march(const InstDev* inst, const Ctl* ctl, Tab tab, int l, int dir, int vc, int zc) {
+    begin_level(inst, tab, l, 1);
     if (vc_idle(ctl, tab.n, vc)) return;
     constexpr int T = kMarchT[K];
     __shared__ float2 ring[4][T];
@@ -1507,6 +1556,7 @@ __device__ __forceinline__ float sm_res(const Lvl& L, AF_PTR(const float) e, AF_
 
 __global__ void __launch_bounds__(kCoarseThreads) kb_vtail(const InstDev* inst, const Ctl* ctl, Tab tab, int nu,
                                                            int vc) {
+    begin_slot(inst, tab);
     if (vc_idle(ctl, tab.n, vc)) return;
     extern __shared__ float tsm[];
     __shared__ float red[32];
@@ -1945,7 +1995,7 @@ void size_grids(Batch* b) {
 
 #define LAUNCH(b, st, kernel, ...)                                                          \
     do {                                                                                    \
-        kernel<<<grid(b, st), b->shape[st].tpb, 0, s>>>(__VA_ARGS__);                       \
+        launch_pdl(kernel, dim3(grid(b, st)), dim3(b->shape[st].tpb), 0, s, __VA_ARGS__);   \
         ++b->launches;                                                                      \
     } while (0)
 
@@ -1960,10 +2010,8 @@ void enq_sweep(Batch* b, int axis, int parity, int phase, cudaStream_t s) {
     if (b->tma_sweep) {
         const Tab t = tab(b, S_SWEEPT);
         const int g = grid(b, S_SWEEPT);
-        if (axis == 0) kb_sweep_tma<0><<<g, kSwThreads, kSwSmem, s>>>(b->d_inst, b->d_st, t, parity, phase, b->d_diag);
-        else if (axis == 1)
-            kb_sweep_tma<1><<<g, kSwThreads, kSwSmem, s>>>(b->d_inst, b->d_st, t, parity, phase, b->d_diag);
-        else kb_sweep_tma<2><<<g, kSwThreads, kSwSmem, s>>>(b->d_inst, b->d_st, t, parity, phase, b->d_diag);
+        const auto k = axis == 0 ? kb_sweep_tma<0> : (axis == 1 ? kb_sweep_tma<1> : kb_sweep_tma<2>);
+        launch_pdl(k, dim3(g), dim3(kSwThreads), kSwSmem, s, b->d_inst, b->d_st, t, parity, phase, b->d_diag);
         ++b->launches;
         return;
     }
@@ -1984,8 +2032,8 @@ void enq_smooth(Batch* b, int st, int l, int pairs, int vc, cudaStream_t s) {
 // tiles for S_PAIR + l, the narrow column for S_PAIRN + l).
 template <int LANES, int V>
 void launch_pair_v(Batch* b, int st, int l, int dir, int vc, cudaStream_t s) {
-    kb_smooth_pair<LANES, V><<<grid(b, st), PairTile<LANES, V>::THREADS, 0, s>>>(b->d_inst, b->d_ctl, tab(b, st), l,
-                                                                               dir, vc);
+    launch_pdl(kb_smooth_pair<LANES, V>, dim3(grid(b, st)), dim3(PairTile<LANES, V>::THREADS), 0, s, b->d_inst, b->d_ctl,
+               tab(b, st), l, dir, vc);
     ++b->launches;
 }
 
@@ -2012,9 +2060,8 @@ Shape march_shape(int m) {
 void launch_march(Batch* b, int l, int dir, int vc, cudaStream_t s) {
     const int st = S_MARCH + l, g = grid(b, st);
     const MarchShape m = kMarchShapes[b->shape[st].var];
-    if (m.k == 0) kb_smooth_march<0><<<g, kMarchT[0], 0, s>>>(b->d_inst, b->d_ctl, tab(b, st), l, dir, vc, m.zc);
-    else if (m.k == 1) kb_smooth_march<1><<<g, kMarchT[1], 0, s>>>(b->d_inst, b->d_ctl, tab(b, st), l, dir, vc, m.zc);
-    else kb_smooth_march<2><<<g, kMarchT[2], 0, s>>>(b->d_inst, b->d_ctl, tab(b, st), l, dir, vc, m.zc);
+    const auto k = m.k == 0 ? kb_smooth_march<0> : (m.k == 1 ? kb_smooth_march<1> : kb_smooth_march<2>);
+    launch_pdl(k, dim3(g), dim3(kMarchT[m.k]), 0, s, b->d_inst, b->d_ctl, tab(b, st), l, dir, vc, m.zc);
     ++b->launches;
 }
 
@@ -2040,8 +2087,8 @@ void enq_vcycle(Batch* b, int vc, cudaStream_t s) {
         enq_level_smooth(b, l, vc, s);
         LAUNCH(b, S_RESTRICT + l, kb_restrict, b->d_inst, b->d_ctl, tab(b, S_RESTRICT + l), l, vc);
     }
-    kb_vtail<<<grid(b, S_COARSE), kCoarseThreads, b->tail_smem, s>>>(b->d_inst, b->d_ctl, tab(b, S_COARSE), b->nu,
-                                                                      vc);
+    launch_pdl(kb_vtail, dim3(grid(b, S_COARSE)), dim3(kCoarseThreads), b->tail_smem, s, b->d_inst, b->d_ctl,
+               tab(b, S_COARSE), b->nu, vc);
     ++b->launches;
     for (int l = 0; l < L; ++l)
         if (b->graph_big & (1u << l)) enq_smooth(b, S_BIGCOARSE + l, l, 8 * b->nu, vc, s);
@@ -2051,11 +2098,13 @@ void enq_vcycle(Batch* b, int vc, cudaStream_t s) {
     }
 }
 
+constexpr int kStraightPasses = 2;
+
 void enq_pass(Batch* b, cudaStream_t s, cudaGraphConditionalHandle h, int use_cond, int gate) {
     for (int k = 0; k < b->vcycles; ++k) enq_vcycle(b, k, s);
     LAUNCH(b, S_CORR, kb_correct, b->d_inst, b->d_ctl, tab(b, S_CORR));
     LAUNCH(b, S_INT, kb_residual, b->d_inst, b->d_st, b->d_ctl, tab(b, S_INT), gate, 1);
-    kb_check<<<1, 256, 0, s>>>(b->d_inst, b->d_st, b->d_ctl, b->cap, h, use_cond, 1, gate, b->vcycles, b->pass_floor);
+    launch_pdl(kb_check, dim3(1), dim3(256), 0, s, b->d_inst, b->d_st, b->d_ctl, b->cap, h, use_cond, 1, gate, b->vcycles, b->pass_floor);
     ++b->launches;
 }
 
@@ -2064,11 +2113,11 @@ void enq_project(Batch* b, int parity, int gate, cudaStream_t s) {
     rec(b, kEvProj + (gate == 3 ? 0 : 2), s);
     enq_bc(b, parity, gate, s);
     LAUNCH(b, S_DIV, kb_div, b->d_inst, b->d_st, tab(b, S_DIV), parity, gate);
-    kb_init<<<1, 256, 0, s>>>(b->d_inst, b->d_ctl, b->cap);
+    launch_pdl(kb_init, dim3(1), dim3(256), 0, s, b->d_inst, b->d_ctl, b->cap);
     ++b->launches;
     LAUNCH(b, S_INT, kb_residual, b->d_inst, b->d_st, b->d_ctl, tab(b, S_INT), gate, 0);
     if (b->fixed_passes > 0) {
-        kb_check<<<1, 256, 0, s>>>(b->d_inst, b->d_st, b->d_ctl, b->cap, 0, 0, 0, gate, b->vcycles, b->pass_floor);
+        launch_pdl(kb_check, dim3(1), dim3(256), 0, s, b->d_inst, b->d_st, b->d_ctl, b->cap, 0, 0, 0, gate, b->vcycles, b->pass_floor);
         ++b->launches;
         for (int k = 0; k < b->fixed_passes; ++k) enq_pass(b, s, 0, 0, gate);
     } else {
@@ -2086,8 +2135,14 @@ void enq_project(Batch* b, int parity, int gate, cudaStream_t s) {
             b->capture_err = rc;
             return;
         }
-        kb_check<<<1, 256, 0, s>>>(b->d_inst, b->d_st, b->d_ctl, b->cap, h, 1, 0, gate, b->vcycles, b->pass_floor);
+        launch_pdl(kb_check, dim3(1), dim3(256), 0, s, b->d_inst, b->d_st, b->d_ctl, b->cap, h, 0, 0, gate, b->vcycles,
+                   b->pass_floor);
         ++b->launches;
+        // Nearly every projection needs two passes, and an iteration of the
+        // WHILE node costs 50-100 us more than the same launches outside it:
+        // the first two passes stand before it (their kernels return at once
+        // where every slot has converged), the second sets its condition.
+        for (int k = 0; k < kStraightPasses; ++k) enq_pass(b, s, h, k + 1 == kStraightPasses, gate);
         if ((rc = cudaStreamGetCaptureInfo(s, &cs, nullptr, &graph, &deps, nullptr, &ndeps)) != cudaSuccess) {
             b->capture_err = rc;
             return;
@@ -2137,7 +2192,7 @@ void enq_step(Batch* b, cudaStream_t s) {
         if (k == 2) enq_project(b, 1, 3, s);
     }
     enq_project(b, 0, 6, s);
-    kb_tick<<<1, 256, 0, s>>>(b->d_inst, b->d_st, b->cap);
+    launch_pdl(kb_tick, dim3(1), dim3(256), 0, s, b->d_inst, b->d_st, b->cap);
     ++b->launches;
     rec(b, kEvEnd, s);
 }
