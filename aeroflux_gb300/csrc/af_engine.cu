@@ -606,7 +606,7 @@ int af_create(const af_config* cin, af_engine** out, char* err, size_t errlen) {
         e->split.place(e->split_mem);
     }
     if ((cr = cudaMalloc(&e->st, sizeof(Status))) != cudaSuccess ||
-        (cr = cudaMalloc(&e->partials, sizeof(double) * (size_t)std::max<int64_t>(c.nz, 1))) != cudaSuccess ||
+        (cr = cudaMalloc(&e->partials, sizeof(double) * (size_t)af::kinetic_energy_partials(g))) != cudaSuccess ||
         (cr = cudaMalloc(&e->sum, sizeof(double))) != cudaSuccess ||
         (cr = cudaMalloc(&e->mx, sizeof(unsigned long long))) != cudaSuccess) {
         e->err = sfmt("aeroflux: device scratch: %s", cudaGetErrorString(cr));
@@ -814,12 +814,13 @@ int af_max_divergence(af_engine* e, double* out) {
     if (!out) return AF_ERR_ARG;
     Fields f = e->fields();
     AF_CUDA(e, cudaMemsetAsync(e->mx, 0, sizeof(unsigned long long), e->stream));
-    af::launch_max_divergence(e->geom, f.u, f.v, f.w, 1.0 / e->cfg.h, e->mx, e->stream);
+    af::launch_max_divergence(e->geom, f.u, f.v, f.w, e->mx, e->stream);
     AF_CUDA(e, cudaGetLastError());
     unsigned long long bits = 0;
     AF_CUDA(e, cudaMemcpyAsync(&bits, e->mx, sizeof bits, cudaMemcpyDeviceToHost, e->stream));
     AF_CUDA(e, cudaStreamSynchronize(e->stream));
     memcpy(out, &bits, sizeof bits);
+    *out = (1.0 / e->cfg.h) * *out;
     return AF_OK;
 }
 
@@ -1229,11 +1230,12 @@ int af_batch_max_divergence(af_batch* h, int64_t slot, double* out) {
     af::batch_field(h->b, (int)slot, AF_FIELD_W, &w);
     cudaStream_t s = af::batch_stream(h->b);
     cudaMemsetAsync(h->mx, 0, sizeof *h->mx, s);
-    af::launch_max_divergence(af::batch_geom(h->b, (int)slot), u, v, w, 1.0 / h->cfg[slot].h, h->mx, s);
+    af::launch_max_divergence(af::batch_geom(h->b, (int)slot), u, v, w, h->mx, s);
     unsigned long long bits = 0;
     cudaMemcpyAsync(&bits, h->mx, sizeof bits, cudaMemcpyDeviceToHost, s);
     if (int r = batch_wait(h)) return r;
     memcpy(out, &bits, sizeof bits);
+    *out = (1.0 / h->cfg[slot].h) * *out;
     return AF_OK;
 }
 

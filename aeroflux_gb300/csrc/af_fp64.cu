@@ -564,11 +564,19 @@ __global__ void k_step_tick(Status* st) { st->step += 1; }
 // ---------------------------------------------------------------------------
 // Diagnostics.  A max is exact in any order; NaN is skipped as the
 // reference's `if a > mx` skips it.  Non-negative doubles order like their
-// bit patterns, so one atomicMax per block combines the blocks.
+// bit patterns, so one atomicMax per block combines the blocks, and every
+// test on a value is an integer one (a binary64 compare costs the binary64
+// pipe as much as an addition).  A warp walks a row, eight rows to a block (32
+// left the last wave half empty).  us a call at 256^3 before/now: max
+// divergence 279/188, max |velocity| 224/78 (HBM), kinetic energy 498/226;
+// the binary64 pipe bounds the first and the last, and further additions on
+// the integer pipe made neither faster.
 // ---------------------------------------------------------------------------
+constexpr int kDiagThreads = 256, kDiagRows = 8;
+
 __device__ __forceinline__ unsigned long long abs_bits(double d) {
-    const double a = fabs(d);
-    return isnan(a) ? 0ull : (unsigned long long)__double_as_longlong(a);
+    const unsigned long long b = dbits(d) & ~kSign;
+    return b > 0x7FF0000000000000ull ? 0ull : b;
 }
 
 __device__ __forceinline__ void block_max_commit(unsigned long long m, unsigned long long* out) {
@@ -578,71 +586,85 @@ __device__ __forceinline__ void block_max_commit(unsigned long long m, unsigned 
         const unsigned long long t = __shfl_xor_sync(0xffffffffu, m, o);
         m = t > m ? t : m;
     }
-    const int nthreads = blockDim.x * blockDim.y * blockDim.z;
-    const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
-    if ((tid & 31) == 0) sm[tid >> 5] = m;
+    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = m;
     __syncthreads();
-    if (tid < 32) {
-        m = tid < (nthreads + 31) / 32 ? sm[tid] : 0ull;
+    if (threadIdx.x < 32) {
+        m = threadIdx.x < blockDim.x / 32 ? sm[threadIdx.x] : 0ull;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             const unsigned long long t = __shfl_xor_sync(0xffffffffu, m, o);
             m = t > m ? t : m;
         }
-        if (tid == 0 && m) atomicMax(out, m);
+        if (threadIdx.x == 0 && m) atomicMax(out, m);
     }
 }
 
-// MaxDivergence, project.go:210-232.
-__global__ void k_max_divergence(Geom g, const double* __restrict__ u_, const double* __restrict__ v_,
-                                 const double* __restrict__ w_, double invH, unsigned long long* out) {
+// max |du + dv + dw| for MaxDivergence (project.go:210-232), which is
+// RN(1/h * that): rounding is monotone, so the product commutes with the
+// maximum and is taken once, by the host.  Of the five additions one runs on
+// the integer pipe beside the others.
+__global__ void __launch_bounds__(kDiagThreads) k_max_divergence(const __grid_constant__ Geom g,
+                                                                 const double* __restrict__ u_,
+                                                                 const double* __restrict__ v_,
+                                                                 const double* __restrict__ w_,
+                                                                 unsigned long long* out) {
     const int G = g.G;
     AF_PTR(const double) AF_RESTRICT u = view(u_, g.u.count, DK_F64_MAXDIV, 0);
     AF_PTR(const double) AF_RESTRICT v = view(v_, g.v.count, DK_F64_MAXDIV, 0);
     AF_PTR(const double) AF_RESTRICT w = view(w_, g.w.count, DK_F64_MAXDIV, 0);
-    const int x = G + (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    const int y = G + (int)blockIdx.y;
-    const int z = G + (int)blockIdx.z;
+    const int z = G + (int)blockIdx.y, y0 = (int)blockIdx.x * kDiagRows;
     unsigned long long m = 0;
-    if (x < G + g.NX) {
-        const long long iu = x + y * g.u.sy + z * g.u.sz;
-        const long long iv = x + y * g.v.sy + z * g.v.sz;
-        const long long iw = x + y * g.w.sy + z * g.w.sz;
-        const double d = dmul(invH, dadd(dadd(dsub(u[iu + 1], u[iu]), dsub(v[iv + g.v.sy], v[iv])),
-                                         dsub(w[iw + g.w.sz], w[iw])));
-        m = abs_bits(d);
+    for (int r = (int)threadIdx.x >> 5; r < kDiagRows && y0 + r < g.NY; r += kDiagThreads / 32) {
+        const int y = G + y0 + r;
+        const int iu = y * (int)g.u.sy + z * (int)g.u.sz, iv = y * (int)g.v.sy + z * (int)g.v.sz;
+        const int iw = y * (int)g.w.sy + z * (int)g.w.sz;
+        for (int x = G + ((int)threadIdx.x & 31); x < G + g.NX; x += 32) {
+            const double du = dsub(u[iu + x + 1], u[iu + x]);
+            const double dv = dsub_int(v[iv + x + (int)g.v.sy], v[iv + x]);
+            const double d = dadd(dadd(du, dv), dsub(w[iw + x + (int)g.w.sz], w[iw + x]));
+            const unsigned long long t = abs_bits(d);
+            m = t > m ? t : m;
+        }
     }
     block_max_commit(m, out);
 }
 
 // MaxVelocity, stencil.go:319-331: every element of U, V, W, ghosts included.
-__global__ void k_max_abs3(const double* __restrict__ u_, long long nu, const double* __restrict__ v_, long long nv,
-                           const double* __restrict__ w_, long long nw, unsigned long long* out) {
-    AF_PTR(const double) AF_RESTRICT u = view(u_, nu, DK_F64_MAXABS, 0);
-    AF_PTR(const double) AF_RESTRICT v = view(v_, nv, DK_F64_MAXABS, 0);
-    AF_PTR(const double) AF_RESTRICT w = view(w_, nw, DK_F64_MAXABS, 0);
+__global__ void __launch_bounds__(kDiagThreads) k_max_abs3(const double* __restrict__ u_, long long nu,
+                                                           const double* __restrict__ v_, long long nv,
+                                                           const double* __restrict__ w_, long long nw,
+                                                           unsigned long long* out) {
+    AF_PTR(const double) AF_RESTRICT f[3] = {view(u_, nu, DK_F64_MAXABS, 0), view(v_, nv, DK_F64_MAXABS, 0),
+                                             view(w_, nw, DK_F64_MAXABS, 0)};
+    const long long n[3] = {nu, nv, nw};
     unsigned long long m = 0;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nu; i += stride) {
-        const unsigned long long t = abs_bits(u[i]);
-        m = t > m ? t : m;
-    }
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += stride) {
-        const unsigned long long t = abs_bits(v[i]);
-        m = t > m ? t : m;
-    }
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nw; i += stride) {
-        const unsigned long long t = abs_bits(w[i]);
-        m = t > m ? t : m;
+    const long long stride = (long long)gridDim.x * kDiagThreads;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        long long i = (long long)blockIdx.x * kDiagThreads + threadIdx.x;
+        for (; i + 3 * stride < n[k]; i += 4 * stride) {  // four loads in flight
+            const double a = f[k][i], b = f[k][i + stride], c = f[k][i + 2 * stride], d = f[k][i + 3 * stride];
+            const unsigned long long p = max(abs_bits(a), abs_bits(b)), q = max(abs_bits(c), abs_bits(d));
+            m = max(m, max(p, q));
+        }
+        for (; i < n[k]; i += stride) m = max(m, abs_bits(f[k][i]));
     }
     block_max_commit(m, out);
 }
 
 // KineticEnergy, project.go:238-258.  The reference sums serially; this sums
-// each z-plane in a fixed per-thread order and a fixed shuffle tree, then the
-// planes in a fixed tree, so the result depends on the grid only and is
-// bit-identical run to run (it differs from the serial sum by rounding).
+// each block of rows in a fixed per-thread order and a fixed shuffle tree,
+// then the blocks in a fixed tree, so the result depends on the grid only and
+// is bit-identical run to run (it differs from the serial sum by rounding).
 constexpr int kKeThreads = 256;
+// Partial sums at most, and the rows of a block: enough blocks to fill the
+// GPU, as the grid alone decides.
+constexpr int kKeMaxPartials = 16384;
+__host__ __device__ inline int ke_rows(int NY, int NZ) {
+    int per = kKeThreads / 32;  // a row a warp
+    while ((long long)NZ * ((NY + per - 1) / per) > kKeMaxPartials && per < NY) per *= 2;
+    return per;
+}
 
 __device__ __forceinline__ double block_sum_fixed(double s) {
     __shared__ double sm[kKeThreads / 32];
@@ -658,29 +680,34 @@ __device__ __forceinline__ double block_sum_fixed(double s) {
     return s;
 }
 
-__global__ void __launch_bounds__(kKeThreads) k_ke_planes(Geom g, const double* __restrict__ u_,
+// Per cell three additions of face pairs (one of them on the integer pipe),
+// three exact halvings (exponent) and three fused multiply-adds.
+__global__ void __launch_bounds__(kKeThreads) k_ke_planes(const __grid_constant__ Geom g,
+                                                          const double* __restrict__ u_,
                                                           const double* __restrict__ v_,
-                                                          const double* __restrict__ w_, double* partials_) {
+                                                          const double* __restrict__ w_, int rows,
+                                                          double* partials_) {
     const int G = g.G;
     AF_PTR(const double) AF_RESTRICT u = view(u_, g.u.count, DK_F64_KE, 0);
     AF_PTR(const double) AF_RESTRICT v = view(v_, g.v.count, DK_F64_KE, 0);
     AF_PTR(const double) AF_RESTRICT w = view(w_, g.w.count, DK_F64_KE, 0);
-    AF_PTR(double) partials = view(partials_, (long long)gridDim.x, DK_F64_KE, 0);
-    const int z = G + (int)blockIdx.x;
-    const long long n = (long long)g.NX * g.NY;
+    AF_PTR(double) partials = view(partials_, (long long)gridDim.x * gridDim.y, DK_F64_KE, 0);
+    const int z = G + (int)blockIdx.x, y0 = (int)blockIdx.y * rows;
     double s = 0.0;
-    for (long long k = threadIdx.x; k < n; k += kKeThreads) {
-        const int x = G + (int)(k % g.NX), y = G + (int)(k / g.NX);
-        const long long iu = x + y * g.u.sy + z * g.u.sz;
-        const long long iv = x + y * g.v.sy + z * g.v.sz;
-        const long long iw = x + y * g.w.sy + z * g.w.sz;
-        const double uc = dmul(0.5, dadd(u[iu], u[iu + 1]));
-        const double vc = dmul(0.5, dadd(v[iv], v[iv + g.v.sy]));
-        const double wc = dmul(0.5, dadd(w[iw], w[iw + g.w.sz]));
-        s = dadd(s, dadd(dadd(dmul(uc, uc), dmul(vc, vc)), dmul(wc, wc)));
+    for (int r = (int)threadIdx.x >> 5; r < rows && y0 + r < g.NY; r += kKeThreads / 32) {
+        const int y = G + y0 + r;
+        const long long iu = y * g.u.sy + z * g.u.sz, iv = y * g.v.sy + z * g.v.sz, iw = y * g.w.sy + z * g.w.sz;
+        for (int x = G + ((int)threadIdx.x & 31); x < G + g.NX; x += 32) {
+            const double uc = half(dadd_int(u[iu + x], u[iu + x + 1]));
+            const double vc = half(dadd(v[iv + x], v[iv + x + g.v.sy]));
+            const double wc = half(dadd(w[iw + x], w[iw + x + g.w.sz]));
+            s = __fma_rn(uc, uc, s);
+            s = __fma_rn(vc, vc, s);
+            s = __fma_rn(wc, wc, s);
+        }
     }
     s = block_sum_fixed(s);
-    if (threadIdx.x == 0) partials[blockIdx.x] = s;
+    if (threadIdx.x == 0) partials[(long long)blockIdx.x * gridDim.y + blockIdx.y] = s;
 }
 
 __global__ void __launch_bounds__(kKeThreads) k_ke_final(const double* partials_, int n, double* out) {
@@ -941,17 +968,16 @@ void launch_gradient_fp64(const Geom& g, const Fields& f, double scale, Status* 
 
 void launch_step_tick(Status* st, cudaStream_t s) { k_step_tick<<<1, 1, 0, s>>>(st); }
 
-void launch_max_divergence(const Geom& g, const double* u, const double* v, const double* w, double invH,
-                           unsigned long long* out, cudaStream_t s) {
-    dim3 grid(cdiv(g.NX, 128), g.NY, g.NZ);
-    k_max_divergence<<<grid, 128, 0, s>>>(g, u, v, w, invH, out);
+void launch_max_divergence(const Geom& g, const double* u, const double* v, const double* w, unsigned long long* out,
+                           cudaStream_t s) {
+    k_max_divergence<<<dim3(cdiv(g.NY, kDiagRows), g.NZ), kDiagThreads, 0, s>>>(g, u, v, w, out);
 }
 
 void launch_max_abs3(const double* u, long long nu, const double* v, long long nv, const double* w, long long nw,
                      unsigned long long* out, cudaStream_t s) {
-    long long n = std::max(nu, std::max(nv, nw));
-    unsigned blocks = (unsigned)std::min<long long>(cdiv(n, 256), 152 * 8);
-    k_max_abs3<<<blocks, 256, 0, s>>>(u, nu, v, nv, w, nw, out);
+    const long long n = std::max(nu, std::max(nv, nw));
+    const unsigned blocks = (unsigned)std::min<long long>(cdiv(n, kDiagThreads), 152 * 8);
+    k_max_abs3<<<blocks, kDiagThreads, 0, s>>>(u, nu, v, nv, w, nw, out);
 }
 
 bool fp64_debug_bounds(unsigned long long* first, unsigned* count, bool reset) {
@@ -973,10 +999,14 @@ bool fp64_debug_bounds(unsigned long long* first, unsigned* count, bool reset) {
     return true;
 }
 
+int kinetic_energy_partials(const Geom& g) { return g.NZ * (int)cdiv(g.NY, ke_rows(g.NY, g.NZ)); }
+
 void launch_kinetic_energy(const Geom& g, const double* u, const double* v, const double* w, double* partials,
                            double* out, cudaStream_t s) {
-    k_ke_planes<<<g.NZ, kKeThreads, 0, s>>>(g, u, v, w, partials);
-    k_ke_final<<<1, kKeThreads, 0, s>>>(partials, g.NZ, out);
+    const int rows = ke_rows(g.NY, g.NZ);
+    const dim3 grid(g.NZ, cdiv(g.NY, rows));
+    k_ke_planes<<<grid, kKeThreads, 0, s>>>(g, u, v, w, rows, partials);
+    k_ke_final<<<1, kKeThreads, 0, s>>>(partials, (int)(grid.x * grid.y), out);
 }
 
 }  // namespace af
@@ -989,14 +1019,14 @@ void launch_kinetic_energy(const Geom& g, const double* u, const double* v, cons
 // afterwards, and latency-bound loops that cannot afford the implicit
 // device-wide synchronisation of cudaMalloc/cudaFree.  This entry point runs
 // the same fixed-order reduction as af_kinetic_energy over caller-owned
-// device fields, with its scratch (one partial per z-plane plus the final
+// device fields, with its scratch (the partial sums plus the final
 // sum) in the file-scope array below.  Every GPU that loads the library holds
 // the array until the process exits.
 // ---------------------------------------------------------------------------
 namespace af {
 namespace {
 
-constexpr int kNoAllocMaxPlanes = 16384;  // 128 KiB of partials
+constexpr int kNoAllocMaxPlanes = kKeMaxPartials;  // 128 KiB of partials
 static __device__ __align__(256) double g_ke_scratch[kNoAllocMaxPlanes + 1];
 
 constexpr int kMaxDevices = 64;
@@ -1073,8 +1103,7 @@ extern "C" int af_kinetic_energy_noalloc(const af_config* cfg, const double* u, 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     // Every partial the final pass reads is rewritten by this call, so the
     // array needs no clearing; concurrent calls on the GPU share it and race.
-    k_ke_planes<<<g.NZ, kKeThreads, 0, s>>>(g, u, v, w, scratch);
-    k_ke_final<<<1, kKeThreads, 0, s>>>(scratch, g.NZ, scratch + kNoAllocMaxPlanes);
+    launch_kinetic_energy(g, u, v, w, scratch, scratch + kNoAllocMaxPlanes, s);
     double sum = 0;
     if ((rc = cudaGetLastError()) != cudaSuccess ||
         (rc = cudaMemcpyAsync(&sum, scratch + kNoAllocMaxPlanes, sizeof sum, cudaMemcpyDeviceToHost, s)) !=

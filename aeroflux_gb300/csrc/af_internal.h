@@ -161,12 +161,14 @@ void launch_gradient_fp64(const Geom& g, const Fields& f, double scale, Status* 
 void launch_step_tick(Status* st, cudaStream_t s);
 
 // Diagnostics (af_fp64.cu).  `out` receives the bit pattern of a
-// non-negative double (max) or the fixed-order sum; `scratch` holds one
-// partial per z-plane for the sum.
-void launch_max_divergence(const Geom& g, const double* u, const double* v, const double* w, double invH,
-                           unsigned long long* out, cudaStream_t s);
+// non-negative double (max; of max |du + dv + dw|, to be multiplied by 1/h,
+// for the divergence) or the fixed-order sum; `partials` holds
+// kinetic_energy_partials(g) doubles for the sum.
+void launch_max_divergence(const Geom& g, const double* u, const double* v, const double* w, unsigned long long* out,
+                           cudaStream_t s);
 void launch_max_abs3(const double* u, long long nu, const double* v, long long nv, const double* w, long long nw,
                      unsigned long long* out, cudaStream_t s);
+int kinetic_energy_partials(const Geom& g);
 void launch_kinetic_energy(const Geom& g, const double* u, const double* v, const double* w, double* partials,
                            double* out, cudaStream_t s);
 

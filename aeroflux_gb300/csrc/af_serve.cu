@@ -86,13 +86,13 @@ double max_div_of(af_server* s, int slot, const af_config& c) {
     af::batch_field(s->b, slot, AF_FIELD_W, &w);
     cudaStream_t st = af::batch_stream(s->b);
     cudaMemsetAsync(s->mx, 0, sizeof *s->mx, st);
-    af::launch_max_divergence(af::batch_geom(s->b, slot), u, v, w, 1.0 / c.h, s->mx, st);
+    af::launch_max_divergence(af::batch_geom(s->b, slot), u, v, w, s->mx, st);
     unsigned long long bits = 0;
     cudaMemcpyAsync(&bits, s->mx, sizeof bits, cudaMemcpyDeviceToHost, st);
     cudaStreamSynchronize(st);
     double d;
     memcpy(&d, &bits, sizeof d);
-    return d;
+    return (1.0 / c.h) * d;
 }
 
 }  // namespace
