@@ -293,33 +293,41 @@ __global__ void kb_pbc(const InstDev* inst, Status* st, Tab tab, int gate) {
     END_TILES
 }
 
-// subtractGradient over every face, a warp per (component, y, z) face row.
+// subtractGradient, a thread per cell of the face box (grad_cell), the slot's
+// record in registers (read again a tile: 265 instead of 228 us at 256^3; a
+// thread a face: 311).
 // scratch = 1 (the autotuner's timing runs) stores the new values into the
 // Tmp fields instead, so timing leaves the slots' velocities untouched.
 __global__ void kb_grad(const InstDev* inst, Status* st, Tab tab, int parity, int gate, int scratch) {
     begin_slot(inst, tab);
+    int held = -1;  // the slot whose record is in registers
+    Geom g{};
+    exact::MulC scale{};
+    FastDiv fx, fy;
+    const double* pp = nullptr;
+    double *pf[3] = {}, *po[3] = {};
+    bool off = true;
     FOR_TILES(tab)
-    const InstDev& I = inst[s];
-    if (gated(&st[s], gate)) continue;
-    const Geom& g = I.g;
-    const long long rows = 3ll * (g.NY + 1) * (g.NZ + 1);
-    AF_PTR(double) u = view(cur(I, 1, parity), g.u.count, DK_GRAD, s);
-    AF_PTR(double) v = view(cur(I, 2, parity), g.v.count, DK_GRAD, s);
-    AF_PTR(double) w = view(cur(I, 3, parity), g.w.count, DK_GRAD, s);
+    if (s != held) {
+        held = s;
+        const InstDev& I = inst[s];
+        off = gated(&st[s], gate);
+        g = I.g, scale = I.grad_scale, fx = I.ffx, fy = I.ffy, pp = I.slot[0];
+        for (int c = 0; c < 3; ++c) {
+            pf[c] = cur(I, 1 + c, parity);
+            po[c] = scratch ? cur(I, 5 + c, parity) : pf[c];
+        }
+    }
+    if (off) continue;
+    const unsigned n = fx.d * fy.d * (unsigned)(g.NZ + 1);
     FOR_ELEMS(tab)
-    const long long row = el >> 5;
-    if (row >= rows) break;
-    const int lane = (int)(el & 31);
-    const unsigned r = (unsigned)row, r2 = I.ffy.div(r), cc = I.ffz.div(r2);
-    const int c = (int)cc;
-    const int y = g.G + (int)(r - r2 * (unsigned)(g.NY + 1)), z = g.G + (int)(r2 - cc * (unsigned)(g.NZ + 1));
-    if (y >= g.G + g.NY + (c == 1) || z >= g.G + g.NZ + (c == 2)) continue;
-    const int x1 = g.G + g.NX + (c == 0);
-    AF_PTR(const double) f = c == 0 ? u : (c == 1 ? v : w);
-    const long long fc = c == 0 ? g.u.count : (c == 1 ? g.v.count : g.w.count);
-    AF_PTR(double) out = scratch ? view(cur(I, 5 + c, parity), fc, DK_GRAD, s) : (c == 0 ? u : (c == 1 ? v : w));
-    AF_PTR(const double) p = view((const double*)I.slot[0], g.p.count, DK_GRAD, s);
-    for (int x = g.G + lane; x < x1; x += 32) grad_face_to(g, p, f, out, I.grad_scale, c, x, y, z);
+    if (el >= n) break;
+    const unsigned e = (unsigned)el, r = fx.div(e), z = fy.div(r);
+    grad_cell(g, view(pp, g.p.count, DK_GRAD, s), view((const double*)pf[0], g.u.count, DK_GRAD, s),
+              view((const double*)pf[1], g.v.count, DK_GRAD, s), view((const double*)pf[2], g.w.count, DK_GRAD, s),
+              view(po[0], g.u.count, DK_GRAD, s), view(po[1], g.v.count, DK_GRAD, s),
+              view(po[2], g.w.count, DK_GRAD, s), scale, g.G + (int)(e - r * fx.d), g.G + (int)(r - z * fy.d),
+              g.G + (int)z);
     END_ELEMS
     END_TILES
 }
@@ -780,7 +788,9 @@ __device__ __forceinline__ void warp_max_commit(unsigned long long m, unsigned l
 // running maximum over consecutive tiles of one slot and commits it (one
 // atomic per warp) when the slot changes or the block finishes, so the
 // atomics are per block, not per warp-sized tile.  In the loop a converged
-// slot is skipped.
+// slot is skipped.  Of the seven binary64 operations the x and y neighbour
+// sums run on the integer pipe (the last difference cancels too deeply for
+// it); 256^3: 268 us with none there, 209 so.
 __global__ void kb_residual(const InstDev* inst, Status* st, Ctl* ctl, Tab tab, int gate, int in_loop) {
     begin_slot(inst, tab);
     int held = -1;
@@ -807,21 +817,20 @@ __global__ void kb_residual(const InstDev* inst, Status* st, Ctl* ctl, Tab tab, 
             if (el >= n) continue;
             const unsigned e = (unsigned)el, r2 = I.fnx.div(e), zz = I.fny.div(r2);
             const int xi = (int)(e - r2 * (unsigned)g.NX), yi = (int)(r2 - zz * (unsigned)g.NY), zi = (int)zz;
-            const long long sy = g.p.sy, sz = g.p.sz;
-            const long long i = (g.G + xi) + (g.G + yi) * sy + (g.G + zi) * sz;
+            const int sy = (int)g.p.sy, sz = (int)g.p.sz;  // a field holds < 2^31 elements
+            const int i = (g.G + xi) + (g.G + yi) * sy + (g.G + zi) * sz;
+            // A neighbour across a wall is the cell itself.
             const double pc = p[i];
-            const double xm = xi > 0 ? p[i - 1] : pc;
-            const double xp = xi < g.NX - 1 ? p[i + 1] : pc;
-            const double ym = yi > 0 ? p[i - sy] : pc;
-            const double yp = yi < g.NY - 1 ? p[i + sy] : pc;
-            const double zm = zi > 0 ? p[i - sz] : pc;
-            const double zp = zi < g.NZ - 1 ? p[i + sz] : pc;
-            const double res = bb[i] - fma(-6.0, pc, ((xm + xp) + (ym + yp)) + (zm + zp));
+            const double xm = p[xi > 0 ? i - 1 : i], xp = p[xi < g.NX - 1 ? i + 1 : i];
+            const double ym = p[yi > 0 ? i - sy : i], yp = p[yi < g.NY - 1 ? i + sy : i];
+            const double zm = p[zi > 0 ? i - sz : i], zp = p[zi < g.NZ - 1 ? i + sz : i];
+            const double sum = dadd(dadd(dadd_int(xm, xp), dadd_int(ym, yp)), dadd(zm, zp));
+            const double res = dsub(bb[i], __fma_rn(-6.0, pc, sum));
             r0[el] = f64_to_f32(res);
             e0[el] = 0.0f;
             // |res| and NaN on the bit pattern (integer pipe); NaN reads as
             // +Inf so the loop stops.
-            const unsigned long long a = (unsigned long long)__double_as_longlong(res) & ~kSign;
+            const unsigned long long a = dbits(res) & ~kSign;
             const unsigned long long v = a > 0x7FF0000000000000ull ? 0x7FF0000000000000ull : a;
             m = v > m ? v : m;
         }
@@ -1895,7 +1904,7 @@ long long stage_items(const Batch* b, const SlotHost& S, int st, const Shape& sh
     long long n = 0;
     if (st == S_BC) n = bc_count(I.g);
     else if (st == S_SWEEP) n = sweep_box(I.g);
-    else if (st == S_GRAD) n = 32ll * 3 * (I.g.NY + 1) * (I.g.NZ + 1);
+    else if (st == S_GRAD) n = (long long)(I.g.NX + 1) * (I.g.NY + 1) * (I.g.NZ + 1);
     else if (st == S_SHADOW) n = I.shq[3];
     else if (st == S_SWEEPT) return I.sw_tiles;
     else if (st == S_DIV) n = (long long)I.g.p.nx * I.g.p.ny * I.g.p.nz;

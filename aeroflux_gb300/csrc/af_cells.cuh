@@ -315,30 +315,33 @@ __device__ __forceinline__ void div_cell(const Geom& g, AF_PTR(const double) AF_
 }
 
 // --- subtractGradient, project.go:172-205 ----------------------------------
-// Face (x, y, z) of component c, inside that component's write range: the
-// new value of the face of f (the component's field) is stored to out at the
-// same index -- f itself for the reference's in-place update.
-__device__ __forceinline__ void grad_face_to(const Geom& g, AF_PTR(const double) AF_RESTRICT p,
-                                             AF_PTR(const double) f, AF_PTR(double) out, const exact::MulC& scale, int c, int x,
-                                             int y, int z) {
-    const long long ip = x + y * g.p.sy + z * g.p.sz;
-    if (c == 0) {
-        const long long i = x + y * g.u.sy + z * g.u.sz;
-        out[i] = dsub(f[i], exact::mulc(scale, dsub(p[ip], p[ip - 1])));
-    } else if (c == 1) {
-        const long long i = x + y * g.v.sy + z * g.v.sz;
-        out[i] = dsub(f[i], exact::mulc(scale, dsub(p[ip], p[ip - g.p.sy])));
-    } else {
-        const long long i = x + y * g.w.sy + z * g.w.sz;
-        out[i] = dsub(f[i], exact::mulc(scale, dsub(p[ip], p[ip - g.p.sz])));
-    }
-}
-
-__device__ __forceinline__ void grad_face(const Geom& g, AF_PTR(const double) AF_RESTRICT p, AF_PTR(double) u,
-                                          AF_PTR(double) v, AF_PTR(double) w, const exact::MulC& scale, int c, int x, int y,
+// The three lower faces of cell (x, y, z) of the box one cell larger than the
+// interior, those inside their component's write range: new values of the
+// faces of u, v, w to ou, ov, ow -- the same fields for the reference's
+// in-place update.  One thread for the three shares the cell's own pressure
+// and the index arithmetic; the products are integer instructions, so a face
+// leaves two subtractions to the binary64 pipe.
+__device__ __forceinline__ void grad_cell(const Geom& g, AF_PTR(const double) AF_RESTRICT p, AF_PTR(const double) u,
+                                          AF_PTR(const double) v, AF_PTR(const double) w, AF_PTR(double) ou,
+                                          AF_PTR(double) ov, AF_PTR(double) ow, const exact::MulC& scale, int x, int y,
                                           int z) {
-    AF_PTR(double) f = c == 0 ? u : (c == 1 ? v : w);
-    grad_face_to(g, p, f, f, scale, c, x, y, z);
+    const int psy = (int)g.p.sy, psz = (int)g.p.sz;  // a field holds < 2^31 elements
+    const int ip = x + y * psy + z * psz;
+    const bool xi = x < g.G + g.NX, yi = y < g.G + g.NY, zi = z < g.G + g.NZ;
+    const int iu = x + y * (int)g.u.sy + z * (int)g.u.sz, iv = x + y * (int)g.v.sy + z * (int)g.v.sz;
+    const int iw = x + y * (int)g.w.sy + z * (int)g.w.sz;
+    // Every load before the first store, which may alias the fields.
+    const double pc = p[ip];
+    double px = 0.0, py = 0.0, pz = 0.0, fu = 0.0, fv = 0.0, fw = 0.0;
+    if (yi && zi) px = p[ip - 1], fu = u[iu];
+    if (xi && zi) py = p[ip - psy], fv = v[iv];
+    if (xi && yi) pz = p[ip - psz], fw = w[iw];
+    fu = dsub(fu, exact::mulc(scale, dsub(pc, px)));
+    fv = dsub(fv, exact::mulc(scale, dsub(pc, py)));
+    fw = dsub(fw, exact::mulc(scale, dsub(pc, pz)));
+    if (yi && zi) ou[iu] = fu;
+    if (xi && zi) ov[iv] = fv;
+    if (xi && yi) ow[iw] = fw;
 }
 
 // --- binary64 <-> binary32 on the integer pipe -----------------------------
@@ -348,7 +351,7 @@ __device__ __forceinline__ void grad_face(const Geom& g, AF_PTR(const double) AF
 // Round half away from zero on the magnitude; below FLT_MIN flushes to zero;
 // Inf/NaN kept.
 __device__ __forceinline__ float f64_to_f32(double d) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(d);
+    const unsigned long long b = dbits(d);
     const unsigned hi = (unsigned)(b >> 32), lo = (unsigned)b;
     const unsigned sign = hi & 0x80000000u;
     const int e = (int)((hi >> 20) & 0x7FF);
