@@ -942,7 +942,8 @@ __device__ __forceinline__ float mg_relax(const LevelOrWeights& L, float sx, flo
     return __fmaf_rn(kMgOmega, __fsub_rn(v, c), c);
 }
 // Residual of one cell: r - (wx*dxx + wy*dyy + wz*dzz), d** the second differences.
-__device__ __forceinline__ float mg_res(const Lvl& L, float sx, float sy, float sz, float c, float r) {
+template <class LevelOrWeights>
+__device__ __forceinline__ float mg_res(const LevelOrWeights& L, float sx, float sy, float sz, float c, float r) {
     const float c2 = 2.0f * c;
     return __fsub_rn(r, __fmaf_rn(L.wz, __fsub_rn(sz, c2), __fmaf_rn(L.wy, __fsub_rn(sy, c2), __fmul_rn(L.wx, __fsub_rn(sx, c2)))));
 }
@@ -1531,132 +1532,342 @@ __global__ void __launch_bounds__(kMarchT[K], kMarchBlocks[K])
 // a Neumann problem is solvable only for zero-mean data -- red-black sweeps
 // from zero, the mean of e removed), then prolongation and post-smoothing
 // back up.  Sums use a fixed tree.  Replaces one launch per level and sweep.
-// One colour: the threads walk that colour's cells only, (nx+1)/2 slots per
-// (y, z) row (the last one past the row when the row's colour count is
-// smaller), so a sweep costs half the index decoding of a walk over all cells.
-__device__ void sm_smooth(const Lvl& L, AF_PTR(float) e, AF_PTR(const float) r, int color) {
-    const int hx = (L.nx + 1) / 2, m = hx * L.ny * L.nz, nxy = L.nx * L.ny;
-    const float inv = 1.0f / (2.0f * (L.wx + L.wy + L.wz));
-    for (int j = threadIdx.x; j < m; j += blockDim.x) {
-        const unsigned q = L.fhx.div((unsigned)j), zz = L.fny.div(q);
-        const int y = (int)q - (int)zz * L.ny, z = (int)zz;
-        const int x = (((y + z) & 1) != color ? 1 : 0) + 2 * (j - (int)q * hx);
-        if (x >= L.nx) continue;
-        const int i = x + L.nx * (int)q;
-        const float c = e[i];
-        const float sx = (x > 0 ? e[i - 1] : c) + (x < L.nx - 1 ? e[i + 1] : c);
-        const float sy = (y > 0 ? e[i - L.nx] : c) + (y < L.ny - 1 ? e[i + L.nx] : c);
-        const float sz = (z > 0 ? e[i - nxy] : c) + (z < L.nz - 1 ? e[i + nxy] : c);
-        e[i] = mg_relax(L, sx, sy, sz, r[i], inv, c);
+//
+// It is a chain of short phases, so each is kept short.  e carries a ghost
+// cell on each side of every axis longer than one cell, which always holds
+// the value of the wall cell beside it (the Neumann reflection; an update of
+// a wall cell writes its ghosts too), so neighbours sit at fixed offsets
+// without tests.  A thread keeps its cells of a level -- index, walls, r and
+// its own e -- in registers over all of the level's sweeps.  From the first
+// level of at most kWarpSlots cells a colour on, one warp runs the rest of
+// the way down and back up with warp barriers instead of block ones.
+// A visit's loops appear once and work on copies of its levels' records, and
+// shared memory is indexed as such: the chain otherwise waits on instruction
+// fetches and generic loads.  Measured per Step with index decoding, wall
+// tests and block barriers in every sweep / so: 16^3 (a tail alone, 14
+// V-cycles) 0.72 / 0.59 ms, 48x32x64 1.44 / 1.38 ms, 256^3 10.40 / 10.27 ms.
+constexpr int kWarpSlots = 128;
+
+// A level's layout in shared memory: strides along the axes (0 along an axis
+// of extent 1), offset of cell (0, 0, 0) and floats of e; r is unpadded.
+struct SmLvl {
+    int nx, ny, nz, hx, dx, dy, dz, o, size;
+    SmLvl() = default;
+    __host__ __device__ explicit SmLvl(const Lvl& L) : nx(L.nx), ny(L.ny), nz(L.nz), hx((L.nx + 1) / 2) {
+        const int px = nx > 1 ? nx + 2 : 1, py = ny > 1 ? ny + 2 : 1, pz = nz > 1 ? nz + 2 : 1;
+        dx = nx > 1 ? 1 : 0;
+        dy = ny > 1 ? px : 0;
+        dz = nz > 1 ? px * py : 0;
+        o = dx + dy + dz;
+        size = px * py * pz;
     }
-    __syncthreads();
+    __host__ __device__ int cells() const { return nx * ny * nz; }
+    __host__ __device__ int slots() const { return hx * ny * nz; }  // of one colour
+};
+
+// What the tail reads of a level, in shared memory: its layout, the places of
+// e (cell (0, 0, 0)) and r, weights, dividers, the axes that coarsen.
+struct TailLvl {
+    SmLvl S;
+    MgW W;
+    float inv;  // of the relaxation
+    int e, e0, r;  // cell (0, 0, 0) and start of e, start of r
+    int res;       // residuals of the level being restricted
+    int cx, cy, cz;
+    FastDiv fnx, fny, fhx;
+    // Which walls a cell touches: bit 0 x low, 1 x high, 2 y low, ...
+    __device__ __forceinline__ unsigned walls(int x, int y, int z) const {
+        unsigned w = 0;
+        if (S.nx > 1) w |= (x == 0 ? 1u : 0u) | (x == S.nx - 1 ? 2u : 0u);
+        if (S.ny > 1) w |= (y == 0 ? 4u : 0u) | (y == S.ny - 1 ? 8u : 0u);
+        if (S.nz > 1) w |= (z == 0 ? 16u : 0u) | (z == S.nz - 1 ? 32u : 0u);
+        return w;
+    }
+    __device__ __forceinline__ int at(int x, int y, int z) const { return e + x * S.dx + y * S.dy + z * S.dz; }
+    // Cell of linear index i.
+    __device__ __forceinline__ void cell(int i, int* x, int* y, int* z) const {
+        const unsigned q = fnx.div((unsigned)i), zz = fny.div(q);
+        *x = i - (int)q * S.nx, *y = (int)q - (int)zz * S.ny, *z = (int)zz;
+    }
+};
+
+// The tail's dynamic shared memory, indexed as such (a pointer handed to a
+// function would make every access a generic one); the bounds-checking build
+// checks the index.
+struct TailMem {
+    int n, slot;
+    __device__ __forceinline__ float& operator[](int i) const {
+        extern __shared__ __align__(128) float tail_smem[];
+#if AEROFLUX_DEBUG_BOUNDS
+        return view(tail_smem, (long long)n, DK_VTAIL, slot)[i];
+#else
+        return tail_smem[i];
+#endif
+    }
+};
+
+__device__ __forceinline__ void tail_put(const TailMem& M, const SmLvl& S, int i, unsigned w, float v) {
+    M[i] = v;
+    if (w) {
+        if (w & 1u) M[i - S.dx] = v;
+        if (w & 2u) M[i + S.dx] = v;
+        if (w & 4u) M[i - S.dy] = v;
+        if (w & 8u) M[i + S.dy] = v;
+        if (w & 16u) M[i - S.dz] = v;
+        if (w & 32u) M[i + S.dz] = v;
+    }
 }
 
-__device__ __forceinline__ float sm_res(const Lvl& L, AF_PTR(const float) e, AF_PTR(const float) r, int x, int y,
-                                        int z) {
-    const int nxy = L.nx * L.ny;
-    const int i = x + L.nx * y + nxy * z;
-    const float c = e[i];
-    const float sx = (x > 0 ? e[i - 1] : c) + (x < L.nx - 1 ? e[i + 1] : c);
-    const float sy = (y > 0 ? e[i - L.nx] : c) + (y < L.ny - 1 ? e[i + L.nx] : c);
-    const float sz = (z > 0 ? e[i - nxy] : c) + (z < L.nz - 1 ? e[i + nxy] : c);
-    return mg_res(L, sx, sy, sz, c, r[i]);
+// The threads that run a level: the block, or its first warp.
+template <bool WARP>
+struct TailGroup {
+    static constexpr int N = WARP ? 32 : kCoarseThreads;
+    static __device__ __forceinline__ int id() { return (int)threadIdx.x; }
+    static __device__ __forceinline__ void sync() {
+        if (WARP) __syncwarp();
+        else __syncthreads();
+    }
+};
+
+// `pairs` red-black pairs of a level, NC cells of a colour a thread at most.
+template <bool WARP, int NC>
+__device__ __forceinline__ void tail_smooth_n(const TailMem& M, const TailLvl& L, int pairs) {
+    using Gr = TailGroup<WARP>;
+    const SmLvl S = L.S;
+    const MgW W = L.W;
+    const float inv = L.inv;
+    int at[2][NC];  // walls << 20 | index; -1: none
+    float rr[2][NC], own[2][NC];
+#pragma unroll
+    for (int k = 0; k < NC; ++k) {
+        const int m = Gr::id() + k * Gr::N;
+        const unsigned q = L.fhx.div((unsigned)m), zz = L.fny.div(q);
+        const int j = m - (int)q * S.hx, y = (int)q - (int)zz * S.ny, z = (int)zz;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const int x = 2 * j + (((y + z) & 1) != c ? 1 : 0);
+            at[c][k] = -1;
+            rr[c][k] = own[c][k] = 0.0f;
+            if (m < S.slots() && x < S.nx) {
+                const int i = L.at(x, y, z);
+                at[c][k] = (int)(L.walls(x, y, z) << 20) | i;
+                rr[c][k] = M[L.r + x + S.nx * (int)q];
+                own[c][k] = M[i];
+            }
+        }
+    }
+    for (int p = 0; p < pairs; ++p)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+#pragma unroll
+            for (int k = 0; k < NC; ++k)
+                if (at[c][k] >= 0) {
+                    const int i = at[c][k] & 0xFFFFF;
+                    const float v = mg_relax(W, M[i - S.dx] + M[i + S.dx], M[i - S.dy] + M[i + S.dy],
+                                             M[i - S.dz] + M[i + S.dz], rr[c][k], inv, own[c][k]);
+                    own[c][k] = v;
+                    tail_put(M, S, i, (unsigned)at[c][k] >> 20, v);
+                }
+            Gr::sync();
+        }
 }
 
-__global__ void __launch_bounds__(kCoarseThreads) kb_vtail(const InstDev* inst, const Ctl* ctl, Tab tab, int nu,
-                                                           int vc) {
+// Thin levels of more slots than four a thread (half of a row's slots may be
+// of no colour): decoded in every sweep.
+__device__ __noinline__ void tail_smooth_thin(const TailMem M, const TailLvl* lv, int pairs) {
+    const TailLvl L = *lv;
+    const SmLvl& S = L.S;
+    for (int p = 0; p < 2 * pairs; ++p) {
+        for (int m = (int)threadIdx.x; m < S.slots(); m += kCoarseThreads) {
+            const unsigned q = L.fhx.div((unsigned)m), zz = L.fny.div(q);
+            const int j = m - (int)q * S.hx, y = (int)q - (int)zz * S.ny, z = (int)zz;
+            const int x = 2 * j + (((y + z) & 1) != (p & 1) ? 1 : 0);
+            if (x >= S.nx) continue;
+            const int i = L.at(x, y, z);
+            const float v = mg_relax(L.W, M[i - S.dx] + M[i + S.dx], M[i - S.dy] + M[i + S.dy],
+                                     M[i - S.dz] + M[i + S.dz], M[L.r + x + S.nx * (int)q], L.inv, M[i]);
+            tail_put(M, S, i, L.walls(x, y, z), v);
+        }
+        __syncthreads();
+    }
+}
+
+// Sum over the coarsest level's cells in the fixed order of 512 threads: a
+// partial each over cells i, i + 512, ..., a shuffle tree over each warp, one
+// over the warps.  One warp forms the same tree where the level has at most
+// 256 cells.
+template <bool WARP, class F>
+__device__ __forceinline__ float tail_sum(int n, float* red, F cell) {
+    if (!WARP) {
+        float part = 0.0f;
+        for (int i = (int)threadIdx.x; i < n; i += kCoarseThreads) part += cell(i);
+        return block_sum(part, red);
+    }
+    const int lane = (int)threadIdx.x;
+    float mine = 0.0f;
+    for (int w = 0; w * 32 < n; ++w) {
+        const int i = w * 32 + lane;
+        float v = i < n ? 0.0f + cell(i) : 0.0f;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane == w) mine = v;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
+    return __shfl_sync(0xffffffffu, mine, 0);
+}
+
+// Levels l0 .. nl - 1 (lv[l]): down, the coarsest solve, and back up to l0.
+// One loop over the visits, each part of a visit written once (the chain of
+// short phases waits on instruction fetches otherwise); a visit works on a
+// copy of its levels' records (stores could alias the table).
+template <bool WARP>
+__device__ __noinline__ void tail_levels(const TailMem M, const TailLvl* lv, int l0, int nl, int coarse_sweeps,
+                                         float* red, int nu) {
+    using Gr = TailGroup<WARP>;
+    bool up = false;
+    for (int l = l0; l >= l0;) {
+        if (!WARP && !up && lv[l].S.slots() <= kWarpSlots) {
+            if (threadIdx.x < 32) tail_levels<true>(M, lv, l, nl, coarse_sweeps, red, nu);
+            __syncthreads();
+            up = true;
+            --l;
+            continue;
+        }
+        const TailLvl F = lv[l];
+        const bool coarsest = l == nl - 1;
+        const int n = F.S.cells();
+        if (up) {  // prolongation
+            const TailLvl C = lv[l + 1];
+            // A thread takes the fine cells 2X and 2X + 1 of a parent column X
+            // where x coarsens: they share four coarse values.  The next coarse
+            // cell toward the fine one is the parent again across a wall (edge
+            // and corner ghosts are unset).
+            const float ax = F.cx ? 0.75f : 1.0f, ay = F.cy ? 0.75f : 1.0f, az = F.cz ? 0.75f : 1.0f;
+            const int items = C.S.nx * F.S.ny * F.S.nz;
+            for (int j = Gr::id(); j < items; j += Gr::N) {
+                const unsigned q = C.fnx.div((unsigned)j), zz = F.fny.div(q);
+                const int X = j - (int)q * C.S.nx, y = (int)q - (int)zz * F.S.ny, z = (int)zz;
+                const int Y = F.cy ? y >> 1 : y, Z = F.cz ? z >> 1 : z;
+                auto toward = [](int coarsens, int f, int c, int m, int d) {
+                    return !coarsens ? 0 : ((f & 1) ? (c < m - 1 ? d : 0) : (c > 0 ? -d : 0));
+                };
+                const int k = C.at(X, Y, Z);
+                const int oy = toward(F.cy, y, Y, C.S.ny, C.S.dy), oz = toward(F.cz, z, Z, C.S.nz, C.S.dz);
+                const float a = M[k], b = M[k + oy], c = M[k + oz], d = M[k + oz + oy];
+#pragma unroll
+                for (int o = 0; o < 2; ++o) {
+                    if (o && !F.cx) break;
+                    const int x = F.cx ? 2 * X + o : X, ox = toward(F.cx, o, X, C.S.nx, C.S.dx);
+                    const float v = mg_interp(ax, ay, az, a, M[k + ox], b, M[k + oy + ox], c, M[k + oz + ox], d,
+                                              M[k + oz + oy + ox]);
+                    const int i = F.at(x, y, z);
+                    tail_put(M, F.S, i, F.walls(x, y, z), __fadd_rn(M[i], v));
+                }
+            }
+            Gr::sync();
+        }
+        if (coarsest) {
+            const float mean_r = tail_sum<WARP>(n, red, [&](int i) { return M[F.r + i]; }) / (float)n;
+            for (int i = Gr::id(); i < n; i += Gr::N) M[F.r + i] -= mean_r;
+            for (int i = Gr::id(); i < F.S.size; i += Gr::N) M[F.e0 + i] = 0.0f;
+            Gr::sync();
+        }
+        const int pairs = coarsest ? coarse_sweeps : nu;
+        if (F.S.slots() <= Gr::N) tail_smooth_n<WARP, 1>(M, F, pairs);
+        else if (WARP || F.S.slots() <= 4 * Gr::N) tail_smooth_n<WARP, 4>(M, F, pairs);
+        else tail_smooth_thin(M, lv + l, pairs);
+        if (coarsest) {
+            const float mean_e = tail_sum<WARP>(n, red, [&](int i) {
+                int x, y, z;
+                F.cell(i, &x, &y, &z);
+                return M[F.at(x, y, z)];
+            }) / (float)n;
+            Gr::sync();
+            for (int i = Gr::id(); i < n; i += Gr::N) {
+                int x, y, z;
+                F.cell(i, &x, &y, &z);
+                const int k = F.at(x, y, z);
+                tail_put(M, F.S, k, F.walls(x, y, z), M[k] - mean_e);
+            }
+            Gr::sync();
+            up = true;
+        } else if (!up) {  // restriction
+            // Every cell's residual once, then the means of the children in
+            // their order.
+            const TailLvl C = lv[l + 1];
+            const SmLvl& S = F.S;
+            for (int j = Gr::id(); j < n; j += Gr::N) {
+                int x, y, z;
+                F.cell(j, &x, &y, &z);
+                const int i = F.at(x, y, z);
+                M[F.res + j] = mg_res(F.W, M[i - S.dx] + M[i + S.dx], M[i - S.dy] + M[i + S.dy],
+                                      M[i - S.dz] + M[i + S.dz], M[i], M[F.r + j]);
+            }
+            Gr::sync();
+            const int ex = F.cx ? 2 : 1, ey = F.cy ? 2 : 1, ez = F.cz ? 2 : 1;
+            const float inv = 1.0f / (float)(ex * ey * ez);
+            for (int j = Gr::id(); j < C.S.cells(); j += Gr::N) {
+                int X, Y, Z;
+                C.cell(j, &X, &Y, &Z);
+                const int i = F.res + X * ex + S.nx * (Y * ey + S.ny * (Z * ez));
+                float sum = 0.0f;
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+                    if (((k & 1) == 0 || F.cx) && ((k & 2) == 0 || F.cy) && ((k & 4) == 0 || F.cz))
+                        sum += M[i + (k & 1) + ((k >> 1) & 1) * S.nx + (k >> 2) * S.nx * S.ny];
+                M[C.r + j] = sum * inv;
+            }
+            for (int j = Gr::id(); j < C.S.size; j += Gr::N) M[C.e0 + j] = 0.0f;
+            Gr::sync();
+        }
+        l += up ? -1 : 1;
+    }
+}
+
+__global__ void __launch_bounds__(kCoarseThreads) kb_vtail(const InstDev* inst, const TailLvl* tables,
+                                                           const Ctl* ctl, Tab tab, int nu, int vc) {
     begin_slot(inst, tab);
     if (vc_idle(ctl, tab.n, vc)) return;
-    extern __shared__ float tsm[];
     __shared__ float red[32];
+    __shared__ __align__(8) TailLvl lv[kMaxLev];
     for (int item = blockIdx.x, total = tab.prefix[tab.n]; item < total; item += gridDim.x) {
         const int s = find_slot(tab.prefix, tab.n, item);
         if (mg_off(ctl[s], vc)) continue;
         const InstDev& I = inst[s];
-        const int t = I.tail, nl = I.nlev;
-        AF_PTR(float) E[kMaxLev];
-        AF_PTR(float) R[kMaxLev];
-        {
-            float* p = tsm;
-            for (int l = t; l < nl; ++l) {
-                const int n = lvl_cells(I.lev[l]);
-                E[l] = view(p, (long long)n, DK_VTAIL, s);
-                R[l] = view(p + n, (long long)n, DK_VTAIL, s);
-                p += 2 * n;
-            }
+        const int t = I.tail, nl = I.nlev, cs = I.coarse_sweeps;
+        const TailMem M{I.tail_floats, s};
+        AF_PTR(float) te = view(I.lev[t].e, lvl_cells(I.lev[t]), DK_VTAIL, s);
+        AF_PTR(const float) tr = view((const float*)I.lev[t].r, lvl_cells(I.lev[t]), DK_VTAIL, s);
+        static_assert(sizeof(TailLvl) % 4 == 0, "the table is copied by words");
+        for (int k = threadIdx.x; k < (int)sizeof(lv) / 4; k += kCoarseThreads)
+            ((unsigned*)lv)[k] = ((const unsigned*)(tables + (size_t)s * kMaxLev))[k];
+        __syncthreads();
+        const TailLvl T = lv[t];
+        const int n = T.S.cells();
+        float ve[kCoarseMax / kCoarseThreads], vr[kCoarseMax / kCoarseThreads];
+#pragma unroll
+        for (int k = 0; k < kCoarseMax / kCoarseThreads; ++k) {
+            const int i = (int)threadIdx.x + k * kCoarseThreads;
+            if (i < n) ve[k] = te[i], vr[k] = tr[i];
         }
-        const Lvl T = I.lev[t];
-        AF_PTR(float) te = view(T.e, lvl_cells(T), DK_VTAIL, s);
-        AF_PTR(const float) tr = view((const float*)T.r, lvl_cells(T), DK_VTAIL, s);
-        for (int i = threadIdx.x; i < lvl_cells(T); i += blockDim.x) {
-            E[t][i] = te[i];
-            R[t][i] = tr[i];
+#pragma unroll
+        for (int k = 0; k < kCoarseMax / kCoarseThreads; ++k) {
+            const int i = (int)threadIdx.x + k * kCoarseThreads;
+            if (i < n) {
+                int x, y, z;
+                T.cell(i, &x, &y, &z);
+                tail_put(M, T.S, T.at(x, y, z), T.walls(x, y, z), ve[k]);
+                M[T.r + i] = vr[k];
+            }
         }
         __syncthreads();
-        for (int l = t; l + 1 < nl; ++l) {
-            const Lvl F = I.lev[l], C = I.lev[l + 1];
-            for (int k = 0; k < nu; ++k) {
-                sm_smooth(F, E[l], R[l], 0);
-                sm_smooth(F, E[l], R[l], 1);
-            }
-            const int ex = F.cx ? 2 : 1, ey = F.cy ? 2 : 1, ez = F.cz ? 2 : 1;
-            const float inv = 1.0f / (float)(ex * ey * ez);
-            for (int j = threadIdx.x; j < lvl_cells(C); j += blockDim.x) {
-                const unsigned q = C.fnx.div((unsigned)j), zz = C.fny.div(q);
-                const int X = j - (int)q * C.nx, Y = (int)q - (int)zz * C.ny, Z = (int)zz;
-                float sum = 0.0f;
-                for (int dz = 0; dz < ez; ++dz)
-                    for (int dy = 0; dy < ey; ++dy)
-                        for (int dx = 0; dx < ex; ++dx) sum += sm_res(F, E[l], R[l], X * ex + dx, Y * ey + dy, Z * ez + dz);
-                R[l + 1][j] = sum * inv;
-                E[l + 1][j] = 0.0f;
-            }
-            __syncthreads();
+        tail_levels<false>(M, lv, t, nl, cs, red, nu);
+        for (int i = threadIdx.x; i < n; i += kCoarseThreads) {
+            int x, y, z;
+            T.cell(i, &x, &y, &z);
+            te[i] = M[T.at(x, y, z)];
         }
-        {  // coarsest solve
-            const Lvl C = I.lev[nl - 1];
-            const int n = lvl_cells(C);
-            float part = 0.0f;
-            for (int i = threadIdx.x; i < n; i += blockDim.x) part += R[nl - 1][i];
-            const float mean_r = block_sum(part, red) / (float)n;
-            for (int i = threadIdx.x; i < n; i += blockDim.x) {
-                R[nl - 1][i] -= mean_r;
-                E[nl - 1][i] = 0.0f;
-            }
-            __syncthreads();
-            for (int k = 0; k < I.coarse_sweeps; ++k) {
-                sm_smooth(C, E[nl - 1], R[nl - 1], 0);
-                sm_smooth(C, E[nl - 1], R[nl - 1], 1);
-            }
-            part = 0.0f;
-            for (int i = threadIdx.x; i < n; i += blockDim.x) part += E[nl - 1][i];
-            const float mean_e = block_sum(part, red) / (float)n;
-            for (int i = threadIdx.x; i < n; i += blockDim.x) E[nl - 1][i] -= mean_e;
-            __syncthreads();
-        }
-        for (int l = nl - 2; l >= t; --l) {
-            const Lvl F = I.lev[l], C = I.lev[l + 1];
-            for (int i = threadIdx.x; i < lvl_cells(F); i += blockDim.x) {
-                const unsigned q = F.fnx.div((unsigned)i), zz = F.fny.div(q);
-                const int x = i - (int)q * F.nx, y = (int)q - (int)zz * F.ny, z = (int)zz;
-                int X0 = x, X1 = x, Y0 = y, Y1 = y, Z0 = z, Z1 = z;
-                float ax = 1.0f, ay = 1.0f, az = 1.0f;
-                if (F.cx) { X0 = x >> 1; X1 = min(max(X0 + ((x & 1) ? 1 : -1), 0), C.nx - 1); ax = 0.75f; }
-                if (F.cy) { Y0 = y >> 1; Y1 = min(max(Y0 + ((y & 1) ? 1 : -1), 0), C.ny - 1); ay = 0.75f; }
-                if (F.cz) { Z0 = z >> 1; Z1 = min(max(Z0 + ((z & 1) ? 1 : -1), 0), C.nz - 1); az = 0.75f; }
-                AF_PTR(const float) ec = E[l + 1];
-                auto Ev = [&](int a, int b, int c) { return ec[a + C.nx * (b + C.ny * c)]; };
-                E[l][i] = __fadd_rn(E[l][i], mg_interp(ax, ay, az, Ev(X0, Y0, Z0), Ev(X1, Y0, Z0), Ev(X0, Y1, Z0),
-                                                       Ev(X1, Y1, Z0), Ev(X0, Y0, Z1), Ev(X1, Y0, Z1), Ev(X0, Y1, Z1),
-                                                       Ev(X1, Y1, Z1)));
-            }
-            __syncthreads();
-            for (int k = 0; k < nu; ++k) {
-                sm_smooth(F, E[l], R[l], 0);
-                sm_smooth(F, E[l], R[l], 1);
-            }
-        }
-        for (int i = threadIdx.x; i < lvl_cells(T); i += blockDim.x) te[i] = E[t][i];
         __syncthreads();
     }
 }
@@ -1793,13 +2004,15 @@ struct Batch {
     cudaStream_t stream = nullptr;
     cudaStream_t body = nullptr;
     InstDev* d_inst = nullptr;
+    TailLvl* d_tails = nullptr;      // kMaxLev per slot: the tail levels' tables
+    std::vector<TailLvl> h_tails;
     Status* d_st = nullptr;
     Ctl* d_ctl = nullptr;
     int* d_tab = nullptr;            // S_COUNT prefix arrays of cap+1 ints
     std::vector<int> h_tab;
     Shape shape[S_COUNT];
     int grid_sz[S_COUNT] = {};       // blocks per stage, fixed when the graph is captured
-    int graph_levels = 0;            // levels the captured graph covers
+    int graph_levels = 0;            // levels the captured graph runs per-level kernels on
     unsigned graph_big = 0;          // levels whose large-coarsest smoothing the graph carries
     unsigned graph_pair = 0;         // levels with wide fused-pair tiles in the graph
     unsigned graph_pairn = 0;        // levels with narrow fused-pair tiles in the graph
@@ -1839,6 +2052,15 @@ int max_levels(const Batch* b) {
     return m;
 }
 
+// Levels some slot smooths and coarsens with per-level kernels.
+int slot_levels(const SlotHost& S) { return S.d.tail >= 0 ? S.d.tail : S.d.nlev - 1; }
+int kernel_levels(const Batch* b) {
+    int m = 0;
+    for (const auto& s : b->slots)
+        if (s.used) m = std::max(m, slot_levels(s));
+    return m;
+}
+
 // Levels at which some slot's coarsest grid is too large for the one-block
 // solver (smoothed in place instead).
 unsigned big_coarse_levels(const Batch* b) {
@@ -1853,7 +2075,7 @@ unsigned single_levels(const Batch* b) {
     unsigned m = 0;
     for (const auto& s : b->slots) {
         if (!s.used) continue;
-        const int lim = s.d.tail >= 0 ? s.d.tail : s.d.nlev - 1;
+        const int lim = slot_levels(s);
         for (int l = 0; l < lim; ++l)
             if (!s.d.lev[l].e2) m |= 1u << l;
     }
@@ -1868,7 +2090,7 @@ unsigned march_levels(const Batch* b) {
     unsigned m = 0;
     for (const auto& s : b->slots) {
         if (!s.used) continue;
-        const int lim = s.d.tail >= 0 ? s.d.tail : s.d.nlev - 1;
+        const int lim = slot_levels(s);
         for (int l = 0; l < lim; ++l)
             if (s.d.lev[l].e2 && marches(b, s, l)) m |= 1u << l;
     }
@@ -1880,7 +2102,7 @@ unsigned pair_levels(const Batch* b, bool narrow) {
     unsigned m = 0;
     for (const auto& s : b->slots) {
         if (!s.used) continue;
-        const int lim = s.d.tail >= 0 ? s.d.tail : s.d.nlev - 1;
+        const int lim = slot_levels(s);
         for (int l = 0; l < lim; ++l) {
             const Lvl& L = s.d.lev[l];
             if (L.e2 && !marches(b, s, l) && (narrow ? L.nxw < L.nx : L.nxw > 0)) m |= 1u << l;
@@ -1979,6 +2201,9 @@ cudaError_t upload_tables(Batch* b) {
                               b->stream)) != cudaSuccess)
         return rc;
     if (b->tmaps_dirty) {
+        if ((rc = cudaMemcpyAsync(b->d_tails, b->h_tails.data(), b->h_tails.size() * sizeof(TailLvl),
+                                  cudaMemcpyHostToDevice, b->stream)) != cudaSuccess)
+            return rc;
         if ((rc = cudaMemcpyAsync(b->d_tmaps, b->h_tmaps.data(), b->h_tmaps.size() * sizeof(CUtensorMap),
                                   cudaMemcpyHostToDevice, b->stream)) != cudaSuccess)
             return rc;
@@ -2092,16 +2317,18 @@ void enq_level_smooth(Batch* b, int l, int vc, cudaStream_t s) {
 // skip it.
 void enq_vcycle(Batch* b, int vc, cudaStream_t s) {
     const int L = b->graph_levels;
-    for (int l = 0; l + 1 < L; ++l) {
+    for (int l = 0; l < L; ++l) {
         enq_level_smooth(b, l, vc, s);
         LAUNCH(b, S_RESTRICT + l, kb_restrict, b->d_inst, b->d_ctl, tab(b, S_RESTRICT + l), l, vc);
     }
-    launch_pdl(kb_vtail, dim3(grid(b, S_COARSE)), dim3(kCoarseThreads), b->tail_smem, s, b->d_inst, b->d_ctl,
-               tab(b, S_COARSE), b->nu, vc);
-    ++b->launches;
-    for (int l = 0; l < L; ++l)
+    if (b->tail_smem) {
+        launch_pdl(kb_vtail, dim3(grid(b, S_COARSE)), dim3(kCoarseThreads), b->tail_smem, s, b->d_inst, b->d_tails,
+                   b->d_ctl, tab(b, S_COARSE), b->nu, vc);
+        ++b->launches;
+    }
+    for (int l = 0; l < kMaxLev; ++l)
         if (b->graph_big & (1u << l)) enq_smooth(b, S_BIGCOARSE + l, l, 8 * b->nu, vc, s);
-    for (int l = L - 2; l >= 0; --l) {
+    for (int l = L - 1; l >= 0; --l) {
         LAUNCH(b, S_PROLONG + l, kb_prolong, b->d_inst, b->d_ctl, tab(b, S_PROLONG + l), l, vc);
         enq_level_smooth(b, l, vc, s);
     }
@@ -2251,7 +2478,7 @@ cudaError_t prepare(Batch* b) {
     cudaError_t rc;
     default_pair_variants(b);
     if (b->tables_dirty && (rc = upload_tables(b)) != cudaSuccess) return rc;
-    const int L = max_levels(b);
+    const int L = kernel_levels(b);
     const unsigned big = big_coarse_levels(b), pair = pair_levels(b, false), pairn = pair_levels(b, true),
                    single = single_levels(b), march = march_levels(b);
     const size_t tsm = tail_smem_bytes(b);
@@ -2408,6 +2635,7 @@ Batch* batch_create(int capacity, size_t pool_bytes, std::string* err) {
     if ((rc = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking)) != cudaSuccess ||
         (rc = cudaStreamCreateWithFlags(&b->body, cudaStreamNonBlocking)) != cudaSuccess ||
         (rc = cudaMalloc(&b->d_inst, sizeof(InstDev) * capacity)) != cudaSuccess ||
+        (rc = cudaMalloc(&b->d_tails, sizeof(TailLvl) * kMaxLev * (size_t)capacity)) != cudaSuccess ||
         (rc = cudaMalloc(&b->d_st, sizeof(Status) * capacity)) != cudaSuccess ||
         (rc = cudaMalloc(&b->d_ctl, sizeof(Ctl) * (capacity + 1))) != cudaSuccess ||
         (rc = cudaMalloc(&b->d_tab, sizeof(int) * (size_t)S_COUNT * (capacity + 1))) != cudaSuccess ||
@@ -2420,6 +2648,7 @@ Batch* batch_create(int capacity, size_t pool_bytes, std::string* err) {
     cudaMemsetAsync(b->d_ctl, 0, sizeof(Ctl) * (capacity + 1), b->stream);
     cudaMemsetAsync(b->d_diag, 0, sizeof(unsigned), b->stream);
     b->h_tmaps.assign(12 * (size_t)capacity, CUtensorMap{});
+    b->h_tails.assign(kMaxLev * (size_t)capacity, TailLvl{});
     // The fused pairs' tile variant for every level (0-2 and 4; 3: marching
     // where a slot's level allows it), instead of the tuned or size-based choice.
     if (const char* pv = getenv("AEROFLUX_PAIR_VARIANT")) b->force_pair_var = std::min(4, std::max(0, atoi(pv)));
@@ -2449,6 +2678,7 @@ void batch_destroy(Batch* b) {
         if (s.used && !b->use_pool) cudaFree(s.mem);
     if (b->use_pool) cudaFree(b->pool.base);
     cudaFree(b->d_inst);
+    cudaFree(b->d_tails);
     cudaFree(b->d_st);
     cudaFree(b->d_ctl);
     cudaFree(b->d_tab);
@@ -2520,8 +2750,27 @@ int plan_tail(const Lvl* lev, int n, int* floats, bool coarsest_only = false) {
     if (lvl_cells(lev[n - 1]) > kCoarseMax) return -1;
     int t = n - 1;
     while (!coarsest_only && t > 0 && lvl_cells(lev[t - 1]) <= kCoarseMax) --t;
-    for (int l = t; l < n; ++l) *floats += 2 * (int)lvl_cells(lev[l]);
+    for (int l = t; l < n; ++l) *floats += SmLvl(lev[l]).size + SmLvl(lev[l]).cells();
+    if (t + 1 < n) *floats += SmLvl(lev[t]).cells();  // the residuals of a restriction
     return t;
+}
+
+// The tail levels' table: places from 0 on, the residual scratch last.
+void plan_tail_table(const InstDev& I, TailLvl* lv) {
+    if (I.tail < 0) return;
+    int p = 0;
+    for (int l = I.tail; l < I.nlev; ++l) {
+        const Lvl& L = I.lev[l];
+        TailLvl& t = lv[l];
+        t.S = SmLvl(L);
+        t.W = MgW{L.wx, L.wy, L.wz};
+        t.inv = 1.0f / (2.0f * (L.wx + L.wy + L.wz));
+        t.e0 = p, t.e = p + t.S.o, t.r = p + t.S.size;
+        t.cx = L.cx, t.cy = L.cy, t.cz = L.cz;
+        t.fnx = L.fnx, t.fny = L.fny, t.fhx = L.fhx;
+        p += t.S.size + t.S.cells();
+    }
+    for (int l = I.tail; l < I.nlev; ++l) lv[l].res = p;
 }
 
 af_field_desc fdesc(int64_t* off, int64_t nx, int64_t ny, int64_t nz) {
@@ -2746,6 +2995,7 @@ int batch_assign(Batch* b, const af_config& c, char* arena, std::string* err) {
     }
     cudaMemsetAsync(p, 0, mg, b->stream);
     plan_march(I);
+    plan_tail_table(I, &b->h_tails[kMaxLev * (size_t)s]);
     const double half = c.dt * 0.5;  // aeroflux.go:353
     const double invH = 1.0 / c.h;
     I.dt_invh = (float)(half * invH);
@@ -2815,11 +3065,11 @@ cudaError_t batch_prepare_capture(Batch* b) {
     cudaError_t rc;
     default_pair_variants(b);
     if (b->tables_dirty && (rc = upload_tables(b)) != cudaSuccess) return rc;
-    if (max_levels(b) > b->graph_levels && b->graph) {
+    if (kernel_levels(b) > b->graph_levels && b->graph) {
         cudaGraphExecDestroy(b->graph);
         b->graph = nullptr;
     }
-    b->graph_levels = std::max(b->graph_levels, max_levels(b));
+    b->graph_levels = std::max(b->graph_levels, kernel_levels(b));
     b->graph_big |= big_coarse_levels(b);
     b->graph_pair |= pair_levels(b, false);
     b->graph_pairn |= pair_levels(b, true);
