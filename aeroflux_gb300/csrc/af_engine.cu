@@ -308,6 +308,17 @@ void swap_fields(Fields& f) {
     std::swap(f.w, f.t2);
 }
 
+// The red-black sweeps of one solve over the split arrays; returns the launches.
+int64_t enqueue_red_black(af_engine* e) {
+    const int64_t pairs = e->cfg.gauss_seidel_iters;
+    if (af::launch_rbgs_all_fp64(e->split, pairs, e->stream)) return 1;
+    for (int64_t it = 0; it < pairs; ++it) {
+        af::launch_rbgs_fp64(e->split, 0, e->stream);
+        af::launch_rbgs_fp64(e->split, 1, e->stream);
+    }
+    return 2 * pairs;
+}
+
 // project, project.go:12-34, FP64 plain form.
 void enqueue_project_fp64(af_engine* e, const Fields& f, int gate) {
     const Geom& g = e->geom;
@@ -318,13 +329,10 @@ void enqueue_project_fp64(af_engine* e, const Fields& f, int gate) {
     const double h2 = c.h * c.h;                    // project.go:107
     af::launch_divergence_fp64(g, f, &e->split, scale, h2, e->st, gate, s);
     rec(e, kEvRb + (gate == 3 ? 0 : 2));
-    for (int64_t it = 0; it < c.gauss_seidel_iters; ++it) {
-        af::launch_rbgs_fp64(e->split, 0, s);
-        af::launch_rbgs_fp64(e->split, 1, s);
-    }
+    const int64_t launches = enqueue_red_black(e);
     rec(e, kEvRb + (gate == 3 ? 1 : 3));
-    e->launches_per_step += 5 + 2 * c.gauss_seidel_iters;
-    e->rbgs_launches_per_step += 2 * c.gauss_seidel_iters;
+    e->launches_per_step += 5 + launches;
+    e->rbgs_launches_per_step += launches;
     af::launch_join_fp64(g, e->split, f.p, e->st, gate, s);
     af::launch_gradient_fp64(g, f, c.dt / (c.density * c.h), e->st, gate, s);  // project.go:179
     af::launch_velocity_bc(g, f.u, f.v, f.w, e->st, gate, s);
@@ -783,10 +791,7 @@ int af_phase_red_black(af_engine* e) {
     // as the divergence kernel would have left it.
     Fields f = e->fields();
     af::launch_split_from_div(e->geom, f.div, e->split, e->cfg.h * e->cfg.h, e->stream);
-    for (int64_t it = 0; it < e->cfg.gauss_seidel_iters; ++it) {
-        af::launch_rbgs_fp64(e->split, 0, e->stream);
-        af::launch_rbgs_fp64(e->split, 1, e->stream);
-    }
+    enqueue_red_black(e);
     af::launch_join_fp64(e->geom, e->split, f.p, e->st, 0, e->stream);
     AF_CUDA(e, cudaGetLastError());
     return sync_and_check(e);

@@ -30,6 +30,7 @@ inline unsigned cdiv(long long a, long long b) { return (unsigned)((a + b - 1) /
 // applyVelocityBC, stencil.go:246-315: 3 components x 3 write sets, each cell
 // written once (see bc_cell).
 __global__ void k_velocity_bc(Geom g, double* u, double* v, double* w, Status* st, int gate) {
+    pdl_wait();
     if (gated(st, gate)) return;
     const int comp = blockIdx.y / 3, set = blockIdx.y % 3;
     const BcComp c = bc_comp(g, comp, view(u, g.u.count, DK_F64_BC, 0), view(v, g.v.count, DK_F64_BC, 0),
@@ -284,6 +285,7 @@ dim3 face_grid(const Geom& g, dim3 block) {
 
 template <int AX>
 __global__ void k_sweep_fp64(const __grid_constant__ SweepArgs a) {
+    pdl_wait();
     if (gated(a.st, a.phase)) return;
     int c, x, y, z;
     if (!block_face(a, &c, &x, &y, &z)) return;
@@ -390,6 +392,7 @@ __device__ __forceinline__ void maccormack_face(const SweepArgs& a, const double
 template <int AX>
 __global__ void k_maccormack_fp64(const __grid_constant__ SweepArgs a, const double* fu, const double* fv,
                                   const double* fw) {
+    pdl_wait();
     if (gated(a.st, a.phase)) return;
     int c, x, y, z;
     if (!block_face(a, &c, &x, &y, &z)) return;
@@ -422,6 +425,7 @@ __global__ void k_divergence_fp64(const __grid_constant__ Geom g, const double* 
                                   const __grid_constant__ Split S, int with_b,
                                   const __grid_constant__ exact::MulC scale, const __grid_constant__ exact::MulC h2,
                                   Status* st, int gate) {
+    pdl_wait();
     if (gated(st, gate)) return;
     if (with_b) split_zero(S);
     const int xi = blockIdx.x * blockDim.x + threadIdx.x;
@@ -513,11 +517,121 @@ __global__ void __launch_bounds__(128) k_rbgs_fp64(const __grid_constant__ Split
     }
 }
 
+// ---------------------------------------------------------------------------
+// All the sweeps of one solve on a small grid, in one launch: a cluster of
+// kRbCluster blocks holds P in its shared memory.  Block k owns the rows
+// (y, z) from k * rows on, both colours; a thread owns up to NC cells of each
+// colour, whose B, own value and the shared-memory addresses of their six
+// neighbours -- in whichever block they lie; its own cell's across a wall --
+// it keeps in registers over all sweeps.  A colour costs the neighbour loads,
+// the update (the subtraction on the integer pipe: a thread waits for its own
+// chain here, and the first addition there would be a longer link than on the
+// binary64 pipe), one store and a cluster barrier.
+// us per colour, a launch each / so: 12^3 1.75 / 0.77, 16^3 1.75 / 0.68, 24^3
+// 1.88 / 1.33, 40x12x33 1.9 / 1.37, 28^3 1.88 / 1.84, 32^3 1.92 / 2.26: past
+// kRbMaxCells the binary64 pipe bounds it, of which a cluster has only its
+// SMs' share.
+// ---------------------------------------------------------------------------
+constexpr int kRbCluster = 16, kRbThreads = 512;
+constexpr int kRbMaxCells = 20480;
+
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// The address, in the cluster's shared window, of a block's copy of a
+// shared-memory address.
+__device__ __forceinline__ unsigned cluster_addr(unsigned addr, unsigned rank) {
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ double cluster_ld(unsigned addr) {
+    double v;
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <int NC>
+__global__ void __launch_bounds__(kRbThreads) k_rbgs_cluster(const __grid_constant__ Split S, long long pairs) {
+    extern __shared__ __align__(16) double rb_smem[];  // [colour][row of the block][half index]
+    pdl_wait();
+    const int rows = (S.NY * S.NZ + kRbCluster - 1) / kRbCluster;  // per block
+    const int mine = (int)cluster_rank(), row0 = mine * rows;
+    const int n = max(0, min(rows, S.NY * S.NZ - row0)) * S.hx;    // slots of a colour here
+    const unsigned base = (unsigned)__cvta_generic_to_shared(rb_smem);
+    AF_PTR(double) sm = view(rb_smem, 2ll * rows * S.hx, DK_F64_RBGS, 0);
+    AF_PTR(const double) b = view((const double*)S.b, 2 * S.bn, DK_F64_RBGS, 0);
+    AF_PTR(double) p = view(S.p, 2 * S.pn, DK_F64_RBGS, 0);
+    unsigned nb[2][NC][6];
+    int at[2][NC];
+    double bv[2][NC], own[2][NC];
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int k = 0; k < NC; ++k) {
+            const int t = (int)threadIdx.x + k * kRbThreads;
+            const int r = (int)S.fhx.div((unsigned)t), j = t - r * S.hx, row = row0 + r;
+            const int z = row / S.NY, y = row - z * S.NY;
+            const int q = (c + S.G + y + z) & 1, x = 2 * j + q;
+            at[c][k] = -1;
+            own[c][k] = bv[c][k] = 0.0;
+            if (t < n && x < S.NX) {
+                at[c][k] = c * rows * S.hx + t;
+                bv[c][k] = b[(c ? S.bn : 0) + j + S.hx * row];
+                // The other colour's cell at half index jj of a row.
+                auto other = [&](int rr, int jj) {
+                    const int k2 = rr / rows;
+                    return cluster_addr(base + 8u * (unsigned)(((c ^ 1) * rows + rr - k2 * rows) * S.hx + jj),
+                                        (unsigned)k2);
+                };
+                const unsigned self = cluster_addr(base + 8u * (unsigned)at[c][k], (unsigned)mine);
+                nb[c][k][0] = x > 0 ? other(row, (x - 1) >> 1) : self;
+                nb[c][k][1] = x < S.NX - 1 ? other(row, (x + 1) >> 1) : self;
+                nb[c][k][2] = y > 0 ? other(row - 1, j) : self;
+                nb[c][k][3] = y < S.NY - 1 ? other(row + 1, j) : self;
+                nb[c][k][4] = z > 0 ? other(row - S.NY, j) : self;
+                nb[c][k][5] = z < S.NZ - 1 ? other(row + S.NY, j) : self;
+            }
+        }
+    for (int i = (int)threadIdx.x; i < 2 * rows * S.hx; i += kRbThreads) sm[i] = 0.0;  // project.go:81-83
+    cluster_sync();
+    for (long long it = 0; it < pairs; ++it)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            double v[NC];
+#pragma unroll
+            for (int k = 0; k < NC; ++k)
+                if (at[c][k] >= 0)
+                    v[k] = rb_update<0x20>(cluster_ld(nb[c][k][0]), cluster_ld(nb[c][k][1]), cluster_ld(nb[c][k][2]),
+                                        cluster_ld(nb[c][k][3]), cluster_ld(nb[c][k][4]), cluster_ld(nb[c][k][5]),
+                                        bv[c][k]);
+#pragma unroll
+            for (int k = 0; k < NC; ++k)
+                if (at[c][k] >= 0) sm[at[c][k]] = own[c][k] = v[k];
+            cluster_sync();
+        }
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int k = 0; k < NC; ++k)
+            if (at[c][k] >= 0) {
+                const int t = (int)threadIdx.x + k * kRbThreads;
+                const int r = (int)S.fhx.div((unsigned)t), row = row0 + r, z = row / S.NY, y = row - z * S.NY;
+                p[(c ? S.pn : 0) + (t - r * S.hx + 1 + S.px * (y + 1) + S.plane * (z + 1))] = own[c][k];
+            }
+}
+
 // The split P into P: a ghost of the first layer holds the interior cell at
 // the clamped coordinates (applyPressureBC, project.go:139-163, composed),
 // the layers past it stay zero (project.go:81-83).
 __global__ void k_join_fp64(const __grid_constant__ Geom g, const __grid_constant__ Split S, double* p_, Status* st,
                             int gate) {
+    pdl_wait();
     if (gated(st, gate)) return;
     const int x = blockIdx.x * blockDim.x + threadIdx.x - g.G;
     const int y = blockIdx.y * blockDim.y + threadIdx.y - g.G;
@@ -548,6 +662,7 @@ __global__ void __launch_bounds__(256) k_gradient_fp64(const __grid_constant__ G
                                                        const double* __restrict__ p, double* u_, double* v_, double* w_,
                                                        const __grid_constant__ exact::MulC scale, Status* st,
                                                        int gate) {
+    pdl_wait();
     if (gated(st, gate)) return;
     const unsigned e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= (unsigned)(g.NX + 1) * (unsigned)(g.NY + 1)) return;
@@ -559,7 +674,10 @@ __global__ void __launch_bounds__(256) k_gradient_fp64(const __grid_constant__ G
               g.G + (int)blockIdx.y);
 }
 
-__global__ void k_step_tick(Status* st) { st->step += 1; }
+__global__ void k_step_tick(Status* st) {
+    pdl_wait();
+    st->step += 1;
+}
 
 // ---------------------------------------------------------------------------
 // Diagnostics.  A max is exact in any order; NaN is skipped as the
@@ -867,7 +985,7 @@ void launch_velocity_bc(const Geom& g, double* u, double* v, double* w, Status* 
         mx = std::max(mx, 2ll * (n[0] + 1) * (n[1] + 2));
     }
     dim3 grid(cdiv(mx, 256), 9);
-    k_velocity_bc<<<grid, 256, 0, s>>>(g, u, v, w, st, gate);
+    launch_pdl(k_velocity_bc, grid, dim3(256), 0, s, g, u, v, w, st, gate);
 }
 
 void launch_sweep_fp64(const Geom& g, int axis, const Fields& f, double dt, double invH, double lam, Status* st,
@@ -884,9 +1002,7 @@ void launch_sweep_fp64(const Geom& g, int axis, const Fields& f, double dt, doub
     a.set_scheme(axis, dt, invH, lam);
     a.st = st; a.phase = phase;
     const dim3 block(32, 8), grid = face_grid(g, block);
-    if (axis == 0) k_sweep_fp64<0><<<grid, block, 0, s>>>(a);
-    else if (axis == 1) k_sweep_fp64<1><<<grid, block, 0, s>>>(a);
-    else k_sweep_fp64<2><<<grid, block, 0, s>>>(a);
+    launch_pdl(axis == 0 ? k_sweep_fp64<0> : (axis == 1 ? k_sweep_fp64<1> : k_sweep_fp64<2>), grid, block, 0, s, a);
 }
 
 void launch_maccormack_fp64(const Geom& g, int axis, const Fields& f, const Fields& fwd, double dt, double invH,
@@ -905,16 +1021,15 @@ void launch_maccormack_fp64(const Geom& g, int axis, const Fields& f, const Fiel
     a.set_scheme(axis, dt, invH, lam);
     a.st = st; a.phase = phase;
     const dim3 block(32, 8), grid = face_grid(g, block);
-    if (axis == 0) k_maccormack_fp64<0><<<grid, block, 0, s>>>(a, fwd.t0, fwd.t1, fwd.t2);
-    else if (axis == 1) k_maccormack_fp64<1><<<grid, block, 0, s>>>(a, fwd.t0, fwd.t1, fwd.t2);
-    else k_maccormack_fp64<2><<<grid, block, 0, s>>>(a, fwd.t0, fwd.t1, fwd.t2);
+    launch_pdl(axis == 0 ? k_maccormack_fp64<0> : (axis == 1 ? k_maccormack_fp64<1> : k_maccormack_fp64<2>), grid, block,
+               0, s, a, fwd.t0, fwd.t1, fwd.t2);
 }
 
 void launch_divergence_fp64(const Geom& g, const Fields& f, const Split* split, double scale, double h2, Status* st,
                             int gate, cudaStream_t s) {
     const dim3 block(32, 8), grid(cdiv(g.NX, 32), cdiv(g.NY, 8), g.NZ);
-    k_divergence_fp64<<<grid, block, 0, s>>>(g, f.u, f.v, f.w, f.div, split ? *split : Split{}, split ? 1 : 0,
-                                             exact::mul_const(scale), exact::mul_const(h2), st, gate);
+    launch_pdl(k_divergence_fp64, grid, block, 0, s, g, f.u, f.v, f.w, f.div, split ? *split : Split{}, split ? 1 : 0,
+               exact::mul_const(scale), exact::mul_const(h2), st, gate);
 }
 
 void launch_split_from_div(const Geom& g, const double* div, const Split& split, double h2, cudaStream_t s) {
@@ -949,9 +1064,52 @@ void launch_rbgs_fp64(const Split& split, int color, cudaStream_t s) {
     launch_pdl(k, grid, dim3(128), 0, s, split, color);
 }
 
+// The cluster kernel for this grid, its cells a thread in *nc; null where the
+// grid is too large for it or the device cannot hold such a cluster.
+typedef void (*RbClusterKernel)(const Split, long long);
+static RbClusterKernel rbgs_cluster_kernel(const Split& S, size_t* smem) {
+    if ((long long)S.NX * S.NY * S.NZ > kRbMaxCells) return nullptr;
+    const int rows = (S.NY * S.NZ + kRbCluster - 1) / kRbCluster, n = rows * S.hx;
+    *smem = (size_t)2 * n * sizeof(double);
+    const RbClusterKernel k = n <= kRbThreads ? k_rbgs_cluster<1> : (n <= 2 * kRbThreads ? k_rbgs_cluster<2> : nullptr);
+    if (!k) return nullptr;
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return k;
+}
+
+bool launch_rbgs_all_fp64(const Split& split, long long pairs, cudaStream_t s) {
+    size_t smem = 0;
+    const RbClusterKernel k = rbgs_cluster_kernel(split, &smem);
+    if (!k) return false;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(kRbCluster);
+    cfg.blockDim = dim3(kRbThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[2] = {};
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = kRbCluster;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) != cudaSuccess || clusters < 1) {
+        cudaGetLastError();
+        return false;
+    }
+    cudaLaunchKernelEx(&cfg, k, split, pairs);
+    return true;
+}
+
 void launch_join_fp64(const Geom& g, const Split& split, double* p, Status* st, int gate, cudaStream_t s) {
     const dim3 block(64, 4), grid(cdiv(g.p.nx, 64), cdiv(g.p.ny, 4), g.p.nz);
-    k_join_fp64<<<grid, block, 0, s>>>(g, split, p, st, gate);
+    launch_pdl(k_join_fp64, grid, block, 0, s, g, split, p, st, gate);
 }
 
 void launch_pressure_bc_fp64(const Geom& g, double* p, Status* st, int gate, cudaStream_t s) {
@@ -962,11 +1120,11 @@ void launch_pressure_bc_fp64(const Geom& g, double* p, Status* st, int gate, cud
 
 void launch_gradient_fp64(const Geom& g, const Fields& f, double scale, Status* st, int gate, cudaStream_t s) {
     const dim3 grid(cdiv((long long)(g.NX + 1) * (g.NY + 1), 256), g.NZ + 1);
-    k_gradient_fp64<<<grid, 256, 0, s>>>(g, FastDiv((unsigned)(g.NX + 1)), f.p, f.u, f.v, f.w,
-                                         exact::mul_const(scale), st, gate);
+    launch_pdl(k_gradient_fp64, grid, dim3(256), 0, s, g, FastDiv((unsigned)(g.NX + 1)), f.p, f.u, f.v, f.w,
+               exact::mul_const(scale), st, gate);
 }
 
-void launch_step_tick(Status* st, cudaStream_t s) { k_step_tick<<<1, 1, 0, s>>>(st); }
+void launch_step_tick(Status* st, cudaStream_t s) { launch_pdl(k_step_tick, dim3(1), dim3(1), 0, s, st); }
 
 void launch_max_divergence(const Geom& g, const double* u, const double* v, const double* w, unsigned long long* out,
                            cudaStream_t s) {

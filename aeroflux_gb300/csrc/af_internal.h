@@ -153,6 +153,9 @@ void launch_divergence_fp64(const Geom& g, const Fields& f, const Split* split, 
 void launch_split_from_div(const Geom& g, const double* div, const Split& split, double h2, cudaStream_t s);
 // One colour sweep over the split arrays (scratch only: not gated).
 void launch_rbgs_fp64(const Split& split, int color, cudaStream_t s);
+// Every sweep of a solve (`pairs` red-black pairs) from zero P in one launch,
+// for grids small enough for it; false, nothing launched, for the others.
+bool launch_rbgs_all_fp64(const Split& split, long long pairs, cudaStream_t s);
 // The split P back into P, with applyPressureBC's ghosts; cells no one
 // writes (ghost layers past the first) are zero.
 void launch_join_fp64(const Geom& g, const Split& split, double* p, Status* st, int gate, cudaStream_t s);
