@@ -65,6 +65,7 @@ struct Lvl {
         int w, q, rows;
         FastDiv fq, fcol, fty;
     } march[3];
+    int v4;  // every axis coarsens, rows of whole quads, e, r and the next level's on 16-byte boundaries
 };
 
 struct Ctl {
@@ -856,7 +857,17 @@ __global__ void kb_correct(const InstDev* inst, Ctl* ctl, Tab tab) {
                        (g.G + (long long)(g.G + y) * g.p.sy + (long long)(g.G + z) * g.p.sz);
     AF_PTR(const float) e = view((const float*)I.lev[0].e, lvl_cells(I.lev[0]), DK_CORRECT, s) +
                             ((long long)g.NX * y + (long long)g.NX * g.NY * z);
-    for (int x = lane; x < g.NX; x += 32) p[x] += f32_to_f64(e[x]);
+    // Four cells a lane at a time, loads before stores.
+    for (int x0 = lane; x0 < g.NX; x0 += 128) {
+        double v[4];
+        float d[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (x0 + 32 * k < g.NX) v[k] = p[x0 + 32 * k], d[k] = e[x0 + 32 * k];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (x0 + 32 * k < g.NX) p[x0 + 32 * k] = v[k] + f32_to_f64(d[k]);
+    }
     END_ELEMS
     END_TILES
 }
@@ -1012,71 +1023,98 @@ __device__ __forceinline__ float mg_residual(const Lvl& L, int x, int y, int z, 
     return mg_res(L, sx, sy, sz, c, lr[i]);
 }
 
-// Coarse rhs = mean of the children's residuals; coarse solution = 0.  One
-// thread per coarse cell (row-wise forms of this kernel measured slower).
-// 32 registers a thread (without spilling) let a whole SM's threads be
-// resident: the finest restriction at 256^3 measured 43.5 -> 37.4 us against
-// the compiler's 56 registers.  (The prolongation spills at 32 and measured
-// slower at 32 and 40.)
-__global__ void __launch_bounds__(1024, 2) kb_restrict(const InstDev* inst, const Ctl* ctl, Tab tab, int l, int vc) {
+// Four cells of a level's row from an even one on.  V4: rows and arrays start
+// on 16-byte boundaries (Lvl::v4), one access; otherwise two of 8 bytes, the
+// second of them (cells 2 and 3) only where `two` (nx is even, so each pair is
+// whole).
+template <bool V4, class P>
+__device__ __forceinline__ float4 ld_quad(P p, long long i, bool two) {
+    if (V4) return AF_VEC(const float4, p, i, 4);
+    const float2 a = AF_VEC(const float2, p, i, 2), b = AF_VEC(const float2, p, i + (two ? 2 : 0), 2);
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+
+// Means of the residuals of two coarse cells' children, from the 2 x 2 rows of
+// four fine cells at b (e) and rb (r); a neighbour across a wall is the cell
+// itself.  The children in the order z, y, x with x fastest.
+template <bool V4, class P>
+__device__ __forceinline__ float2 restrict_two(const Lvl& F, P b, P rb, int x0, int y0, int z0, bool two, float inv) {
+    const long long sy = F.nx, sz = (long long)F.nx * F.ny;
+    const int xm = x0 > 0 ? -1 : 0, xp = x0 + 4 < F.nx ? 4 : (two ? 3 : 1);
+    const long long ym = y0 > 0 ? -sy : 0, yp = y0 + 2 < F.ny ? 2 * sy : sy;
+    const long long zm = z0 > 0 ? -sz : 0, zp = z0 + 2 < F.nz ? 2 * sz : sz;
+    float4 E[2][2];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) E[k >> 1][k & 1] = ld_quad<V4>(b, (k & 1) * sy + (k >> 1) * sz, two);
+    float s0 = 0.0f, s1 = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int dy = k & 1, dz = k >> 1;
+        const long long o = dy * sy + dz * sz;
+        const float4 c = E[dz][dy], R = ld_quad<V4>(rb, o, two);
+        const float4 my = E[dz][dy ^ 1], ny = ld_quad<V4>(b, dz * sz + (dy ? yp : ym), two);
+        const float4 mz = E[dz ^ 1][dy], nz = ld_quad<V4>(b, dy * sy + (dz ? zp : zm), two);
+        const float l = b[o + xm], r = b[o + xp];
+        s0 += mg_res(F, l + c.y, ny.x + my.x, nz.x + mz.x, c.x, R.x);
+        s0 += mg_res(F, c.x + (two ? c.z : r), ny.y + my.y, nz.y + mz.y, c.y, R.y);
+        s1 += mg_res(F, c.y + c.w, ny.z + my.z, nz.z + mz.z, c.z, R.z);
+        s1 += mg_res(F, c.z + r, ny.w + my.w, nz.w + mz.w, c.w, R.w);
+    }
+    return make_float2(s0 * inv, s1 * inv);
+}
+
+// Coarse rhs = mean of the children's residuals; coarse solution = 0.  Where
+// every axis coarsens a thread takes two coarse cells along x, whose children
+// are rows of four cells: 16 wide loads and 8 narrow ones where a cell a
+// thread made 80 narrow ones.  Bound by memory: e and r are read once from it
+// (8 bytes a fine cell).  Measured at 256^3 / 512^3, a cell a thread / two:
+// 38.8 / 34.7 and 239 / 214 us.  Otherwise a thread a coarse cell.
+__host__ __device__ inline bool restrict_pairs(const Lvl& F) { return F.cx && F.cy && F.cz; }
+__host__ __device__ inline long long restrict_items(const Lvl& F, const Lvl& C) {
+    return restrict_pairs(F) ? (long long)((C.nx + 1) / 2) * C.ny * C.nz : lvl_cells(C);
+}
+
+__global__ void __launch_bounds__(1024, 1) kb_restrict(const InstDev* inst, const Ctl* ctl, Tab tab, int l, int vc) {
     begin_level(inst, tab, l, 2);
     if (vc_idle(ctl, tab.n, vc)) return;
     FOR_TILES(tab)
     if (mg_off(ctl[s], vc)) continue;
-    const Lvl F = inst[s].lev[l];
-    const Lvl C = inst[s].lev[l + 1];
-    const long long n = lvl_cells(C);
+    const Lvl& F = inst[s].lev[l];
+    const Lvl& C = inst[s].lev[l + 1];
+    const long long n = restrict_items(F, C);
     const int ex = F.cx ? 2 : 1, ey = F.cy ? 2 : 1, ez = F.cz ? 2 : 1;
     const float inv = 1.0f / (float)(ex * ey * ez);
-    const bool full = ex == 2 && ey == 2 && ez == 2;
-    const long long nxy = (long long)F.nx * F.ny;
+    AF_PTR(float) cr = view(C.r, lvl_cells(C), DK_RESTRICT, s);
+    AF_PTR(float) ce = view(C.e, lvl_cells(C), DK_RESTRICT, s);
     FOR_ELEMS(tab)
     if (el >= n) break;
-    const unsigned e = (unsigned)el, r = C.fnx.div(e), zz = C.fny.div(r);
+    const unsigned e = (unsigned)el;
+    if (restrict_pairs(F)) {
+        const unsigned row = C.fhx.div(e), zz = C.fny.div(row);
+        const int X = 2 * (int)(e - row * C.fhx.d), Y = (int)(row - zz * (unsigned)C.ny), Z = (int)zz;
+        const bool two = X + 1 < C.nx;
+        const long long o = lidx(2 * X, 2 * Y, 2 * Z, F.nx, F.ny), i = lidx(X, Y, Z, C.nx, C.ny);
+        AF_PTR(const float) b = view((const float*)F.e, lvl_cells(F), DK_RESTRICT, s) + o;
+        AF_PTR(const float) rb = view((const float*)F.r, lvl_cells(F), DK_RESTRICT, s) + o;
+        if (F.v4) {
+            AF_VEC(float2, cr, i, 2) = restrict_two<true>(F, b, rb, 2 * X, 2 * Y, 2 * Z, true, inv);
+            AF_VEC(float2, ce, i, 2) = make_float2(0.0f, 0.0f);
+        } else {
+            const float2 m = restrict_two<false>(F, b, rb, 2 * X, 2 * Y, 2 * Z, two, inv);
+            cr[i] = m.x;
+            ce[i] = 0.0f;
+            if (two) cr[i + 1] = m.y, ce[i + 1] = 0.0f;
+        }
+        continue;
+    }
+    const unsigned r = C.fnx.div(e), zz = C.fny.div(r);
     const int X = (int)(e - r * (unsigned)C.nx), Y = (int)(r - zz * (unsigned)C.ny), Z = (int)zz;
     float sum = 0.0f;
-    if (full) {
-        // The 2x2x2 children and their 24 face neighbours, each loaded once
-        // (a neighbour across a wall is the child itself); then the eight
-        // residuals of mg_residual in the same order.
-        const int x0 = 2 * X, y0 = 2 * Y, z0 = 2 * Z;
-        AF_PTR(const float) b = view((const float*)F.e, lvl_cells(F), DK_RESTRICT, s) + lidx(x0, y0, z0, F.nx, F.ny);
-        AF_PTR(const float) rb = view((const float*)F.r, lvl_cells(F), DK_RESTRICT, s) + lidx(x0, y0, z0, F.nx, F.ny);
-        const long long sy = F.nx, sz = nxy;
-        float E[2][2][2], R[2][2][2];
-#pragma unroll
-        for (int dz = 0; dz < 2; ++dz)
-#pragma unroll
-            for (int dy = 0; dy < 2; ++dy)
-#pragma unroll
-                for (int dx = 0; dx < 2; ++dx) {
-                    E[dz][dy][dx] = b[dx + dy * sy + dz * sz];
-                    R[dz][dy][dx] = rb[dx + dy * sy + dz * sz];
-                }
-        const bool xl = x0 > 0, xh = x0 + 2 < F.nx, yl = y0 > 0, yh = y0 + 2 < F.ny, zl = z0 > 0, zh = z0 + 2 < F.nz;
-#pragma unroll
-        for (int dz = 0; dz < 2; ++dz)
-#pragma unroll
-            for (int dy = 0; dy < 2; ++dy)
-#pragma unroll
-                for (int dx = 0; dx < 2; ++dx) {
-                    const long long o = dx + dy * sy + dz * sz;
-                    const float c = E[dz][dy][dx];
-                    const float xm = dx ? E[dz][dy][0] : (xl ? b[o - 1] : c);
-                    const float xp = dx ? (xh ? b[o + 1] : c) : E[dz][dy][1];
-                    const float ym = dy ? E[dz][0][dx] : (yl ? b[o - sy] : c);
-                    const float yp = dy ? (yh ? b[o + sy] : c) : E[dz][1][dx];
-                    const float zm = dz ? E[0][dy][dx] : (zl ? b[o - sz] : c);
-                    const float zp = dz ? (zh ? b[o + sz] : c) : E[1][dy][dx];
-                    sum += mg_res(F, xm + xp, ym + yp, zm + zp, c, R[dz][dy][dx]);
-                }
-    } else {
-        for (int dz = 0; dz < ez; ++dz)
-            for (int dy = 0; dy < ey; ++dy)
-                for (int dx = 0; dx < ex; ++dx) sum += mg_residual(F, X * ex + dx, Y * ey + dy, Z * ez + dz, s);
-    }
-    view(C.r, lvl_cells(C), DK_RESTRICT, s)[el] = sum * inv;
-    view(C.e, lvl_cells(C), DK_RESTRICT, s)[el] = 0.0f;
+    for (int dz = 0; dz < ez; ++dz)
+        for (int dy = 0; dy < ey; ++dy)
+            for (int dx = 0; dx < ex; ++dx) sum += mg_residual(F, X * ex + dx, Y * ey + dy, Z * ez + dz, s);
+    cr[el] = sum * inv;
+    ce[el] = 0.0f;
     END_ELEMS
     END_TILES
 }
@@ -1088,15 +1126,20 @@ __global__ void __launch_bounds__(1024, 2) kb_restrict(const InstDev* inst, cons
 // (at most 16 lane iterations) share a warp two or four to a warp, so the
 // per-row setup is not paid by idle lanes.  The iteration space counts 32
 // lanes per warp (prolong_box).
+// Where every axis coarsens, a work row is a coarse row (Y0, Z0) and covers
+// the four fine rows (2 Y0 + {0, 1}, 2 Z0 + {0, 1}); a lane takes two coarse
+// cells of it, four cells of each fine row: 27 coarse loads (9 of them wide
+// where rows allow it, Lvl::v4) and 4 wide accesses of e each way for 16 fine
+// cells, all of a step's loads issued before its stores.  Bound by memory: e
+// is read and written once (8 bytes a fine cell).  Measured at 256^3 / 512^3,
+// one coarse cell a lane / two: 34.7 / 26.5 and 352 / 211 us.  Otherwise a work
+// row is a fine row.
+__host__ __device__ inline bool prolong_blocks(const Lvl& F) { return F.cx && F.cy && F.cz; }
 __host__ __device__ inline int prolong_lanes_log(const Lvl& F, const Lvl& C) {
-    const int w = F.cx ? C.nx : F.nx;  // lane iterations of a row
+    // Lane iterations of a row.
+    const int w = prolong_blocks(F) ? (C.nx + 1) / 2 : (F.cx ? C.nx : F.nx);
     return w > 16 ? 5 : (w > 8 ? 4 : 3);
 }
-// Where every axis coarsens, a work row is a coarse row (Y0, Z0) and covers
-// the four fine rows (2 Y0 + {0, 1}, 2 Z0 + {0, 1}), which share the coarse
-// rows Y0 - 1 .. Y0 + 1 x Z0 - 1 .. Z0 + 1: 27 coarse loads per 8 fine
-// cells instead of 48.  Otherwise a work row is a fine row.
-__host__ __device__ inline bool prolong_blocks(const Lvl& F) { return F.cx && F.cy && F.cz; }
 __host__ __device__ inline long long prolong_rows(const Lvl& F, const Lvl& C) {
     return prolong_blocks(F) ? (long long)C.ny * C.nz : (long long)F.ny * F.nz;
 }
@@ -1105,7 +1148,70 @@ __host__ __device__ inline long long prolong_box(const Lvl& F, const Lvl& C) {
     return 32ll * ((prolong_rows(F, C) + (1 << sh) - 1) >> sh);
 }
 
-__global__ void kb_prolong(const InstDev* inst, const Ctl* ctl, Tab tab, int l, int vc) {
+// Fine rows (2 Y0 + b, 2 Z0 + c), b, c in {0, 1}.  Row b takes neighbour row
+// Y0 + 1 if b else Y0 - 1, and likewise c (clamped at the walls, as the fine
+// cells' neighbours are); operands and order are mg_interp's.
+template <bool V4>
+__device__ __forceinline__ void prolong_rows4(const Lvl& F, const Lvl& C, int Y0, int Z0, int lane, int lanes, int s) {
+    AF_PTR(const float) AF_RESTRICT ce = view((const float*)C.e, lvl_cells(C), DK_PROLONG, s);
+    AF_PTR(float) AF_RESTRICT fe = view(F.e, lvl_cells(F), DK_PROLONG, s);
+    const int Ys[3] = {max(Y0 - 1, 0), Y0, min(Y0 + 1, C.ny - 1)};
+    const int Zm = max(Z0 - 1, 0), Zp = min(Z0 + 1, C.nz - 1);
+    const long long f0 = lidx(0, 2 * Y0, 2 * Z0, F.nx, F.ny), sy = F.nx, sz = (long long)F.nx * F.ny;
+    auto lerp = [](float p, float q) { return __fmaf_rn(0.25f, q, __fmul_rn(0.75f, p)); };
+    for (int X = 2 * lane; X < C.nx; X += 2 * lanes) {
+        const bool two = X + 1 < C.nx;
+        const int Xm = max(X - 1, 0), Xp = min(X + 2, C.nx - 1);
+        // Coarse plane Z interpolated along x and y: v[b][x].
+        auto plane = [&](int Z, float(&v)[2][4]) {
+            float lx[3][4];
+#pragma unroll
+            for (int b = 0; b < 3; ++b) {
+                const long long o = lidx(0, Ys[b], Z, C.nx, C.ny);
+                float c0, c1;
+                if (V4) {
+                    const float2 c = AF_VEC(const float2, ce, o + X, 2);
+                    c0 = c.x, c1 = c.y;
+                } else {
+                    c0 = ce[o + X], c1 = ce[o + X + (two ? 1 : 0)];
+                }
+                lx[b][0] = lerp(c0, ce[o + Xm]);
+                lx[b][1] = lerp(c0, c1);
+                lx[b][2] = lerp(c1, c0);
+                lx[b][3] = lerp(c1, ce[o + Xp]);
+            }
+#pragma unroll
+            for (int x = 0; x < 4; ++x) v[0][x] = lerp(lx[1][x], lx[0][x]), v[1][x] = lerp(lx[1][x], lx[2][x]);
+        };
+        float here[2][4];
+        plane(Z0, here);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const long long o = f0 + c * sz + 2 * X;
+            float4 f[2];
+            f[0] = ld_quad<V4>((AF_PTR(const float))fe, o, two);
+            f[1] = ld_quad<V4>((AF_PTR(const float))fe, o + sy, two);
+            float next[2][4];
+            plane(c ? Zp : Zm, next);
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                float4 g = f[b];
+                g.x = __fadd_rn(g.x, lerp(here[b][0], next[b][0]));
+                g.y = __fadd_rn(g.y, lerp(here[b][1], next[b][1]));
+                g.z = __fadd_rn(g.z, lerp(here[b][2], next[b][2]));
+                g.w = __fadd_rn(g.w, lerp(here[b][3], next[b][3]));
+                if (V4) {
+                    AF_VEC(float4, fe, o + b * sy, 4) = g;
+                } else {
+                    AF_VEC(float2, fe, o + b * sy, 2) = make_float2(g.x, g.y);
+                    if (two) AF_VEC(float2, fe, o + b * sy + 2, 2) = make_float2(g.z, g.w);
+                }
+            }
+        }
+    }
+}
+
+__global__ void __launch_bounds__(1024) kb_prolong(const InstDev* inst, const Ctl* ctl, Tab tab, int l, int vc) {
     begin_level(inst, tab, l, 2);
     if (vc_idle(ctl, tab.n, vc)) return;
     FOR_TILES(tab)
@@ -1119,49 +1225,10 @@ __global__ void kb_prolong(const InstDev* inst, const Ctl* ctl, Tab tab, int l, 
     if (row >= rows) break;
     const int lane = (int)(el & (lanes - 1));
     if (prolong_blocks(F)) {
-        // Coarse rows Ym, Y0, Yp x Zm, Z0, Zp (clamped at the walls, as the
-        // fine rows' neighbours are); fine row (2 Y0 + b, 2 Z0 + c) takes
-        // neighbour row Yp if b else Ym, and plane Zp if c else Zm.
         const unsigned cz = C.fny.div((unsigned)row);
         const int Y0 = (int)((unsigned)row - cz * (unsigned)C.ny), Z0 = (int)cz;
-        const int Ys[3] = {max(Y0 - 1, 0), Y0, min(Y0 + 1, C.ny - 1)};
-        const int Zs[3] = {max(Z0 - 1, 0), Z0, min(Z0 + 1, C.nz - 1)};
-        AF_PTR(const float) ce = view((const float*)C.e, lvl_cells(C), DK_PROLONG, s);
-        AF_PTR(float) fe = view(F.e, lvl_cells(F), DK_PROLONG, s);
-        int co[3][3];  // coarse row offsets [z][y]
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-#pragma unroll
-            for (int b = 0; b < 3; ++b) co[a][b] = (int)lidx(0, Ys[b], Zs[a], C.nx, C.ny);
-        int fo[2][2];  // fine row offsets [c][b]
-#pragma unroll
-        for (int c = 0; c < 2; ++c)
-#pragma unroll
-            for (int b = 0; b < 2; ++b) fo[c][b] = (int)lidx(0, 2 * Y0 + b, 2 * Z0 + c, F.nx, F.ny);
-        for (int X = lane; X < C.nx; X += lanes) {
-            const int Xm = max(X - 1, 0), Xp = min(X + 1, C.nx - 1);
-            float a0[3][3], am[3][3], ap[3][3];
-#pragma unroll
-            for (int a = 0; a < 3; ++a)
-#pragma unroll
-                for (int b = 0; b < 3; ++b) {
-                    a0[a][b] = ce[co[a][b] + X];
-                    am[a][b] = ce[co[a][b] + Xm];
-                    ap[a][b] = ce[co[a][b] + Xp];
-                }
-#pragma unroll
-            for (int c = 0; c < 2; ++c)
-#pragma unroll
-                for (int b = 0; b < 2; ++b) {
-                    const int y1 = b ? 2 : 0, z1 = c ? 2 : 0;  // the neighbour row and plane
-                    float2 f = AF_VEC(float2, fe, fo[c][b] + 2 * X, 2);
-                    f.x = __fadd_rn(f.x, mg_interp(0.75f, 0.75f, 0.75f, a0[1][1], am[1][1], a0[1][y1], am[1][y1],
-                                                   a0[z1][1], am[z1][1], a0[z1][y1], am[z1][y1]));
-                    f.y = __fadd_rn(f.y, mg_interp(0.75f, 0.75f, 0.75f, a0[1][1], ap[1][1], a0[1][y1], ap[1][y1],
-                                                   a0[z1][1], ap[z1][1], a0[z1][y1], ap[z1][y1]));
-                    AF_VEC(float2, fe, fo[c][b] + 2 * X, 2) = f;
-                }
-        }
+        if (F.v4) prolong_rows4<true>(F, C, Y0, Z0, lane, lanes, s);
+        else prolong_rows4<false>(F, C, Y0, Z0, lane, lanes, s);
         continue;
     }
     const unsigned zz = F.fny.div((unsigned)row);
@@ -2142,7 +2209,7 @@ long long stage_items(const Batch* b, const SlotHost& S, int st, const Shape& sh
         n = (l < lim && !I.lev[l].e2) ? row_box(I.lev[l]) : 0;
     } else if (st >= S_RESTRICT && st < S_PROLONG) {
         const int l = st - S_RESTRICT;
-        n = l < lim ? lvl_cells(I.lev[l + 1]) : 0;
+        n = l < lim ? restrict_items(I.lev[l], I.lev[l + 1]) : 0;
     } else if (st >= S_PROLONG && st < S_BIGCOARSE) {
         const int l = st - S_PROLONG;
         n = l < lim ? prolong_box(I.lev[l], I.lev[l + 1]) : 0;
@@ -2994,6 +3061,11 @@ int batch_assign(Batch* b, const af_config& c, char* arena, std::string* err) {
         }
     }
     cudaMemsetAsync(p, 0, mg, b->stream);
+    for (int l = 0; l + 1 < I.nlev; ++l) {
+        Lvl &F = I.lev[l], &C = I.lev[l + 1];
+        auto aligned = [](const float* q) { return ((uintptr_t)q & 15) == 0; };
+        F.v4 = restrict_pairs(F) && F.nx % 4 == 0 && aligned(F.e) && aligned(F.r) && aligned(C.e) && aligned(C.r);
+    }
     plan_march(I);
     plan_tail_table(I, &b->h_tails[kMaxLev * (size_t)s]);
     const double half = c.dt * 0.5;  // aeroflux.go:353
