@@ -477,11 +477,20 @@ __global__ void kb_sweep(const InstDev* inst, Status* st, Tab tab, int parity, i
 // instead.  Every face's arithmetic is the row kernel's (mx_face_vel4,
 // mx_backtrace, mx_face_value): the same bits.
 // Six planes deep: a thread computes six faces per tile, so the tile's
-// set-up (decode, slot search, geometry, transfer wait, barriers) is spread
-// over more faces than with four planes, while four blocks still fit an SM
-// (measured per sweep launch at 256^3: 4 planes 268-281 us, 6 planes
-// 236-250 us, 8 planes at three blocks per SM 290-311 us).
+// set-up (transfer wait, barrier, indices) is spread over more faces than
+// with four planes, while four blocks still fit an SM (measured per sweep
+// launch at 256^3, with the tile decoded by every thread: 4 planes 268-281 us,
+// 6 planes 236-250 us, 8 planes at three blocks per SM 290-311 us).
+//
+// Bound by issue (two thirds of the slots; 3.8 TB/s from memory), so the work
+// is in what a face costs: a backtrace of less than a cell interpolates
+// between values the diffusion has loaded anyway, values shared along z stay
+// in registers, the result is widened on the integer pipe, and a warp of its
+// own decodes tiles.  113 -> 68 instructions a face, 256^3 235-243 ->
+// 156-162 us a sweep (207-218 without the loading warp; 158-168 with the z
+// loop not unrolled).
 constexpr int kSwTX = 32, kSwTY = 8, kSwTZ = 6, kSwHA = 2, kSwThreads = kSwTX * kSwTY;
+constexpr int kSwBlock = kSwThreads + 32;  // and the loading warp
 // Box roles: 0-2 the own component for a sweep along x, y, z; 3 the axis
 // component.  First x of a box (a multiple of 4) and its width.
 __host__ __device__ constexpr int sw_box_x(int role, int x0) {
@@ -573,110 +582,163 @@ __device__ __forceinline__ void tma_load_3d(float* dst, const CUtensorMap* map, 
         : "memory");
 }
 
+// A tile of the staged sweep as the loading thread hands it to its block: the slot, the
+// component and the first face, and what a face needs of the slot, so that
+// the block's other threads neither decode the tile nor read the slot's
+// record.
+struct SwTile {
+    int live;  // 0 past the work list, without faces, or when the slot is gated by a fault
+    int s, c, x0, y0, z0;
+    int xhi, yhi, zend;   // one past the tile's last face (the component's last row: yhi)
+    int na, cmax;         // padded extent along the sweep axis; last coordinate a short backtrace is unclamped at
+    int dsy, dsz;         // strides of the component's binary64 field
+    int py, pz, dnz;      // row pitch and plane of its shadow, its planes
+    float dt_invh, lam;
+    double* dd;           // the binary64 field written
+    long long count;
+    const float* sh;      // the shadow
+    Status* st;
+};
+
 // Faces of one tile of component C (the loads have landed in own / axv).
 template <int AX, int C>
-__device__ __forceinline__ void sweep_tile_faces(const InstDev& I, Status* st, const float* own_, const float* axv_,
-                                                 double* __restrict__ dd_, int x0, int y0, int z0, int phase,
-                                                 int slot) {
-    const Geom& g = I.g;
-    const Dims& d = C == 0 ? g.u : (C == 1 ? g.v : g.w);
+__device__ __forceinline__ void sweep_tile_faces(const SwTile& T, const float* own_, const float* axv_, int phase) {
+    const int slot = T.s;
     AF_PTR(const float) own = view(own_, (long long)kSwOwnMax, DK_SWEEP_TMA, slot);
     AF_PTR(const float) axv = view(axv_, (long long)kSwAxCount, DK_SWEEP_TMA, slot);
-    AF_PTR(double) AF_RESTRICT dd = view(dd_, d.count, DK_SWEEP_TMA, slot);
+    AF_PTR(double) AF_RESTRICT dd = view(T.dd, T.count, DK_SWEEP_TMA, slot);
     constexpr int BX = sw_bx(AX), BY = sw_by(AX), BZ = sw_bz(AX);
     constexpr int SO = AX == 0 ? 1 : (AX == 1 ? BX : BX * BY);  // own-box stride along the sweep axis
     constexpr int AXX = sw_bx(3), AXY = sw_by(3);
     // Axis-box strides along the component's axis and the sweep axis.
     constexpr int EC = C == 0 ? 1 : (C == 1 ? AXX : AXX * AXY);
     constexpr int EA = AX == 0 ? 1 : (AX == 1 ? AXX : AXX * AXY);
+    const int x0 = T.x0, y0 = T.y0, z0 = T.z0;
     const int ox = sw_box_x(AX, x0), oy = y0 - (AX == 1 ? kSwHA : 0), oz = z0 - (AX == 2 ? kSwHA : 0);
     const int oa = AX == 0 ? ox : (AX == 1 ? oy : oz);  // own box's first coordinate along the axis
     const int ax0 = sw_box_x(3, x0);
     const int lx = threadIdx.x & 31, ly = threadIdx.x >> 5;
     const int y = y0 + ly;
-    const int G = g.G;
-    if (y >= G + g.NY + (C == 1)) return;
-    // The last tile of a row runs to the component's last face.
-    const int xhi = x0 + kSwTX >= G + g.NX ? G + g.NX + (C == 0) : x0 + kSwTX;
-    const int zend = min(z0 + kSwTZ, G + g.NZ + (C == 2));
-    const int na = AX == 0 ? d.nx : (AX == 1 ? d.ny : d.nz);
-    const long long py = I.shp[C], pz = py * d.ny;
-    const long long gs = AX == 0 ? 1 : (AX == 1 ? py : pz);
-    const float dt_invh = I.dt_invh, lam = I.lam;
-    const long long dsy = d.sy, dsz = d.sz;
-    const float* shc = I.sh[C];
+    if (y >= T.yhi) return;
+    const int xhi = T.xhi, zend = T.zend, cmax = T.cmax, dsz = T.dsz;
+    const float dt_invh = T.dt_invh, lam = T.lam;
+    // A backtrace of less than a cell whose taps lie inside the field, which
+    // mx_backtrace leaves unclamped: off > -1 and ca >= 1 give a position
+    // above 0, off < 1 and ca <= na - 3 one below na - 1 (SwTile::cmax).
     for (int x = x0 + lx; x < xhi; x += kSwTX) {
         // Walk z with every index advanced by its plane stride: the face's
-        // own box, the axis box and the binary64 destination.
+        // own box, the axis box and the binary64 destination.  What the next
+        // plane's face reads again stays in registers: along z the face's own
+        // values, and two of the four velocity taps where the component's or
+        // the sweep's axis is z.
         int io = ((z0 - oz) * BY + (y - oy)) * BX + (x - ox);
         int ia = (AXY + (y - y0 + 1)) * AXX + (x - ax0);
-        AF_PTR(double) dz = dd + ((long long)x + (long long)y * dsy + (long long)z0 * dsz);
+        AF_PTR(double) dz = dd + (x + y * T.dsy + z0 * dsz);  // a field holds < 2^31 elements
+        const bool in_xy = AX == 2 || (AX == 0 ? x : y) <= cmax;
+        float m = 0.0f, c = 0.0f, v0 = 0.0f, v1 = 0.0f;
+        if (AX == 2) m = own[io - SO], c = own[io];
+        if (C != AX && AX == 2) v0 = axv[ia - EC], v1 = axv[ia];
+        if (C != AX && C == 2) v0 = axv[ia - EC], v1 = axv[ia + EA - EC];
+#pragma unroll 2
         for (int z = z0; z < zend; ++z, io += BX * BY, ia += AXX * AXY, dz += dsz) {
+            if (AX != 2) m = own[io - SO], c = own[io];
+            const float p = own[io + SO];
             float vel;
+            // The row kernel's tap order: before the sweep axis's own
+            // component, (-e_C, 0, e_AX - e_C, e_AX); after it,
+            // (-e_C, e_AX - e_C, 0, e_AX).
             if (C == AX) {
-                vel = own[io];
+                vel = c;
+            } else if (AX == 2 || C == 2) {
+                const float w0 = AX == 2 ? axv[ia + EA - EC] : axv[ia], w1 = axv[ia + EA];
+                vel = mx_face_vel4(v0, v1, w0, w1);
+                v0 = w0, v1 = w1;
+            } else if (AX > C) {
+                vel = mx_face_vel4(axv[ia - EC], axv[ia], axv[ia + EA - EC], axv[ia + EA]);
             } else {
-                // The row kernel's tap order: before the sweep axis's own
-                // component, (-e_C, 0, e_AX - e_C, e_AX); after it,
-                // (-e_C, e_AX - e_C, 0, e_AX).
-                if (AX > C) vel = mx_face_vel4(axv[ia - EC], axv[ia], axv[ia + EA - EC], axv[ia + EA]);
-                else vel = mx_face_vel4(axv[ia - EC], axv[ia + EA - EC], axv[ia], axv[ia + EA]);
+                vel = mx_face_vel4(axv[ia - EC], axv[ia + EA - EC], axv[ia], axv[ia + EA]);
             }
             const int ca = AX == 0 ? x : (AX == 1 ? y : z);
-            int i0;
-            float t;
-            if (!mx_backtrace(vel, ca, na, dt_invh, &i0, &t)) {
-                atomicMin(&st->fault_gate, st->step * 8u + (unsigned)phase);
-                atomicMin(&st->fault_key, fault_key(C, x, y, z));
-                continue;
-            }
-            float d0, d1;
-            const int rel = i0 - ca;
-            if (i0 >= oa && i0 + 1 < oa + (AX == 0 ? BX : (AX == 1 ? BY : BZ))) {
-                d0 = own[io + rel * SO];
-                d1 = own[io + (rel + 1) * SO];
+            const float off = -__fmul_rn(vel, dt_invh);
+            float t, d0, d1;
+            if (fabsf(off) < 1.0f && (AX == 2 ? z <= cmax : in_xy)) {
+                const bool back = off < 0.0f;
+                t = __fadd_rn(off, back ? 1.0f : 0.0f);  // off - floor(off), and +0 of -0
+                d0 = back ? m : c;
+                d1 = back ? c : p;
             } else {
-                AF_PTR(const float) gp =
-                    view(shc, pz * d.nz, DK_SWEEP_TMA, slot) + (x + y * py + z * pz + rel * gs);
-                d0 = gp[0];
-                d1 = gp[gs];
+                int i0;
+                if (!mx_backtrace(vel, ca, T.na, dt_invh, &i0, &t)) {
+                    atomicMin(&T.st->fault_gate, T.st->step * 8u + (unsigned)phase);
+                    atomicMin(&T.st->fault_key, fault_key(C, x, y, z));
+                    if (AX == 2) m = c, c = p;
+                    continue;
+                }
+                const int rel = i0 - ca;
+                if (i0 >= oa && i0 + 1 < oa + (AX == 0 ? BX : (AX == 1 ? BY : BZ))) {
+                    d0 = own[io + rel * SO];
+                    d1 = own[io + (rel + 1) * SO];
+                } else {
+                    AF_PTR(const float) gp =
+                        view(T.sh, (long long)T.pz * T.dnz, DK_SWEEP_TMA, slot) + (x + y * T.py + (long long)z * T.pz);
+                    const int gs = AX == 0 ? 1 : (AX == 1 ? T.py : T.pz);
+                    d0 = gp[(long long)rel * gs];
+                    d1 = gp[(long long)(rel + 1) * gs];
+                }
             }
-            const float res = mx_face_value(t, d0, d1, own[io - SO], own[io], own[io + SO], lam);
-            dz[0] = (double)res;  // widening is exact
+            dz[0] = widen(mx_face_value(t, d0, d1, m, c, p, lam));
+            if (AX == 2) m = c, c = p;
         }
     }
 }
 
-// A decoded tile of the staged sweep: slot, component and first face; dead
-// when past the work list or its slot is gated by a fault.
-struct SwTile {
-    int s, c, x0, y0, z0;
-    bool live;
-};
-
-__device__ __forceinline__ SwTile sw_decode(const InstDev* inst, const Status* st, const Tab& tab, int item, int total,
-                                            int phase) {
-    SwTile t{0, 0, 0, 0, 0, false};
-    if (item >= total) return t;
-    t.s = find_slot(tab.prefix, tab.n, item);
-    const InstDev& I = inst[t.s];
-    if (gated(&st[t.s], phase)) return t;
+// Called by a whole warp (find_slot); its first lane writes the tile.
+template <int AX>
+__device__ __forceinline__ void sw_decode(const InstDev* inst, Status* st, const Tab& tab, int item, int total,
+                                          int parity, int phase, SwTile* t) {
+    const int s = item < total ? find_slot(tab.prefix, tab.n, item) : -1;
+    if ((threadIdx.x & 31) != 0) return;
+    t->live = 0;
+    if (s < 0) return;
+    const InstDev& I = inst[s];
+    if (gated(&st[s], phase)) return;
     // The three components of one spatial tile are consecutive items, so
     // the axis component's box, staged again for the other two, is still in
     // L2.  A spatial tile past one component's last face row or plane holds
     // no faces of it.
-    const unsigned local = (unsigned)(item - tab.prefix[t.s]);
+    const Geom& g = I.g;
+    const unsigned local = (unsigned)(item - tab.prefix[s]);
     const unsigned r = local / 3u;
-    t.c = (int)(local - 3u * r);
+    const int c = (int)(local - 3u * r);
     const unsigned q1 = I.swx.div(r), q2 = I.swy.div(q1);
-    t.x0 = I.g.G + (int)(r - q1 * I.swx.d) * kSwTX;
-    t.y0 = I.g.G + (int)(q1 - q2 * I.swy.d) * kSwTY;
-    t.z0 = I.g.G + (int)q2 * kSwTZ;
-    t.live = t.y0 < I.g.G + I.g.NY + (t.c == 1) && t.z0 < I.g.G + I.g.NZ + (t.c == 2);
-    return t;
+    t->s = s;
+    t->c = c;
+    t->x0 = g.G + (int)(r - q1 * I.swx.d) * kSwTX;
+    t->y0 = g.G + (int)(q1 - q2 * I.swy.d) * kSwTY;
+    t->z0 = g.G + (int)q2 * kSwTZ;
+    t->yhi = g.G + g.NY + (c == 1);
+    t->zend = min(t->z0 + kSwTZ, g.G + g.NZ + (c == 2));
+    if (t->y0 >= t->yhi || t->z0 >= t->zend) return;
+    // The last tile of a row runs to the component's last face.
+    t->xhi = t->x0 + kSwTX >= g.G + g.NX ? g.G + g.NX + (c == 0) : t->x0 + kSwTX;
+    const Dims& d = c == 0 ? g.u : (c == 1 ? g.v : g.w);
+    t->na = AX == 0 ? d.nx : (AX == 1 ? d.ny : d.nz);
+    t->cmax = g.G >= 1 ? t->na - 3 : -1;
+    t->dsy = (int)d.sy;
+    t->dsz = (int)d.sz;
+    t->py = I.shp[c];
+    t->pz = I.shp[c] * d.ny;
+    t->dnz = d.nz;
+    t->dt_invh = I.dt_invh;
+    t->lam = I.lam;
+    t->dd = cur(I, 5 + c, parity);
+    t->count = d.count;
+    t->sh = I.sh[c];
+    t->st = st + s;
+    t->live = 1;
 }
 
-// Thread 0: the TMA loads of tile t into one buffer pair.  The buffers' last
+// The loading thread: the TMA loads of tile t into one buffer pair.  The buffers' last
 // reads (generic proxy) finished before the caller's barrier; the fence
 // orders them before these writes (async proxy).
 template <int AX>
@@ -690,10 +752,11 @@ __device__ __forceinline__ void sw_issue(const InstDev& I, const SwTile& t, floa
     if (t.c != AX) tma_load_3d(axv, I.tmap + AX * 4 + 3, sw_box_x(3, t.x0), t.y0 - 1, t.z0 - 1, bar);
 }
 
-// Persistent blocks walk their tiles with two buffer pairs: the loads of the
-// next tile are in flight while the current tile's faces are computed.
+// Persistent blocks walk their tiles with two buffer pairs: a warp of its own
+// decodes the next tile and issues its loads while the others compute the
+// current one's faces.
 template <int AX>
-__global__ void __launch_bounds__(kSwThreads, 4)
+__global__ void __launch_bounds__(kSwBlock, 4)
     kb_sweep_tma(const InstDev* inst, Status* st, Tab tab, int parity, int phase, unsigned* diag) {
     begin_slot(inst, tab);
     extern __shared__ __align__(128) float swsm[];
@@ -717,36 +780,45 @@ __global__ void __launch_bounds__(kSwThreads, 4)
     const int total = tab.prefix[tab.n];
     unsigned ph = 0u;  // bit k: the phase parity buffer k waits for next
     int item = blockIdx.x, k = 0;
-    SwTile tile = sw_decode(inst, st, tab, item, total, phase);
-    if (tile.live && threadIdx.x == 0) sw_issue<AX>(inst[tile.s], tile, own(0), axv(0), &bar[0]);
+    __shared__ __align__(8) SwTile tile[2];  // of buffer pair k
+    // The loading warp, all its lanes; the first one does the work.
+    const bool loading = threadIdx.x >= kSwThreads, loader = threadIdx.x == kSwThreads;
+    auto begin_tile = [&](int it, int kk) {
+        sw_decode<AX>(inst, st, tab, it, total, parity, phase, &tile[kk]);
+        if (loader && tile[kk].live) sw_issue<AX>(inst[tile[kk].s], tile[kk], own(kk), axv(kk), &bar[kk]);
+    };
+    if (loading) begin_tile(item, 0);
+    __syncthreads();
     while (item < total) {
         const int next_item = item + gridDim.x;
-        const SwTile next = sw_decode(inst, st, tab, next_item, total, phase);
-        if (next.live && threadIdx.x == 0) sw_issue<AX>(inst[next.s], next, own(k ^ 1), axv(k ^ 1), &bar[k ^ 1]);
-        if (tile.live) {
-            const bool ok = __syncthreads_and(mbar_wait_bounded(&bar[k], (ph >> k) & 1u) ? 1 : 0) != 0;
-            ph ^= 1u << k;
+        const SwTile& T = tile[k];
+        bool ok = true;
+        if (loading) {
+            begin_tile(next_item, k ^ 1);
+        } else if (T.live) {
+            ok = mbar_wait_bounded(&bar[k], (ph >> k) & 1u);
             if (!ok) {
-                // A transfer did not land in time: record it, give the copies
-                // in flight a second bounded wait, and stop.
-                if (threadIdx.x == 0) {
-                    atomicOr(diag, 1u);
-                    mbar_wait_bounded(&bar[k], ((ph >> k) & 1u) ^ 1u);
-                    if (next.live) mbar_wait_bounded(&bar[k ^ 1], (ph >> (k ^ 1)) & 1u);
-                }
-                __syncthreads();
-                return;
+            } else if (T.c == 0) {
+                sweep_tile_faces<AX, 0>(T, own(k), axv(k), phase);
+            } else if (T.c == 1) {
+                sweep_tile_faces<AX, 1>(T, own(k), axv(k), phase);
+            } else {
+                sweep_tile_faces<AX, 2>(T, own(k), axv(k), phase);
             }
-            const InstDev& I = inst[tile.s];
-            double* dd = cur(I, 5 + tile.c, parity);
-            if (tile.c == 0)
-                sweep_tile_faces<AX, 0>(I, st + tile.s, own(k), axv(k), dd, tile.x0, tile.y0, tile.z0, phase, tile.s);
-            else if (tile.c == 1)
-                sweep_tile_faces<AX, 1>(I, st + tile.s, own(k), axv(k), dd, tile.x0, tile.y0, tile.z0, phase, tile.s);
-            else sweep_tile_faces<AX, 2>(I, st + tile.s, own(k), axv(k), dd, tile.x0, tile.y0, tile.z0, phase, tile.s);
         }
-        __syncthreads();  // every thread is done with buffer k before it is loaded again
-        tile = next;
+        if (T.live) ph ^= 1u << k;
+        // Every thread is done with buffer pair k before it is loaded again.
+        if (__syncthreads_or(ok ? 0 : 1)) {
+            // A transfer did not land in time: record it, give the copies in
+            // flight a second bounded wait, and stop.
+            if (loader) {
+                atomicOr(diag, 1u);
+                mbar_wait_bounded(&bar[k], ((ph >> k) & 1u) ^ 1u);
+                if (tile[k ^ 1].live) mbar_wait_bounded(&bar[k ^ 1], (ph >> (k ^ 1)) & 1u);
+            }
+            __syncthreads();
+            return;
+        }
         item = next_item;
         k ^= 1;
     }
@@ -2312,7 +2384,7 @@ void enq_sweep(Batch* b, int axis, int parity, int phase, cudaStream_t s) {
         const Tab t = tab(b, S_SWEEPT);
         const int g = grid(b, S_SWEEPT);
         const auto k = axis == 0 ? kb_sweep_tma<0> : (axis == 1 ? kb_sweep_tma<1> : kb_sweep_tma<2>);
-        launch_pdl(k, dim3(g), dim3(kSwThreads), kSwSmem, s, b->d_inst, b->d_st, t, parity, phase, b->d_diag);
+        launch_pdl(k, dim3(g), dim3(kSwBlock), kSwSmem, s, b->d_inst, b->d_st, t, parity, phase, b->d_diag);
         ++b->launches;
         return;
     }
@@ -2687,7 +2759,7 @@ Batch* batch_create(int capacity, size_t pool_bytes, std::string* err) {
     // The row sweep (gathers through L1) instead of the staged tile sweep: the same bits.
     if (const char* sr = getenv("AEROFLUX_SWEEP_ROWS")) b->tma_sweep = atoi(sr) == 0;
     if (b->tma_sweep && !tensor_map_encoder()) b->tma_sweep = false;
-    b->shape[S_SWEEPT] = Shape{kSwThreads, 1, 4};  // shared memory holds four blocks' buffers per SM
+    b->shape[S_SWEEPT] = Shape{kSwBlock, 1, 4};  // shared memory holds four blocks' buffers per SM
     cudaFuncSetAttribute(kb_sweep_tma<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSwSmem);
     cudaFuncSetAttribute(kb_sweep_tma<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSwSmem);
     cudaFuncSetAttribute(kb_sweep_tma<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSwSmem);

@@ -377,6 +377,21 @@ __device__ __forceinline__ double f32_to_f64(float f) {
     return __longlong_as_double((long long)(((unsigned long long)hi << 32) | lo));
 }
 
+// (double)f on the integer pipe: the conversion instruction runs on the
+// binary64 one, which a warp holds for as long as some 70 others take.
+// Subnormals, infinities and NaN, which are rare, take the instruction, in a
+// function of their own so that it is never predicated.
+static __device__ __noinline__ double widen_native(float f) { return (double)f; }
+__device__ __forceinline__ double widen(float f) {
+    const unsigned u = __float_as_uint(f), m = u & 0x7FFFFFFFu;
+    unsigned hi = (m >> 3) + (896u << 20);
+    if (m - 0x800000u >= 0x7F000000u) {  // not a normal number
+        if (m) return widen_native(f);
+        hi = 0u;
+    }
+    return __longlong_as_double((long long)(((unsigned long long)(hi | (u & 0x80000000u)) << 32) | (u << 29)));
+}
+
 // --- binary32 advection + diffusion of one face (stencil.go:44-225) --------
 // The sweep interpolates along its axis only (the other two weights are 0).
 // Every rounding is explicit, so the result does not depend on how the

@@ -3,9 +3,11 @@
 Grids whose sizes sit on or next to a limit of a kernel's split: rows of an
 odd number of cell pairs and rows longer than a warp's lanes in the
 restriction and prolongation, tile columns and z chunks of the marching pair,
+backtraces of exactly one cell and results next to zero in the staged sweep,
 and the largest grids whose red-black solve runs in one cluster launch.  The
 comparison is on bit patterns, so there is no tolerance.
 """
+import numpy as np
 import pytest
 
 from aeroflux_gb300 import Config
@@ -41,3 +43,25 @@ def test_red_black_solve_at_cluster_edges(n, ghost):
     gpu.project()
     orc.project()
     assert_bit_identical(gpu, orc, ["P", "U", "V", "W", "Div"], f"{n} projection")
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("nu", [0.0, 1e-4])
+def test_sweep_at_backtrace_edges(axis, nu):
+    # Velocities whose backtrace is 0 of either sign, exactly one cell, or its
+    # neighbouring floats (dt / h = 0.5), among values whose interpolation is
+    # subnormal; n is odd against the sweep's 32 x 8 x 6 tile.
+    n = (37, 11, 13)
+    e, o = make_mixed_pair(n, apply_bc=False, H=0.0625, Viscosity=nu)
+    two = np.float32(2.0)
+    values = np.array([0.0, -0.0, 2.0, -2.0, np.nextafter(two, np.float32(0)), -np.nextafter(two, np.float32(3)),
+                       np.nextafter(two, np.float32(3)), 1.2e-38, -1.2e-38, 1e-40, 0.75, -1.5], np.float64)
+    rng = np.random.default_rng(11 + axis)
+    for i, name in enumerate(("U", "V", "W"), start=1):
+        a = rng.choice(values, o.data(i).size)
+        e.upload(name, a)
+        o.data(i)[:] = a
+    e.sweep(axis, 0.03125)
+    o.sweep(axis, 0.03125)
+    assert_same(e.download, o, ("U", "V", "W", "Tmp0", "Tmp1", "Tmp2"), f"axis {axis}")
+    e.Close()
