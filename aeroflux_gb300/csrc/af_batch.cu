@@ -101,6 +101,7 @@ struct InstDev {
     int coarse_sweeps;  // sweeps of the coarsest solve inside the tail V-cycle
     int tail;           // first level of the one-block tail V-cycle; -1: coarsest too large, smoothed instead
     int tail_floats;    // shared-memory floats of the tail levels (e and r)
+    int res_lg;         // log2 of the planes a thread of the residual takes
     int parity;         // 1 when U/V/W live in the Tmp slots
     int active;
     FastDiv fpx, fpy;        // padded P extents
@@ -225,6 +226,9 @@ __host__ __device__ inline long long face_box(const Geom& g) {
 }
 __host__ __device__ inline long long pbc_count(const Geom& g) {
     return 2ll * g.NY * g.NZ + 2ll * (g.NX + 2) * g.NZ + 2ll * (g.NX + 2) * (g.NY + 2);
+}
+__host__ __device__ inline long long residual_items(const Geom& g, int lg) {
+    return (long long)g.NX * g.NY * ((g.NZ + (1 << lg) - 1) >> lg);
 }
 __host__ __device__ inline long long lvl_cells(const Lvl& L) { return (long long)L.nx * L.ny * L.nz; }
 
@@ -861,9 +865,12 @@ __device__ __forceinline__ void warp_max_commit(unsigned long long m, unsigned l
 // running maximum over consecutive tiles of one slot and commits it (one
 // atomic per warp) when the slot changes or the block finishes, so the
 // atomics are per block, not per warp-sized tile.  In the loop a converged
-// slot is skipped.  Of the seven binary64 operations the x and y neighbour
-// sums run on the integer pipe (the last difference cancels too deeply for
-// it); 256^3: 268 us with none there, 209 so.
+// slot is skipped.  Bound by the binary64 pipe: of the seven operations the x
+// and y neighbour sums run on the integer pipe (the last difference cancels
+// too deeply for it; a third sum there costs more issue than it saves).  A
+// thread takes 2^res_lg cells of a column, so that their indices are worked
+// out once and a cell's z neighbours stay in registers (residual_planes_log).
+// 256^3: 268 us with no integer sums, 222 a cell a thread, 184 with eight.
 __global__ void kb_residual(const InstDev* inst, Status* st, Ctl* ctl, Tab tab, int gate, int in_loop) {
     begin_slot(inst, tab);
     int held = -1;
@@ -884,28 +891,37 @@ __global__ void kb_residual(const InstDev* inst, Status* st, Ctl* ctl, Tab tab, 
         AF_PTR(const double) AF_RESTRICT bb = view((const double*)I.b, g.p.count, DK_RESIDUAL, s);
         AF_PTR(float) AF_RESTRICT r0 = view(I.lev[0].r, nl0, DK_RESIDUAL, s);
         AF_PTR(float) AF_RESTRICT e0 = view(I.lev[0].e, nl0, DK_RESIDUAL, s);
-        const long long n = (long long)g.NX * g.NY * g.NZ;
+        const int planes = 1 << I.res_lg;
+        const long long n = residual_items(g, I.res_lg);
         for (int k = 0; k < tab.ept; ++k) {
             const long long el = first + (long long)k * blockDim.x + threadIdx.x;
             if (el >= n) continue;
             const unsigned e = (unsigned)el, r2 = I.fnx.div(e), zz = I.fny.div(r2);
-            const int xi = (int)(e - r2 * (unsigned)g.NX), yi = (int)(r2 - zz * (unsigned)g.NY), zi = (int)zz;
+            const int xi = (int)(e - r2 * (unsigned)g.NX), yi = (int)(r2 - zz * (unsigned)g.NY), z0 = (int)zz << I.res_lg;
             const int sy = (int)g.p.sy, sz = (int)g.p.sz;  // a field holds < 2^31 elements
-            const int i = (g.G + xi) + (g.G + yi) * sy + (g.G + zi) * sz;
+            int i = (g.G + xi) + (g.G + yi) * sy + (g.G + z0) * sz;
+            int j = xi + g.NX * (yi + g.NY * z0);
             // A neighbour across a wall is the cell itself.
-            const double pc = p[i];
-            const double xm = p[xi > 0 ? i - 1 : i], xp = p[xi < g.NX - 1 ? i + 1 : i];
-            const double ym = p[yi > 0 ? i - sy : i], yp = p[yi < g.NY - 1 ? i + sy : i];
-            const double zm = p[zi > 0 ? i - sz : i], zp = p[zi < g.NZ - 1 ? i + sz : i];
-            const double sum = dadd(dadd(dadd_int(xm, xp), dadd_int(ym, yp)), dadd(zm, zp));
-            const double res = dsub(bb[i], __fma_rn(-6.0, pc, sum));
-            r0[el] = f64_to_f32(res);
-            e0[el] = 0.0f;
-            // |res| and NaN on the bit pattern (integer pipe); NaN reads as
-            // +Inf so the loop stops.
-            const unsigned long long a = dbits(res) & ~kSign;
-            const unsigned long long v = a > 0x7FF0000000000000ull ? 0x7FF0000000000000ull : a;
-            m = v > m ? v : m;
+            const int xm = xi > 0 ? -1 : 0, xp = xi < g.NX - 1 ? 1 : 0;
+            const int ym = yi > 0 ? -sy : 0, yp = yi < g.NY - 1 ? sy : 0;
+            double below = p[z0 > 0 ? i - sz : i], pc = p[i];
+            const int zend = min(z0 + planes, g.NZ);
+#pragma unroll 1
+            for (int z = z0; z < zend; ++z, i += sz, j += g.NX * g.NY) {
+                const double above = p[z < g.NZ - 1 ? i + sz : i];
+                const double sum = dadd(dadd(dadd_int(p[i + xm], p[i + xp]), dadd_int(p[i + ym], p[i + yp])),
+                                        dadd(below, above));
+                const double res = dsub(bb[i], __fma_rn(-6.0, pc, sum));
+                r0[j] = f64_to_f32(res);
+                e0[j] = 0.0f;
+                below = pc;
+                pc = above;
+                // |res| and NaN on the bit pattern (integer pipe); NaN reads as
+                // +Inf so the loop stops.
+                const unsigned long long a = dbits(res) & ~kSign;
+                const unsigned long long v = a > 0x7FF0000000000000ull ? 0x7FF0000000000000ull : a;
+                m = v > m ? v : m;
+            }
         }
     }
     if (held >= 0) warp_max_commit(m, &ctl[held].maxr_bits);
@@ -2269,7 +2285,7 @@ long long stage_items(const Batch* b, const SlotHost& S, int st, const Shape& sh
     else if (st == S_SHADOW) n = I.shq[3];
     else if (st == S_SWEEPT) return I.sw_tiles;
     else if (st == S_DIV) n = (long long)I.g.p.nx * I.g.p.ny * I.g.p.nz;
-    else if (st == S_INT) n = (long long)I.g.NX * I.g.NY * I.g.NZ;
+    else if (st == S_INT) n = residual_items(I.g, I.res_lg);
     else if (st == S_CORR) n = 32ll * I.g.NY * I.g.NZ;
     else if (st == S_PBC) n = pbc_count(I.g);
     else if (st == S_COARSE) return I.tail >= 0 ? 1 : 0;
@@ -2323,8 +2339,21 @@ cudaError_t upload_stage(Batch* b, int st) {
     return cudaMemcpyAsync(b->d_tab + st * w, &b->h_tab[st * w], w * sizeof(int), cudaMemcpyHostToDevice, b->stream);
 }
 
+// Cells a thread of the residual takes: eight where that leaves every slot's
+// cells together at least 64 Ki threads, else two.  Measured at one, two, four,
+// eight: 48x32x64 10.2, 7.8, 14.7, 19.2 us; 96^3 20.8, 19.3, 19.8, 17.0; 128^3
+// 37.2, 34.3, 34.2, 33.2; 256^3 222, 219, -, 184.
+int residual_planes_log(const Batch* b) {
+    long long cells = 0;
+    for (const auto& s : b->slots)
+        if (s.used && s.active) cells += (long long)s.d.g.NX * s.d.g.NY * s.d.g.NZ;
+    return cells >= (512ll << 10) ? 3 : 1;
+}
+
 cudaError_t upload_tables(Batch* b) {
     const int w = b->cap + 1;
+    const int lg = residual_planes_log(b);
+    for (auto& s : b->slots) s.d.res_lg = lg;
     b->h_tab.assign((size_t)S_COUNT * w, 0);
     for (int st = 0; st < S_COUNT; ++st) fill_tab(b, st);
     std::vector<InstDev> inst(b->cap);
