@@ -227,6 +227,10 @@ __host__ __device__ inline long long face_box(const Geom& g) {
 __host__ __device__ inline long long pbc_count(const Geom& g) {
     return 2ll * g.NY * g.NZ + 2ll * (g.NX + 2) * g.NZ + 2ll * (g.NX + 2) * (g.NY + 2);
 }
+constexpr int kCorrZ = 4;  // cells of a column a thread of the correction takes
+__host__ __device__ inline long long correct_items(const Geom& g) {
+    return (long long)g.NX * g.NY * ((g.NZ + kCorrZ - 1) / kCorrZ);
+}
 __host__ __device__ inline long long residual_items(const Geom& g, int lg) {
     return (long long)g.NX * g.NY * ((g.NZ + (1 << lg) - 1) >> lg);
 }
@@ -927,35 +931,35 @@ __global__ void kb_residual(const InstDev* inst, Status* st, Ctl* ctl, Tab tab, 
     if (held >= 0) warp_max_commit(m, &ctl[held].maxr_bits);
 }
 
-// p += e over the interior, a warp per (y, z) row (32 lanes per row).
+// p += e over the interior.  Bound by memory (20 bytes a cell).  A thread takes
+// kCorrZ cells of a column, loads before stores, and neighbouring threads
+// neighbouring cells across the ends of rows: a warp per row left lanes idle
+// on rows that are no multiple of 32 and had one load in flight.  48x32x64 5.8 ->
+// 4.8 us, 256^3 60 -> 58, a 256-grid batch 512 -> 453; a warp per row with four
+// cells a lane: 54.7 at 256^3, 712 for the batch.
 __global__ void kb_correct(const InstDev* inst, Ctl* ctl, Tab tab) {
     begin_slot(inst, tab);
     FOR_TILES(tab)
     const InstDev& I = inst[s];
     if (ctl[s].stopped) continue;
     const Geom& g = I.g;
-    const long long rows = (long long)g.NY * g.NZ;
+    AF_PTR(double) AF_RESTRICT p = view(I.slot[0], g.p.count, DK_CORRECT, s);
+    AF_PTR(const float) AF_RESTRICT e0 = view((const float*)I.lev[0].e, lvl_cells(I.lev[0]), DK_CORRECT, s);
+    const long long n = correct_items(g);
     FOR_ELEMS(tab)
-    const long long row = el >> 5;
-    if (row >= rows) break;
-    const int lane = (int)(el & 31);
-    const unsigned zz = I.fny.div((unsigned)row);
-    const int y = (int)((unsigned)row - zz * (unsigned)g.NY), z = (int)zz;
-    AF_PTR(double) p = view(I.slot[0], g.p.count, DK_CORRECT, s) +
-                       (g.G + (long long)(g.G + y) * g.p.sy + (long long)(g.G + z) * g.p.sz);
-    AF_PTR(const float) e = view((const float*)I.lev[0].e, lvl_cells(I.lev[0]), DK_CORRECT, s) +
-                            ((long long)g.NX * y + (long long)g.NX * g.NY * z);
-    // Four cells a lane at a time, loads before stores.
-    for (int x0 = lane; x0 < g.NX; x0 += 128) {
-        double v[4];
-        float d[4];
+    if (el >= n) break;
+    const unsigned q = (unsigned)el, r2 = I.fnx.div(q), zz = I.fny.div(r2);
+    const int x = (int)(q - r2 * (unsigned)g.NX), y = (int)(r2 - zz * (unsigned)g.NY), z = (int)zz * kCorrZ;
+    const int sy = (int)g.p.sy, sz = (int)g.p.sz, se = g.NX * g.NY;
+    const int i = (g.G + x) + (g.G + y) * sy + (g.G + z) * sz, j = x + g.NX * y + se * z;
+    double v[kCorrZ];
+    float d[kCorrZ];
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if (x0 + 32 * k < g.NX) v[k] = p[x0 + 32 * k], d[k] = e[x0 + 32 * k];
+    for (int k = 0; k < kCorrZ; ++k)
+        if (z + k < g.NZ) v[k] = p[i + k * sz], d[k] = e0[j + k * se];
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if (x0 + 32 * k < g.NX) p[x0 + 32 * k] = v[k] + f32_to_f64(d[k]);
-    }
+    for (int k = 0; k < kCorrZ; ++k)
+        if (z + k < g.NZ) p[i + k * sz] = v[k] + f32_to_f64(d[k]);
     END_ELEMS
     END_TILES
 }
@@ -2286,7 +2290,7 @@ long long stage_items(const Batch* b, const SlotHost& S, int st, const Shape& sh
     else if (st == S_SWEEPT) return I.sw_tiles;
     else if (st == S_DIV) n = (long long)I.g.p.nx * I.g.p.ny * I.g.p.nz;
     else if (st == S_INT) n = residual_items(I.g, I.res_lg);
-    else if (st == S_CORR) n = 32ll * I.g.NY * I.g.NZ;
+    else if (st == S_CORR) n = correct_items(I.g);
     else if (st == S_PBC) n = pbc_count(I.g);
     else if (st == S_COARSE) return I.tail >= 0 ? 1 : 0;
     const int lim = I.tail >= 0 ? I.tail : I.nlev - 1;  // levels smoothed by per-level kernels
