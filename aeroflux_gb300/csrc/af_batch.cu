@@ -101,7 +101,7 @@ struct InstDev {
     int coarse_sweeps;  // sweeps of the coarsest solve inside the tail V-cycle
     int tail;           // first level of the one-block tail V-cycle; -1: coarsest too large, smoothed instead
     int tail_floats;    // shared-memory floats of the tail levels (e and r)
-    int res_lg;         // log2 of the planes a thread of the residual takes
+    int res_lg;         // log2 of the planes a thread of the residual takes (at most kResMaxLg)
     int parity;         // 1 when U/V/W live in the Tmp slots
     int active;
     FastDiv fpx, fpy;        // padded P extents
@@ -227,6 +227,7 @@ __host__ __device__ inline long long face_box(const Geom& g) {
 __host__ __device__ inline long long pbc_count(const Geom& g) {
     return 2ll * g.NY * g.NZ + 2ll * (g.NX + 2) * g.NZ + 2ll * (g.NX + 2) * (g.NY + 2);
 }
+constexpr int kResMaxLg = 3;
 constexpr int kCorrZ = 4;  // cells of a column a thread of the correction takes
 __host__ __device__ inline long long correct_items(const Geom& g) {
     return (long long)g.NX * g.NY * ((g.NZ + kCorrZ - 1) / kCorrZ);
@@ -874,7 +875,7 @@ __device__ __forceinline__ void warp_max_commit(unsigned long long m, unsigned l
 // too deeply for it; a third sum there costs more issue than it saves).  A
 // thread takes 2^res_lg cells of a column, so that their indices are worked
 // out once and a cell's z neighbours stay in registers (residual_planes_log).
-// 256^3: 268 us with no integer sums, 222 a cell a thread, 184 with eight.
+// 256^3: 268 us with no integer sums, 222 a cell a thread, 186 with eight.
 __global__ void kb_residual(const InstDev* inst, Status* st, Ctl* ctl, Tab tab, int gate, int in_loop) {
     begin_slot(inst, tab);
     int held = -1;
@@ -909,9 +910,12 @@ __global__ void kb_residual(const InstDev* inst, Status* st, Ctl* ctl, Tab tab, 
             const int xm = xi > 0 ? -1 : 0, xp = xi < g.NX - 1 ? 1 : 0;
             const int ym = yi > 0 ? -sy : 0, yp = yi < g.NY - 1 ? sy : 0;
             double below = p[z0 > 0 ? i - sz : i], pc = p[i];
-            const int zend = min(z0 + planes, g.NZ);
+            // A constant count with an early exit: 186 us where a computed one
+            // takes 200.
 #pragma unroll 1
-            for (int z = z0; z < zend; ++z, i += sz, j += g.NX * g.NY) {
+            for (int c = 0; c < 1 << kResMaxLg; ++c, i += sz, j += g.NX * g.NY) {
+                const int z = z0 + c;
+                if (z >= g.NZ || c >= planes) break;
                 const double above = p[z < g.NZ - 1 ? i + sz : i];
                 const double sum = dadd(dadd(dadd_int(p[i + xm], p[i + xp]), dadd_int(p[i + ym], p[i + yp])),
                                         dadd(below, above));
@@ -2351,7 +2355,7 @@ int residual_planes_log(const Batch* b) {
     long long cells = 0;
     for (const auto& s : b->slots)
         if (s.used && s.active) cells += (long long)s.d.g.NX * s.d.g.NY * s.d.g.NZ;
-    return cells >= (512ll << 10) ? 3 : 1;
+    return cells >= (512ll << 10) ? kResMaxLg : 1;
 }
 
 cudaError_t upload_tables(Batch* b) {
