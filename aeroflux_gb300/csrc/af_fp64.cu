@@ -534,6 +534,11 @@ __global__ void __launch_bounds__(128) k_rbgs_fp64(const __grid_constant__ Split
 // ---------------------------------------------------------------------------
 constexpr int kRbCluster = 16, kRbThreads = 512;
 constexpr int kRbMaxCells = 20480;
+// A block's two colours of at most 2 * kRbThreads slots fit the shared memory
+// a launch gets without asking for more.  The limit is not set per solve: it
+// belongs to the function, not to an engine, and a smaller engine on another
+// thread would lower it between a larger one's check and its launch.
+static_assert(2 * 2 * kRbThreads * sizeof(double) <= 48 * 1024, "no larger shared-memory limit is asked for");
 
 __device__ __forceinline__ unsigned cluster_rank() {
     unsigned r;
@@ -1073,8 +1078,7 @@ static RbClusterKernel rbgs_cluster_kernel(const Split& S, size_t* smem) {
     *smem = (size_t)2 * n * sizeof(double);
     const RbClusterKernel k = n <= kRbThreads ? k_rbgs_cluster<1> : (n <= 2 * kRbThreads ? k_rbgs_cluster<2> : nullptr);
     if (!k) return nullptr;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem) != cudaSuccess) {
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
         cudaGetLastError();
         return nullptr;
     }
