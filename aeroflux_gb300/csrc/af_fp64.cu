@@ -1107,7 +1107,10 @@ bool launch_rbgs_all_fp64(const Split& split, long long pairs, cudaStream_t s) {
         cudaGetLastError();
         return false;
     }
-    cudaLaunchKernelEx(&cfg, k, split, pairs);
+    if (cudaLaunchKernelEx(&cfg, k, split, pairs) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
     return true;
 }
 

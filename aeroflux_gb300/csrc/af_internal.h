@@ -154,7 +154,8 @@ void launch_split_from_div(const Geom& g, const double* div, const Split& split,
 // One colour sweep over the split arrays (scratch only: not gated).
 void launch_rbgs_fp64(const Split& split, int color, cudaStream_t s);
 // Every sweep of a solve (`pairs` red-black pairs) from zero P in one launch,
-// for grids small enough for it; false, nothing launched, for the others.
+// for grids small enough for it; false, nothing launched, for the others and
+// where the device refuses the launch.
 bool launch_rbgs_all_fp64(const Split& split, long long pairs, cudaStream_t s);
 // The split P back into P, with applyPressureBC's ghosts; cells no one
 // writes (ghost layers past the first) are zero.
