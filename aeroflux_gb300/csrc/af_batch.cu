@@ -2555,8 +2555,11 @@ void enq_project(Batch* b, int parity, int gate, cudaStream_t s) {
         // the first two passes stand before it (their kernels return at once
         // where every slot has converged), the second sets its condition.
         for (int k = 0; k < kStraightPasses; ++k) enq_pass(b, s, h, k + 1 == kStraightPasses, gate);
-        if ((rc = cudaStreamGetCaptureInfo(s, &cs, nullptr, &graph, &deps, nullptr, &ndeps)) != cudaSuccess) {
-            b->capture_err = rc;
+        // A launch of the passes that the device refused has ended the capture:
+        // the graph and its nodes are then no longer ours to use.
+        rc = cudaStreamGetCaptureInfo(s, &cs, nullptr, &graph, &deps, nullptr, &ndeps);
+        if (rc != cudaSuccess || cs != cudaStreamCaptureStatusActive) {
+            b->capture_err = rc != cudaSuccess ? rc : cudaErrorStreamCaptureInvalidated;
             return;
         }
         cudaGraphNodeParams params{cudaGraphNodeTypeConditional};  // the other members value-initialised
