@@ -2615,6 +2615,7 @@ void enq_step(Batch* b, cudaStream_t s) {
 template <class F>
 cudaError_t capture(Batch* b, F body, cudaGraphExec_t* out) {
     cudaGraph_t graph = nullptr;
+    b->capture_err = cudaSuccess;  // an ended capture has left its own
     cudaError_t rc = cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal);
     if (rc != cudaSuccess) return rc;
     body();
@@ -3247,6 +3248,7 @@ cudaError_t batch_step(Batch* b, int64_t nsteps, std::string* err, const std::ve
 
 cudaError_t batch_prepare_capture(Batch* b) {
     cudaError_t rc;
+    b->capture_err = cudaSuccess;
     default_pair_variants(b);
     if (b->tables_dirty && (rc = upload_tables(b)) != cudaSuccess) return rc;
     if (kernel_levels(b) > b->graph_levels && b->graph) {
