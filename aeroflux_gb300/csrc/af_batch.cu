@@ -1710,6 +1710,11 @@ __global__ void __launch_bounds__(kMarchT[K], kMarchBlocks[K])
 // tests and block barriers in every sweep / so: 16^3 (a tail alone, 14
 // V-cycles) 0.72 / 0.59 ms, 48x32x64 1.44 / 1.38 ms, 256^3 10.40 / 10.27 ms.
 constexpr int kWarpSlots = 128;
+// The most dynamic shared memory a tail takes (plan_tail): ghost cells on
+// every side make the thinnest hierarchy, 2 x 2 x 1024 cells, the largest.  The
+// limit belongs to the kernel, not to a batch, so every batch sets this one: a
+// batch that set its own would take it from another on another thread.
+constexpr int kTailSmem = 181344;
 
 // A level's layout in shared memory: strides along the axes (0 along an axis
 // of extent 1), offset of cell (0, 0, 0) and floats of e; r is unpadded.
@@ -2677,7 +2682,6 @@ cudaError_t prepare(Batch* b) {
         b->graph_single |= single;
         b->tail_smem = std::max(b->tail_smem, tsm);
         b->graph_nu = b->nu;
-        cudaFuncSetAttribute(kb_vtail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->tail_smem);
         b->launches = 0;
         size_grids(b);
         if ((rc = capture(b, [&] { enq_step(b, b->stream); }, &b->graph)) != cudaSuccess) {
@@ -2804,6 +2808,7 @@ Batch* batch_create(int capacity, size_t pool_bytes, std::string* err) {
     cudaFuncSetAttribute(kb_sweep_tma<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSwSmem);
     cudaFuncSetAttribute(kb_sweep_tma<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSwSmem);
     cudaFuncSetAttribute(kb_sweep_tma<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSwSmem);
+    cudaFuncSetAttribute(kb_vtail, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmem);
     // Shapes: the tiny per-slot control and coarse stages keep their own.
     b->shape[S_COARSE] = Shape{kCoarseThreads, 1, 2};
     for (int l = 0; l < kMaxLev; ++l) {
@@ -3262,9 +3267,6 @@ cudaError_t batch_prepare_capture(Batch* b) {
     b->graph_march |= march_levels(b);
     b->graph_single |= single_levels(b);
     b->tail_smem = std::max(b->tail_smem, tail_smem_bytes(b));
-    if ((rc = cudaFuncSetAttribute(kb_vtail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->tail_smem)) !=
-        cudaSuccess)
-        return rc;
     size_grids(b);
     return cudaSuccess;
 }

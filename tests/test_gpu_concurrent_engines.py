@@ -6,7 +6,7 @@ import threading
 import numpy as np
 import pytest
 
-from aeroflux_gb300 import Config, New
+from aeroflux_gb300 import AF_PRECISION_MIXED, Config, New
 from tests.helpers import same_bits
 
 pytestmark = pytest.mark.gpu
@@ -53,4 +53,33 @@ def test_red_black_solves_of_two_sizes_at_once(sizes):
     assert not _in_threads([lambda e=e: solves(e) for e in engines])
     for e, p in zip(engines, want):
         assert same_bits(e.download("P"), p).all()
+        e.Close()
+
+
+def test_mixed_projections_of_two_sizes_at_once():
+    # Each projection is captured anew; the two tails of the V-cycle take 64
+    # and 2 KiB of shared memory.
+    def engine(n):
+        e = New(Config(NX=n, NY=n, NZ=n, H=1.0 / n, DT=0.004, Viscosity=1e-4, Precision=AF_PRECISION_MIXED, DivTol=1e-10))
+        e.SeedDevice(1.0, 0.05, 42, 0)
+        e.applyVelocityBC()
+        return e
+
+    def project(e):
+        for _ in range(400):
+            e.project()
+
+    def fields(e):
+        return np.concatenate([e.download(name) for name in ("P", "U", "V", "W")])
+
+    want = []
+    for n in (16, 4):
+        e = engine(n)
+        project(e)
+        want.append(fields(e))
+        e.Close()
+    engines = [engine(n) for n in (16, 4)]
+    assert not _in_threads([lambda e=e: project(e) for e in engines])
+    for e, w in zip(engines, want):
+        assert same_bits(fields(e), w).all()
         e.Close()
