@@ -1513,10 +1513,10 @@ __global__ void __launch_bounds__(PairTile<LANES, V>::THREADS, PairTile<LANES, V
 // plane costs a quad 16-byte loads of e two planes ahead, of r one plane
 // ahead and of the two rows beside it, one scalar across the quad's end, and
 // one 16-byte store.  Red values of a plane are exchanged with the rows and
-// quads beside it through a two-plane ring in shared memory, so there is one
-// barrier a plane: while a block computes the red cells of plane z, it
-// computes the black ones of plane z - 1, whose neighbours' red cells the
-// last barrier published.
+// quads beside it through a ring of four planes in shared memory: in the
+// iteration that computes the red cells of plane z, a thread computes the black
+// ones of plane z - 1, whose neighbours' red cells the barrier of that plane
+// published.
 //
 // A tile is a column of at most kMarchQ quads by March::rows rows; its block
 // also computes the red cells of the row on either side, of the quad on
@@ -1554,16 +1554,33 @@ constexpr int kMarchShapeCount = sizeof kMarchShapes / sizeof kMarchShapes[0];
 __device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
-// Waits for the block's own warps only, all resident and none of them waiting
-// for anything else; bounded all the same.
-__device__ __forceinline__ void march_wait(unsigned long long* bar, unsigned parity) {
-    for (unsigned it = 0; it < kSwSpinLimit && !mbar_try_wait(bar, parity); ++it) {
+// Waits for the block's own warps only: all are resident, wait for nothing
+// else and arrive on every plane.  The wait is bounded all the same: `polls`
+// here, then, in a function of its own, 2^16 times as many and, as a transfer's
+// wait, kWaitLimitNs.  A wait that gives up records it, which makes the call an
+// error; the thread goes on, so that its warp still arrives for the others, and
+// the work's later waits end after their first polls.  (Looking at the record
+// at every launch's start instead is a load in its way: 48x32x64 1.51 -> 1.61
+// ms a Step.)
+constexpr unsigned kMarchPolls = 64;
+__device__ __noinline__ void march_wait_long(unsigned long long* bar, unsigned parity, unsigned polls, unsigned* diag) {
+    const unsigned long long t0 = global_ns();
+    for (unsigned it = 0; it < polls << 16; ++it) {
+        if (mbar_try_wait(bar, parity)) return;
+        if ((it & 63u) == 0u && (diag_set(diag) || global_ns() - t0 > kWaitLimitNs)) break;
     }
+    atomicOr(diag, 2u);
+}
+__device__ __forceinline__ void march_wait(unsigned long long* bar, unsigned parity, unsigned polls, unsigned* diag) {
+    for (unsigned it = 0; it < polls; ++it)
+        if (mbar_try_wait(bar, parity)) return;
+    march_wait_long(bar, parity, polls, diag);
 }
 
 template <int K>
 __global__ void __launch_bounds__(kMarchT[K], kMarchBlocks[K])
-    kb_smooth_march(const InstDev* inst, const Ctl* ctl, Tab tab, int l, int dir, int vc, int zc) {
+    kb_smooth_march(const InstDev* inst, const Ctl* ctl, Tab tab, int l, int dir, int vc, int zc, unsigned polls,
+                    unsigned* diag) {
     begin_level(inst, tab, l, 1);
     if (vc_idle(ctl, tab.n, vc)) return;
     constexpr int T = kMarchT[K];
@@ -1658,7 +1675,7 @@ __global__ void __launch_bounds__(kMarchT[K], kMarchBlocks[K])
             // was last read three planes ago.
             __syncwarp();
             if ((tid & 31) == 0) mbar_arrive(&bar[n & 1u]);
-            if (n > 0) march_wait(&bar[(n - 1u) & 1u], ((n - 1u) >> 1) & 1u);
+            if (n > 0) march_wait(&bar[(n - 1u) & 1u], ((n - 1u) >> 1) & 1u, polls, diag);
             if (active) {
                 if (z > z0) {
                     if (out) {
@@ -2208,7 +2225,8 @@ struct Batch {
     unsigned march = ~0u;              // levels whose fused pairs march where a slot's level allows it
     int force_pair_var = -1;           // AEROFLUX_PAIR_VARIANT: every fused pair stage's variant (-1: tuned)
     bool pair_chosen = false;          // the fused pairs' tile variants are set (tuned or by level size)
-    unsigned* d_diag = nullptr;        // nonzero: a kernel gave up waiting on a transfer
+    unsigned march_polls = kMarchPolls;  // AEROFLUX_MARCH_POLLS: march_wait's first polls (0: every wait gives up)
+    unsigned* d_diag = nullptr;        // nonzero: a kernel gave up a bounded wait; lies behind the statuses
 };
 
 namespace {
@@ -2476,7 +2494,8 @@ void launch_march(Batch* b, int l, int dir, int vc, cudaStream_t s) {
     const int st = S_MARCH + l, g = grid(b, st);
     const MarchShape m = kMarchShapes[b->shape[st].var];
     const auto k = m.k == 0 ? kb_smooth_march<0> : (m.k == 1 ? kb_smooth_march<1> : kb_smooth_march<2>);
-    launch_pdl(k, dim3(g), dim3(kMarchT[m.k]), 0, s, b->d_inst, b->d_ctl, tab(b, st), l, dir, vc, m.zc);
+    launch_pdl(k, dim3(g), dim3(kMarchT[m.k]), 0, s, b->d_inst, b->d_ctl, tab(b, st), l, dir, vc, m.zc, b->march_polls,
+               b->d_diag);
     ++b->launches;
 }
 
@@ -2821,19 +2840,21 @@ Batch* batch_create(int capacity, size_t pool_bytes, std::string* err) {
         (rc = cudaStreamCreateWithFlags(&b->body, cudaStreamNonBlocking)) != cudaSuccess ||
         (rc = cudaMalloc(&b->d_inst, sizeof(InstDev) * capacity)) != cudaSuccess ||
         (rc = cudaMalloc(&b->d_tails, sizeof(TailLvl) * kMaxLev * (size_t)capacity)) != cudaSuccess ||
-        (rc = cudaMalloc(&b->d_st, sizeof(Status) * capacity)) != cudaSuccess ||
+        (rc = cudaMalloc(&b->d_st, sizeof(Status) * (capacity + 1))) != cudaSuccess ||
         (rc = cudaMalloc(&b->d_ctl, sizeof(Ctl) * (capacity + 1))) != cudaSuccess ||
         (rc = cudaMalloc(&b->d_tab, sizeof(int) * (size_t)S_COUNT * (capacity + 1))) != cudaSuccess ||
-        (rc = cudaMalloc(&b->d_tmaps, sizeof(CUtensorMap) * 12 * (size_t)capacity)) != cudaSuccess ||
-        (rc = cudaMalloc(&b->d_diag, sizeof(unsigned))) != cudaSuccess) {
+        (rc = cudaMalloc(&b->d_tmaps, sizeof(CUtensorMap) * 12 * (size_t)capacity)) != cudaSuccess) {
         *err = std::string("aeroflux: batch tables: ") + cudaGetErrorString(rc);
         batch_destroy(b);
         return nullptr;
     }
+    b->d_diag = (unsigned*)(b->d_st + capacity);
     cudaMemsetAsync(b->d_ctl, 0, sizeof(Ctl) * (capacity + 1), b->stream);
     cudaMemsetAsync(b->d_diag, 0, sizeof(unsigned), b->stream);
     b->h_tmaps.assign(12 * (size_t)capacity, CUtensorMap{});
     b->h_tails.assign(kMaxLev * (size_t)capacity, TailLvl{});
+    // 0: every wait of the marching pair gives up (how that is reported).
+    if (const char* mp = getenv("AEROFLUX_MARCH_POLLS")) b->march_polls = (unsigned)std::min(4096, std::max(0, atoi(mp)));
     // The fused pairs' tile variant for every level (0-2 and 4; 3: marching
     // where a slot's level allows it), instead of the tuned or size-based choice.
     if (const char* pv = getenv("AEROFLUX_PAIR_VARIANT")) b->force_pair_var = std::min(4, std::max(0, atoi(pv)));
@@ -2868,7 +2889,6 @@ void batch_destroy(Batch* b) {
     cudaFree(b->d_ctl);
     cudaFree(b->d_tab);
     cudaFree(b->d_tmaps);
-    cudaFree(b->d_diag);
     if (b->body) cudaStreamDestroy(b->body);
     if (b->stream) cudaStreamDestroy(b->stream);
     delete b;
@@ -3421,6 +3441,8 @@ bool batch_device_error(Batch* b, std::string* msg) {
     cudaMemset(b->d_diag, 0, sizeof v);
     *msg = (v & 4u)   ? "aeroflux: cuda: a staged kernel's shared-memory buffers are not 128-byte aligned; the step's "
                         "results are invalid"
+           : (v & 2u) ? "aeroflux: cuda: a smoothing kernel gave up waiting for its block; the step's results are "
+                        "invalid"
                       : "aeroflux: cuda: a staged kernel gave up waiting for its tile transfer; the step's results "
                         "are invalid";
     return true;

@@ -73,7 +73,8 @@ cudaError_t batch_seed(Batch* b, int slot, double amp, double noise, uint64_t se
 int batch_collect_faults(Batch* b, std::string* msg, int* first_slot);
 bool batch_slot_faulted(const Batch* b, int slot, std::string* msg);
 // Whether a kernel of the enqueued work gave up a bounded wait (the work's
-// results are then invalid); clears the record and sets *msg.
+// results are then invalid); clears the record and sets *msg.  The record is a
+// word behind the last slot's status (batch_status).
 bool batch_device_error(Batch* b, std::string* msg);
 // Refinement passes, estimated max|div| and multigrid V-cycles of the slot's
 // last projection.

@@ -490,10 +490,16 @@ int batch_check(af_engine* e, cudaError_t rc, const std::string& what) {
 }
 
 int sync_and_check(af_engine* e) {
-    Status s;
-    AF_CUDA(e, cudaMemcpyAsync(&s, e->st, sizeof s, cudaMemcpyDeviceToHost, e->stream));
+    // The multigrid projection's diagnostic word lies behind its one status.
+    struct {
+        Status s;
+        unsigned diag;
+    } w{};
+    const Status& s = w.s;
+    AF_CUDA(e, cudaMemcpyAsync(&w, e->st, e->mg ? sizeof w : sizeof w.s, cudaMemcpyDeviceToHost, e->stream));
     AF_CUDA(e, cudaStreamSynchronize(e->stream));
     if (af::debug_bounds_error(&e->err)) return AF_ERR_CUDA;
+    if (w.diag && af::batch_device_error(e->mg, &e->err)) return AF_ERR_CUDA;
     if (s.fault_gate != af::kNoFault) {
         e->err = fault_message(e, s.fault_gate, s.fault_key);
         // The reference returns before commitVelocity of the faulting sweep:
