@@ -830,8 +830,7 @@ int af_max_divergence(af_engine* e, double* out) {
     unsigned long long bits = 0;
     AF_CUDA(e, cudaMemcpyAsync(&bits, e->mx, sizeof bits, cudaMemcpyDeviceToHost, e->stream));
     AF_CUDA(e, cudaStreamSynchronize(e->stream));
-    memcpy(out, &bits, sizeof bits);
-    *out = (1.0 / e->cfg.h) * *out;
+    *out = af::max_divergence_of(bits, e->cfg.h);
     return AF_OK;
 }
 
@@ -1245,8 +1244,7 @@ int af_batch_max_divergence(af_batch* h, int64_t slot, double* out) {
     unsigned long long bits = 0;
     cudaMemcpyAsync(&bits, h->mx, sizeof bits, cudaMemcpyDeviceToHost, s);
     if (int r = batch_wait(h)) return r;
-    memcpy(out, &bits, sizeof bits);
-    *out = (1.0 / h->cfg[slot].h) * *out;
+    *out = af::max_divergence_of(bits, h->cfg[slot].h);
     return AF_OK;
 }
 

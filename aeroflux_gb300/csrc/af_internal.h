@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
 #include <string>
 
@@ -172,6 +173,15 @@ void launch_max_divergence(const Geom& g, const double* u, const double* v, cons
                            cudaStream_t s);
 void launch_max_abs3(const double* u, long long nu, const double* v, long long nv, const double* w, long long nw,
                      unsigned long long* out, cudaStream_t s);
+// MaxDivergence from launch_max_divergence's word.  A product that is not a
+// number (1/h infinite and nothing to scale, or the reverse) counts for
+// nothing, as in the reference's comparison.
+inline double max_divergence_of(unsigned long long bits, double h) {
+    double m;
+    memcpy(&m, &bits, sizeof m);
+    const double d = (1.0 / h) * m;
+    return d == d ? d : 0.0;
+}
 int kinetic_energy_partials(const Geom& g);
 void launch_kinetic_energy(const Geom& g, const double* u, const double* v, const double* w, double* partials,
                            double* out, cudaStream_t s);

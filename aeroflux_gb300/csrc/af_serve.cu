@@ -90,9 +90,7 @@ double max_div_of(af_server* s, int slot, const af_config& c) {
     unsigned long long bits = 0;
     cudaMemcpyAsync(&bits, s->mx, sizeof bits, cudaMemcpyDeviceToHost, st);
     cudaStreamSynchronize(st);
-    double d;
-    memcpy(&d, &bits, sizeof d);
-    return (1.0 / c.h) * d;
+    return af::max_divergence_of(bits, c.h);
 }
 
 }  // namespace
