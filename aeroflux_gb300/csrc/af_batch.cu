@@ -169,9 +169,9 @@ __device__ __forceinline__ int find_slot(const int* prefix, int n, int item) {
 // kernel wrote.  What no kernel writes -- with one slot, its record (`bytes`
 // from `off`) and work list -- it fetches into its L1 before it waits (with
 // many slots the search for the block's own costs as much as it saves).
-// Measured per Step with the passes before the WHILE node: 16^3 789 -> 722
-// us, 48x32x64 1.62 -> 1.48 ms, 128^3 3.25 -> 3.18, the 256-grid batch
-// unchanged.
+// Measured per Step, launches one after the other / overlapped: 16^3 0.690 /
+// 0.678 ms, 48x32x64 1.56 / 1.50, 128^3 2.755 / 2.69, 256^3 9.19 / 9.12, the
+// 256-grid batch unchanged.
 __device__ __forceinline__ void touch(const void* p) {
     unsigned v;
     asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
@@ -2534,8 +2534,6 @@ void enq_vcycle(Batch* b, int vc, cudaStream_t s) {
     }
 }
 
-constexpr int kStraightPasses = 2;
-
 void enq_pass(Batch* b, cudaStream_t s, cudaGraphConditionalHandle h, int use_cond, int gate) {
     for (int k = 0; k < b->vcycles; ++k) enq_vcycle(b, k, s);
     LAUNCH(b, S_CORR, kb_correct, b->d_inst, b->d_ctl, tab(b, S_CORR));
@@ -2571,16 +2569,18 @@ void enq_project(Batch* b, int parity, int gate, cudaStream_t s) {
             b->capture_err = rc;
             return;
         }
-        launch_pdl(kb_check, dim3(1), dim3(256), 0, s, b->d_inst, b->d_st, b->d_ctl, b->cap, h, 0, 0, gate, b->vcycles,
+        launch_pdl(kb_check, dim3(1), dim3(256), 0, s, b->d_inst, b->d_st, b->d_ctl, b->cap, h, 1, 0, gate, b->vcycles,
                    b->pass_floor);
         ++b->launches;
-        // Nearly every projection needs two passes, and an iteration of the
-        // WHILE node costs 50-100 us more than the same launches outside it:
-        // the first two passes stand before it (their kernels return at once
-        // where every slot has converged), the second sets its condition.
-        for (int k = 0; k < kStraightPasses; ++k) enq_pass(b, s, h, k + 1 == kStraightPasses, gate);
-        // A launch of the passes that the device refused has ended the capture:
-        // the graph and its nodes are then no longer ours to use.
+        // Every pass is an iteration of the node, the first two too, which nearly
+        // every projection needs: as launches before it they save 1-2.5 % of a
+        // Step on small grids and under 1 % from 128^3 on, but a projection that
+        // needs none (a fluid at rest, a loose tolerance) walks all their empty
+        // launches: 0.32 instead of 0.13 ms a Step at 48x32x64, 0.85 instead of
+        // 0.55 at 128^3, and a graph of three passes to capture for one
+        // af_project (0.62 instead of 0.25 ms).
+        // A launch that the device refused has ended the capture: the graph and
+        // its nodes are then no longer ours to use.
         rc = cudaStreamGetCaptureInfo(s, &cs, nullptr, &graph, &deps, nullptr, &ndeps);
         if (rc != cudaSuccess || cs != cudaStreamCaptureStatusActive) {
             b->capture_err = rc != cudaSuccess ? rc : cudaErrorStreamCaptureInvalidated;
