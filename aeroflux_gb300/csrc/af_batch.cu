@@ -1719,14 +1719,18 @@ __global__ void __launch_bounds__(kMarchT[K], kMarchBlocks[K])
 // a wall cell writes its ghosts too), so neighbours sit at fixed offsets
 // without tests.  A thread keeps its cells of a level -- index, walls, r and
 // its own e -- in registers over all of the level's sweeps.  From the first
-// level of at most kWarpSlots cells a colour on, one warp runs the rest of
-// the way down and back up with warp barriers instead of block ones.
+// level of at most a cell of a colour a lane (kWarpSlots) on, one warp runs the
+// rest of the way down and back up with warp barriers instead of block ones.
+// With two to four cells a lane it is slower than the block, above all on
+// coarsest levels of odd extents, which take many sweeps: ms a Step at 128, 64
+// and 32 slots 20^3 1.36, 0.93, 0.93, 15x15x1 2.94, 0.92, 0.92, 9x9x1 0.78, 0.78,
+// 0.45, 12x20x28 1.93, 1.12, 1.12, 48x32x64 1.40, 1.35, 1.35.
 // A visit's loops appear once and work on copies of its levels' records, and
 // shared memory is indexed as such: the chain otherwise waits on instruction
 // fetches and generic loads.  Measured per Step with index decoding, wall
 // tests and block barriers in every sweep / so: 16^3 (a tail alone, 14
 // V-cycles) 0.72 / 0.59 ms, 48x32x64 1.44 / 1.38 ms, 256^3 10.40 / 10.27 ms.
-constexpr int kWarpSlots = 128;
+constexpr int kWarpSlots = 32;  // at most the lanes of a warp
 // The most dynamic shared memory a tail takes (plan_tail): ghost cells on
 // every side make the thinnest hierarchy, 2 x 2 x 1024 cells, the largest.  The
 // limit belongs to the kernel, not to a batch, so every batch sets this one: a
@@ -1880,7 +1884,7 @@ __device__ __noinline__ void tail_smooth_thin(const TailMem M, const TailLvl* lv
 // Sum over the coarsest level's cells in the fixed order of 512 threads: a
 // partial each over cells i, i + 512, ..., a shuffle tree over each warp, one
 // over the warps.  One warp forms the same tree where the level has at most
-// 256 cells.
+// 64 cells.
 template <bool WARP, class F>
 __device__ __forceinline__ float tail_sum(int n, float* red, F cell) {
     if (!WARP) {
@@ -1959,8 +1963,8 @@ __device__ __noinline__ void tail_levels(const TailMem M, const TailLvl* lv, int
             Gr::sync();
         }
         const int pairs = coarsest ? coarse_sweeps : nu;
-        if (F.S.slots() <= Gr::N) tail_smooth_n<WARP, 1>(M, F, pairs);
-        else if (WARP || F.S.slots() <= 4 * Gr::N) tail_smooth_n<WARP, 4>(M, F, pairs);
+        if (WARP || F.S.slots() <= Gr::N) tail_smooth_n<WARP, 1>(M, F, pairs);  // kWarpSlots: a warp's lanes
+        else if (F.S.slots() <= 4 * Gr::N) tail_smooth_n<WARP, 4>(M, F, pairs);
         else tail_smooth_thin(M, lv + l, pairs);
         if (coarsest) {
             const float mean_e = tail_sum<WARP>(n, red, [&](int i) {

@@ -1,0 +1,58 @@
+"""The one-block tail V-cycle on thin and uneven hierarchies, against the
+restatement bit for bit, and its time where a shape has cost it before."""
+import time
+
+import pytest
+
+from aeroflux_gb300 import New
+from tests.helpers import FIELDS
+from tests.test_gpu_mixed_bits import assert_same, env, make_mixed_pair, mixed_cfg
+
+pytestmark = pytest.mark.gpu
+
+
+# Thin tails, whose ghost cells take up to four times their own space; levels
+# of 32 cells of a colour and next to it (one warp's), of 512, 2048 and more;
+# coarsest levels of odd extents, solved with many sweeps.
+@pytest.mark.parametrize("n", [(2, 2, 1024), (2, 1024, 2), (1024, 2, 2), (2, 2, 64), (1, 64, 64), (64, 1, 64), (4, 32, 32),
+                               (1, 1, 4096), (4096, 1, 1), (2, 3, 512), (3, 5, 7), (5, 7, 9), (15, 15, 1), (3, 3, 7), (4, 4, 4),
+                               (8, 4, 4), (10, 6, 10), (20, 20, 20), (6, 10, 14), (12, 20, 28), (1, 8, 4), (1, 3, 11), (7, 2, 8),
+                               (16, 16, 16), (17, 15, 16)])
+def test_tail_vcycle_bit_exact(n):
+    e, o = make_mixed_pair(n, env_kw={"AEROFLUX_FIXED_REFINEMENT_PASSES": 1, "AEROFLUX_MG_VCYCLES": 2},
+                           orc_kw={"fixed_passes": 1, "vcycles": 2}, DT=0.256 / max(n))
+    e.project()
+    o.project()
+    assert_same(e.download, o, ("P", "U", "V", "W", "Div"), f"{n} two V-cycles")
+    e.Close()
+
+
+@pytest.mark.parametrize("n", [(20, 20, 20), (6, 10, 14), (2, 2, 128), (15, 9, 1)])
+def test_tail_steps_bit_exact(n):
+    e, o = make_mixed_pair(n, DT=0.256 / max(n))
+    e.Step(2)
+    o.step(2)
+    assert e.LastProjectionStats()[0] == o.passes
+    assert_same(e.download, o, FIELDS, f"{n} two Steps")
+    e.Close()
+
+
+def step_ms(e, steps=20):
+    e.SeedDevice(1.0, 0.01, 42, 0)
+    e.applyVelocityBC()
+    e.Step(5)
+    best = float("inf")
+    for _ in range(5):
+        t = time.perf_counter()
+        e.Step(steps)
+        best = min(best, time.perf_counter() - t)
+    e.Close()
+    return best / steps * 1e3
+
+
+def test_a_coarsest_level_of_odd_extents_costs_no_more_a_sweep():
+    # 450 pairs over 120 slots a colour against 1000 pairs over 240: the smaller
+    # level's pair is not the dearer one (on one warp it was three times that).
+    with env(AEROFLUX_FIXED_REFINEMENT_PASSES=1, AEROFLUX_MG_VCYCLES=1):
+        small, large = New(mixed_cfg((15, 15, 1))), New(mixed_cfg((31, 15, 1)))
+    assert step_ms(small) / 450 < 1.5 * step_ms(large) / 1000
