@@ -1910,14 +1910,14 @@ __device__ __forceinline__ float tail_sum(int n, float* red, F cell) {
 // One loop over the visits, each part of a visit written once (the chain of
 // short phases waits on instruction fetches otherwise); a visit works on a
 // copy of its levels' records (stores could alias the table).
-template <bool WARP>
+template <bool WARP, bool SMALL>
 __device__ __noinline__ void tail_levels(const TailMem M, const TailLvl* lv, int l0, int nl, int coarse_sweeps,
                                          float* red, int nu) {
     using Gr = TailGroup<WARP>;
     bool up = false;
     for (int l = l0; l >= l0;) {
         if (!WARP && !up && lv[l].S.slots() <= kWarpSlots) {
-            if (threadIdx.x < 32) tail_levels<true>(M, lv, l, nl, coarse_sweeps, red, nu);
+            if (threadIdx.x < 32) tail_levels<true, SMALL>(M, lv, l, nl, coarse_sweeps, red, nu);
             __syncthreads();
             up = true;
             --l;
@@ -1963,7 +1963,8 @@ __device__ __noinline__ void tail_levels(const TailMem M, const TailLvl* lv, int
             Gr::sync();
         }
         const int pairs = coarsest ? coarse_sweeps : nu;
-        if (WARP || F.S.slots() <= Gr::N) tail_smooth_n<WARP, 1>(M, F, pairs);  // kWarpSlots: a warp's lanes
+        // WARP: at most kWarpSlots; SMALL: at most kCoarseThreads.
+        if (WARP || SMALL || F.S.slots() <= Gr::N) tail_smooth_n<WARP, 1>(M, F, pairs);
         else if (F.S.slots() <= 4 * Gr::N) tail_smooth_n<WARP, 4>(M, F, pairs);
         else tail_smooth_thin(M, lv + l, pairs);
         if (coarsest) {
@@ -2014,8 +2015,14 @@ __device__ __noinline__ void tail_levels(const TailMem M, const TailLvl* lv, int
     }
 }
 
-__global__ void __launch_bounds__(kCoarseThreads) kb_vtail(const InstDev* inst, const TailLvl* tables,
-                                                           const Ctl* ctl, Tab tab, int nu, int vc) {
+// SMALL: a batch of more slots than SMs whose tails' levels have at most a cell
+// of a colour a thread (tail_large).  The registers of larger levels' smoothing
+// are then not needed and two blocks fit an SM: with one, 256 grids of 5x7x9
+// took 1.07 ms a Step and take 0.80 so, 1024 of 8^3 2.15 and 1.79, 256 of 20^3 3.18
+// and 2.94; a single 8^3, with nothing to fill the second, 0.333 and 0.345.
+template <bool SMALL>
+__global__ void __launch_bounds__(kCoarseThreads, SMALL ? 2 : 1) kb_vtail(const InstDev* inst, const TailLvl* tables,
+                                                                          const Ctl* ctl, Tab tab, int nu, int vc) {
     begin_slot(inst, tab);
     if (vc_idle(ctl, tab.n, vc)) return;
     __shared__ float red[32];
@@ -2051,7 +2058,7 @@ __global__ void __launch_bounds__(kCoarseThreads) kb_vtail(const InstDev* inst, 
             }
         }
         __syncthreads();
-        tail_levels<false>(M, lv, t, nl, cs, red, nu);
+        tail_levels<false, SMALL>(M, lv, t, nl, cs, red, nu);
         for (int i = threadIdx.x; i < n; i += kCoarseThreads) {
             int x, y, z;
             T.cell(i, &x, &y, &z);
@@ -2208,6 +2215,7 @@ struct Batch {
     unsigned graph_march = 0;        // levels with marching pairs in the graph
     unsigned graph_single = 0;       // levels with in-place colour sweeps in the graph
     size_t tail_smem = 0;            // dynamic shared memory of the tail V-cycle
+    bool tail_large = false;         // the tail V-cycle's form: kb_vtail<!tail_large>
     int graph_nu = 0;                // smoothing sweeps the captured graph carries
     bool per_level = false;          // multigrid without the tail V-cycle above the coarsest level
     bool pairs = true;               // fused red-black pair smoothing below the tail
@@ -2306,6 +2314,14 @@ size_t tail_smem_bytes(const Batch* b) {
     for (const auto& s : b->slots)
         if (s.used && s.d.tail >= 0) m = std::max(m, (size_t)s.d.tail_floats * sizeof(float));
     return m;
+}
+
+// Whether some slot's tail has a level of more than a cell of a colour a
+// thread; the first one is the largest.
+bool tail_large(const Batch* b) {
+    for (const auto& s : b->slots)
+        if (s.used && s.d.tail >= 0 && SmLvl(s.d.lev[s.d.tail]).slots() > kCoarseThreads) return true;
+    return false;
 }
 
 // Items of stage `st` for slot `s` under shape sh.
@@ -2526,8 +2542,8 @@ void enq_vcycle(Batch* b, int vc, cudaStream_t s) {
         LAUNCH(b, S_RESTRICT + l, kb_restrict, b->d_inst, b->d_ctl, tab(b, S_RESTRICT + l), l, vc);
     }
     if (b->tail_smem) {
-        launch_pdl(kb_vtail, dim3(grid(b, S_COARSE)), dim3(kCoarseThreads), b->tail_smem, s, b->d_inst, b->d_tails,
-                   b->d_ctl, tab(b, S_COARSE), b->nu, vc);
+        launch_pdl(b->tail_large ? kb_vtail<false> : kb_vtail<true>, dim3(grid(b, S_COARSE)), dim3(kCoarseThreads),
+                   b->tail_smem, s, b->d_inst, b->d_tails, b->d_ctl, tab(b, S_COARSE), b->nu, vc);
         ++b->launches;
     }
     for (int l = 0; l < kMaxLev; ++l)
@@ -2690,8 +2706,9 @@ cudaError_t prepare(Batch* b) {
     const unsigned big = big_coarse_levels(b), pair = pair_levels(b, false), pairn = pair_levels(b, true),
                    single = single_levels(b), march = march_levels(b);
     const size_t tsm = tail_smem_bytes(b);
+    const bool large = tail_large(b);
     if (b->graph && (L > b->graph_levels || (big & ~b->graph_big) || (pair & ~b->graph_pair) ||
-                     (pairn & ~b->graph_pairn) || (march & ~b->graph_march) || (single & ~b->graph_single) || tsm > b->tail_smem ||
+                     (pairn & ~b->graph_pairn) || (march & ~b->graph_march) || (single & ~b->graph_single) || tsm > b->tail_smem || (large && !b->tail_large) ||
                      b->graph_nu != b->nu)) {
         cudaGraphExecDestroy(b->graph);
         b->graph = nullptr;
@@ -2704,6 +2721,7 @@ cudaError_t prepare(Batch* b) {
         b->graph_march |= march;
         b->graph_single |= single;
         b->tail_smem = std::max(b->tail_smem, tsm);
+        b->tail_large |= large;
         b->graph_nu = b->nu;
         b->launches = 0;
         size_grids(b);
@@ -2831,7 +2849,10 @@ Batch* batch_create(int capacity, size_t pool_bytes, std::string* err) {
     cudaFuncSetAttribute(kb_sweep_tma<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSwSmem);
     cudaFuncSetAttribute(kb_sweep_tma<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSwSmem);
     cudaFuncSetAttribute(kb_sweep_tma<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSwSmem);
-    cudaFuncSetAttribute(kb_vtail, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmem);
+    cudaFuncSetAttribute(kb_vtail<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmem);
+    cudaFuncSetAttribute(kb_vtail<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmem);
+    // No more slots than SMs: a second block an SM would have no tail to take.
+    b->tail_large = capacity <= b->sms;
     // Shapes: the tiny per-slot control and coarse stages keep their own.
     b->shape[S_COARSE] = Shape{kCoarseThreads, 1, 2};
     for (int l = 0; l < kMaxLev; ++l) {
@@ -3291,6 +3312,7 @@ cudaError_t batch_prepare_capture(Batch* b) {
     b->graph_march |= march_levels(b);
     b->graph_single |= single_levels(b);
     b->tail_smem = std::max(b->tail_smem, tail_smem_bytes(b));
+    b->tail_large |= tail_large(b);
     size_grids(b);
     return cudaSuccess;
 }

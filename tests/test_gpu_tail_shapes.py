@@ -5,6 +5,7 @@ import time
 import pytest
 
 from aeroflux_gb300 import New
+from aeroflux_gb300.batch import Batch
 from tests.helpers import FIELDS
 from tests.test_gpu_mixed_bits import assert_same, env, make_mixed_pair, mixed_cfg
 
@@ -56,3 +57,53 @@ def test_a_coarsest_level_of_odd_extents_costs_no_more_a_sweep():
     with env(AEROFLUX_FIXED_REFINEMENT_PASSES=1, AEROFLUX_MG_VCYCLES=1):
         small, large = New(mixed_cfg((15, 15, 1))), New(mixed_cfg((31, 15, 1)))
     assert step_ms(small) / 450 < 1.5 * step_ms(large) / 1000
+
+
+@pytest.mark.parametrize("n,later", [((5, 7, 9), (4, 4, 4)), ((5, 7, 9), (16, 16, 16)), ((16, 16, 16), (5, 7, 9))])
+def test_tails_of_a_batch_of_more_slots_than_sms(n, later):
+    # Small tails, two blocks an SM; a larger one that joins later changes the
+    # form.  Slots of one configuration and field step to the same bits.
+    b, count = Batch(320), 310
+    cfg = mixed_cfg(n, DT=0.256 / max(n))
+    e, o = make_mixed_pair(n, DT=0.256 / max(n))
+    e.Close()
+
+    def fill(slot, orc):
+        for i, name in enumerate(("U", "V", "W"), start=1):
+            b.upload(slot, name, orc.data(i))
+
+    slots = [b.assign(cfg) for _ in range(count)]
+    for s in slots:
+        fill(s, o)
+    b.step(1)
+    o.step(1)
+    e, o2 = make_mixed_pair(later, DT=0.256 / max(later))
+    e.Close()
+    s2 = b.assign(mixed_cfg(later, DT=0.256 / max(later)))
+    fill(s2, o2)
+    b.step(1)
+    o.step(1)
+    o2.step(1)
+    for s in (slots[0], slots[151], slots[152], slots[-1]):
+        assert_same(lambda name: b.download(s, name), o, FIELDS, f"slot {s}")
+    assert_same(lambda name: b.download(s2, name), o2, FIELDS, "the later slot")
+    b.close()
+
+
+def test_small_tails_of_two_slots_an_sm_overlap():
+    def ms(count):
+        b = Batch(304)
+        for k in range(count):
+            b.seed(b.assign(mixed_cfg((5, 7, 9), DT=0.256 / 9)), 1.0, 0.01, 42, k)
+        b.apply_velocity_bc()
+        b.step(5)
+        best = float("inf")
+        for _ in range(5):
+            t = time.perf_counter()
+            b.step(20)
+            best = min(best, time.perf_counter() - t)
+        b.close()
+        return best
+
+    # One tail after the other on every SM takes about 1.7 times as long.
+    assert ms(304) < 1.45 * ms(152)
