@@ -1861,6 +1861,60 @@ __device__ __forceinline__ void tail_smooth_n(const TailMem& M, const TailLvl& L
         }
 }
 
+// Many pairs (a coarsest level's solve) of a level of at most a cell of a
+// colour a thread.  A neighbour across a wall is the cell itself here, by its
+// index, and the ghosts, which only the phases around the sweeps read, are
+// written by the last pair: on thin levels every cell lies at two to four
+// walls.  ms a Step with ghosts in every pair / so: 8x4x194 7.42 / 5.40, 2x2x97
+// 31.2 / 22.7, 15x15x1 0.92 / 0.82, 5x7x9 0.55 / 0.49.  For few pairs its set-up
+// costs more than it saves, and its presence alone costs the other levels
+// registers (16^3 0.613 / 0.656, 48x32x64 with 18 pairs 1.305 / 1.34), so only the
+// forms with MANY hold it.
+constexpr int kManyPairs = 32;
+template <bool WARP>
+__device__ __noinline__ void tail_smooth_many(const TailMem M, const TailLvl* lv, int pairs) {
+    using Gr = TailGroup<WARP>;
+    const TailLvl L = *lv;
+    const SmLvl& S = L.S;
+    const MgW W = L.W;
+    const float inv = L.inv;
+    const int m = Gr::id();
+    const unsigned q = L.fhx.div((unsigned)m), zz = L.fny.div(q);
+    const int j = m - (int)q * S.hx, y = (int)q - (int)zz * S.ny, z = (int)zz;
+    int at[2], nb[2][6];
+    unsigned walls[2];
+    float rr[2], own[2];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        const int x = 2 * j + (((y + z) & 1) != c ? 1 : 0);
+        at[c] = -1;
+        if (m < S.slots() && x < S.nx) {
+            const int i = L.at(x, y, z);
+            at[c] = i;
+            walls[c] = L.walls(x, y, z);
+            rr[c] = M[L.r + x + S.nx * (int)q];
+            own[c] = M[i];
+#pragma unroll
+            for (int k = 0; k < 6; ++k) {
+                const int d = k < 2 ? S.dx : (k < 4 ? S.dy : S.dz);
+                nb[c][k] = (walls[c] >> k) & 1u ? i : (k & 1 ? i + d : i - d);
+            }
+        }
+    }
+    for (int p = 0; p < pairs; ++p)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            if (at[c] >= 0) {
+                const float v = mg_relax(W, M[nb[c][0]] + M[nb[c][1]], M[nb[c][2]] + M[nb[c][3]],
+                                         M[nb[c][4]] + M[nb[c][5]], rr[c], inv, own[c]);
+                own[c] = v;
+                if (p + 1 < pairs) M[at[c]] = v;
+                else tail_put(M, S, at[c], walls[c], v);
+            }
+            Gr::sync();
+        }
+}
+
 // Thin levels of more slots than four a thread (half of a row's slots may be
 // of no colour): decoded in every sweep.
 __device__ __noinline__ void tail_smooth_thin(const TailMem M, const TailLvl* lv, int pairs) {
@@ -1910,14 +1964,14 @@ __device__ __forceinline__ float tail_sum(int n, float* red, F cell) {
 // One loop over the visits, each part of a visit written once (the chain of
 // short phases waits on instruction fetches otherwise); a visit works on a
 // copy of its levels' records (stores could alias the table).
-template <bool WARP, bool SMALL>
+template <bool WARP, bool SMALL, bool MANY>
 __device__ __noinline__ void tail_levels(const TailMem M, const TailLvl* lv, int l0, int nl, int coarse_sweeps,
                                          float* red, int nu) {
     using Gr = TailGroup<WARP>;
     bool up = false;
     for (int l = l0; l >= l0;) {
         if (!WARP && !up && lv[l].S.slots() <= kWarpSlots) {
-            if (threadIdx.x < 32) tail_levels<true, SMALL>(M, lv, l, nl, coarse_sweeps, red, nu);
+            if (threadIdx.x < 32) tail_levels<true, SMALL, MANY>(M, lv, l, nl, coarse_sweeps, red, nu);
             __syncthreads();
             up = true;
             --l;
@@ -1964,7 +2018,10 @@ __device__ __noinline__ void tail_levels(const TailMem M, const TailLvl* lv, int
         }
         const int pairs = coarsest ? coarse_sweeps : nu;
         // WARP: at most kWarpSlots; SMALL: at most kCoarseThreads.
-        if (WARP || SMALL || F.S.slots() <= Gr::N) tail_smooth_n<WARP, 1>(M, F, pairs);
+        if (WARP || SMALL || F.S.slots() <= Gr::N) {
+            if (MANY && pairs > kManyPairs) tail_smooth_many<WARP>(M, lv + l, pairs);
+            else tail_smooth_n<WARP, 1>(M, F, pairs);
+        }
         else if (F.S.slots() <= 4 * Gr::N) tail_smooth_n<WARP, 4>(M, F, pairs);
         else tail_smooth_thin(M, lv + l, pairs);
         if (coarsest) {
@@ -2016,11 +2073,12 @@ __device__ __noinline__ void tail_levels(const TailMem M, const TailLvl* lv, int
 }
 
 // SMALL: a batch of more slots than SMs whose tails' levels have at most a cell
-// of a colour a thread (tail_large).  The registers of larger levels' smoothing
+// of a colour a thread (tail_form).  The registers of larger levels' smoothing
 // are then not needed and two blocks fit an SM: with one, 256 grids of 5x7x9
 // took 1.07 ms a Step and take 0.80 so, 1024 of 8^3 2.15 and 1.79, 256 of 20^3 3.18
 // and 2.94; a single 8^3, with nothing to fill the second, 0.333 and 0.345.
-template <bool SMALL>
+// MANY: some slot's coarsest level takes more than kManyPairs pairs.
+template <bool SMALL, bool MANY>
 __global__ void __launch_bounds__(kCoarseThreads, SMALL ? 2 : 1) kb_vtail(const InstDev* inst, const TailLvl* tables,
                                                                           const Ctl* ctl, Tab tab, int nu, int vc) {
     begin_slot(inst, tab);
@@ -2058,7 +2116,7 @@ __global__ void __launch_bounds__(kCoarseThreads, SMALL ? 2 : 1) kb_vtail(const 
             }
         }
         __syncthreads();
-        tail_levels<false, SMALL>(M, lv, t, nl, cs, red, nu);
+        tail_levels<false, SMALL, MANY>(M, lv, t, nl, cs, red, nu);
         for (int i = threadIdx.x; i < n; i += kCoarseThreads) {
             int x, y, z;
             T.cell(i, &x, &y, &z);
@@ -2215,7 +2273,7 @@ struct Batch {
     unsigned graph_march = 0;        // levels with marching pairs in the graph
     unsigned graph_single = 0;       // levels with in-place colour sweeps in the graph
     size_t tail_smem = 0;            // dynamic shared memory of the tail V-cycle
-    bool tail_large = false;         // the tail V-cycle's form: kb_vtail<!tail_large>
+    int tail_form = 0;               // kTailLarge, kTailMany: the tail V-cycle's kernel (kTailKernels)
     int graph_nu = 0;                // smoothing sweeps the captured graph carries
     bool per_level = false;          // multigrid without the tail V-cycle above the coarsest level
     bool pairs = true;               // fused red-black pair smoothing below the tail
@@ -2316,12 +2374,19 @@ size_t tail_smem_bytes(const Batch* b) {
     return m;
 }
 
-// Whether some slot's tail has a level of more than a cell of a colour a
-// thread; the first one is the largest.
-bool tail_large(const Batch* b) {
-    for (const auto& s : b->slots)
-        if (s.used && s.d.tail >= 0 && SmLvl(s.d.lev[s.d.tail]).slots() > kCoarseThreads) return true;
-    return false;
+// What the tail V-cycle's kernel must hold: a level of more than a cell of a
+// colour a thread (the first one is the largest), many pairs at the coarsest.
+constexpr int kTailLarge = 1, kTailMany = 2;
+void (*const kTailKernels[4])(const InstDev*, const TailLvl*, const Ctl*, Tab, int, int) = {
+    kb_vtail<true, false>, kb_vtail<false, false>, kb_vtail<true, true>, kb_vtail<false, true>};
+int tail_form(const Batch* b) {
+    int f = 0;
+    for (const auto& s : b->slots) {
+        if (!s.used || s.d.tail < 0) continue;
+        if (SmLvl(s.d.lev[s.d.tail]).slots() > kCoarseThreads) f |= kTailLarge;
+        if (s.d.coarse_sweeps > kManyPairs) f |= kTailMany;
+    }
+    return f;
 }
 
 // Items of stage `st` for slot `s` under shape sh.
@@ -2542,7 +2607,7 @@ void enq_vcycle(Batch* b, int vc, cudaStream_t s) {
         LAUNCH(b, S_RESTRICT + l, kb_restrict, b->d_inst, b->d_ctl, tab(b, S_RESTRICT + l), l, vc);
     }
     if (b->tail_smem) {
-        launch_pdl(b->tail_large ? kb_vtail<false> : kb_vtail<true>, dim3(grid(b, S_COARSE)), dim3(kCoarseThreads),
+        launch_pdl(kTailKernels[b->tail_form], dim3(grid(b, S_COARSE)), dim3(kCoarseThreads),
                    b->tail_smem, s, b->d_inst, b->d_tails, b->d_ctl, tab(b, S_COARSE), b->nu, vc);
         ++b->launches;
     }
@@ -2706,9 +2771,9 @@ cudaError_t prepare(Batch* b) {
     const unsigned big = big_coarse_levels(b), pair = pair_levels(b, false), pairn = pair_levels(b, true),
                    single = single_levels(b), march = march_levels(b);
     const size_t tsm = tail_smem_bytes(b);
-    const bool large = tail_large(b);
+    const int form = tail_form(b);
     if (b->graph && (L > b->graph_levels || (big & ~b->graph_big) || (pair & ~b->graph_pair) ||
-                     (pairn & ~b->graph_pairn) || (march & ~b->graph_march) || (single & ~b->graph_single) || tsm > b->tail_smem || (large && !b->tail_large) ||
+                     (pairn & ~b->graph_pairn) || (march & ~b->graph_march) || (single & ~b->graph_single) || tsm > b->tail_smem || (form & ~b->tail_form) ||
                      b->graph_nu != b->nu)) {
         cudaGraphExecDestroy(b->graph);
         b->graph = nullptr;
@@ -2721,7 +2786,7 @@ cudaError_t prepare(Batch* b) {
         b->graph_march |= march;
         b->graph_single |= single;
         b->tail_smem = std::max(b->tail_smem, tsm);
-        b->tail_large |= large;
+        b->tail_form |= form;
         b->graph_nu = b->nu;
         b->launches = 0;
         size_grids(b);
@@ -2849,10 +2914,9 @@ Batch* batch_create(int capacity, size_t pool_bytes, std::string* err) {
     cudaFuncSetAttribute(kb_sweep_tma<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSwSmem);
     cudaFuncSetAttribute(kb_sweep_tma<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSwSmem);
     cudaFuncSetAttribute(kb_sweep_tma<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSwSmem);
-    cudaFuncSetAttribute(kb_vtail<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmem);
-    cudaFuncSetAttribute(kb_vtail<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmem);
+    for (const auto k : kTailKernels) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmem);
     // No more slots than SMs: a second block an SM would have no tail to take.
-    b->tail_large = capacity <= b->sms;
+    b->tail_form = capacity <= b->sms ? kTailLarge : 0;
     // Shapes: the tiny per-slot control and coarse stages keep their own.
     b->shape[S_COARSE] = Shape{kCoarseThreads, 1, 2};
     for (int l = 0; l < kMaxLev; ++l) {
@@ -3312,7 +3376,7 @@ cudaError_t batch_prepare_capture(Batch* b) {
     b->graph_march |= march_levels(b);
     b->graph_single |= single_levels(b);
     b->tail_smem = std::max(b->tail_smem, tail_smem_bytes(b));
-    b->tail_large |= tail_large(b);
+    b->tail_form |= tail_form(b);
     size_grids(b);
     return cudaSuccess;
 }

@@ -107,3 +107,33 @@ def test_small_tails_of_two_slots_an_sm_overlap():
 
     # One tail after the other on every SM takes about 1.7 times as long.
     assert ms(304) < 1.45 * ms(152)
+
+
+@pytest.mark.parametrize("n", [(2, 2, 97), (97, 2, 2), (1, 1, 51), (5, 5, 5), (9, 9, 1), (6, 10, 14)])
+def test_tails_of_a_batch_with_many_pairs(n):
+    # Coarsest levels solved with more than 32 pairs, among slots of few: in a
+    # batch of more slots than SMs and in one of fewer.
+    for capacity in (200, 3):
+        b = Batch(capacity)
+        orcs = {}
+        for k, dims in enumerate((n, (8, 8, 8), n)):
+            e, o = make_mixed_pair(dims, DT=0.256 / max(dims), noise=0.01 * (k + 1))
+            e.Close()
+            s = b.assign(mixed_cfg(dims, DT=0.256 / max(dims)))
+            for i, name in enumerate(("U", "V", "W"), start=1):
+                b.upload(s, name, o.data(i))
+            orcs[s] = o
+        b.step(1)
+        for s, o in orcs.items():
+            o.step(1)
+            assert_same(lambda name: b.download(s, name), o, FIELDS, f"{n} slot {s} of {capacity}")
+        b.close()
+
+
+def test_a_thin_coarsest_level_does_not_pay_for_its_walls():
+    # 1000 pairs over 194 cells of a colour, all at two walls or three, against
+    # 1000 over 564, most at none: 0.53 of the time (with ghosts written in every
+    # pair 0.70).
+    with env(AEROFLUX_FIXED_REFINEMENT_PASSES=1, AEROFLUX_MG_VCYCLES=1):
+        thin, wide = New(mixed_cfg((2, 2, 97))), New(mixed_cfg((7, 7, 23)))
+    assert step_ms(thin) < 0.62 * step_ms(wide)
