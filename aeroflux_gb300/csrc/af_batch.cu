@@ -1752,6 +1752,7 @@ struct SmLvl {
     }
     __host__ __device__ int cells() const { return nx * ny * nz; }
     __host__ __device__ int slots() const { return hx * ny * nz; }  // of one colour
+    __host__ __device__ bool thin() const { return nx == 2 || ny == 2 || nz == 2; }  // every cell at a wall
 };
 
 // What the tail reads of a level, in shared memory: its layout, the places of
@@ -1915,6 +1916,69 @@ __device__ __noinline__ void tail_smooth_many(const TailMem M, const TailLvl* lv
         }
 }
 
+// The same for levels of more than four slots a thread (rows of few cells waste
+// half of theirs) and thin ones of more than one: a coarsest level, its e zero, in
+// the space of its padded e but without ghosts, so that a register holds a cell's
+// place and walls over all sweeps; then spread over the padded layout.  ms a Step
+// decoding in every sweep / with fixed offsets and ghosts / so: 1x63x65 58 / 80 /
+// 41, 7x23x25 14.1 / 22.5 / 11.9, 2x45x45 39.5 / 54 / 24, 2x173x7 156 / 192 / 106; fixed
+// offsets are better for the others of up to four (5x15x41 26.7 / 20.9).
+template <int NC>
+__device__ __noinline__ void tail_solve_plain(const TailMem M, const TailLvl* lv, int pairs) {
+    const TailLvl L = *lv;
+    const SmLvl& S = L.S;
+    const int n = S.cells(), nx = S.nx, nxy = S.nx * S.ny, r = L.r - L.e0;
+    const MgW W = L.W;
+    const float inv = L.inv;
+    int at[2][NC];  // walls << 20 | place of e, -1: none
+#pragma unroll
+    for (int k = 0; k < NC; ++k) {
+        const int m = (int)threadIdx.x + k * kCoarseThreads;
+        const unsigned q = L.fhx.div((unsigned)m), zz = L.fny.div(q);
+        const int j = m - (int)q * S.hx, y = (int)q - (int)zz * S.ny, z = (int)zz;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const int x = 2 * j + (((y + z) & 1) != c ? 1 : 0);
+            unsigned w = (x == 0 ? 1u : 0u) | (x == nx - 1 ? 2u : 0u) | (y == 0 ? 4u : 0u) | (y == S.ny - 1 ? 8u : 0u) |
+                         (z == 0 ? 16u : 0u) | (z == S.nz - 1 ? 32u : 0u);
+            at[c][k] = m < S.slots() && x < nx ? (int)(w << 20) | (L.e0 + x + nx * (int)q) : -1;
+        }
+    }
+    for (int p = 0; p < pairs; ++p)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+#pragma unroll
+            for (int k = 0; k < NC; ++k)
+                if (at[c][k] >= 0) {
+                    const int e = at[c][k] & 0xFFFFF;
+                    const unsigned w = (unsigned)at[c][k] >> 20;
+                    const float o = M[e];
+                    const float sx = (w & 1u ? o : M[e - 1]) + (w & 2u ? o : M[e + 1]);
+                    const float sy = (w & 4u ? o : M[e - nx]) + (w & 8u ? o : M[e + nx]);
+                    const float sz = (w & 16u ? o : M[e - nxy]) + (w & 32u ? o : M[e + nxy]);
+                    M[e] = mg_relax(W, sx, sy, sz, M[e + r], inv, o);
+                }
+            __syncthreads();
+        }
+    float v[kCoarseMax / kCoarseThreads];
+#pragma unroll
+    for (int k = 0; k < kCoarseMax / kCoarseThreads; ++k) {
+        const int i = (int)threadIdx.x + k * kCoarseThreads;
+        if (i < n) v[k] = M[L.e0 + i];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kCoarseMax / kCoarseThreads; ++k) {
+        const int i = (int)threadIdx.x + k * kCoarseThreads;
+        if (i < n) {
+            int x, y, z;
+            L.cell(i, &x, &y, &z);
+            tail_put(M, S, L.at(x, y, z), L.walls(x, y, z), v[k]);
+        }
+    }
+    __syncthreads();
+}
+
 // Thin levels of more slots than four a thread (half of a row's slots may be
 // of no colour): decoded in every sweep.
 __device__ __noinline__ void tail_smooth_thin(const TailMem M, const TailLvl* lv, int pairs) {
@@ -2017,13 +2081,18 @@ __device__ __noinline__ void tail_levels(const TailMem M, const TailLvl* lv, int
             Gr::sync();
         }
         const int pairs = coarsest ? coarse_sweeps : nu;
-        // WARP: at most kWarpSlots; SMALL: at most kCoarseThreads.
+        // WARP: at most kWarpSlots slots; SMALL: at most kCoarseThreads.
+        const bool many = MANY && pairs > kManyPairs;
         if (WARP || SMALL || F.S.slots() <= Gr::N) {
-            if (MANY && pairs > kManyPairs) tail_smooth_many<WARP>(M, lv + l, pairs);
+            if (many) tail_smooth_many<WARP>(M, lv + l, pairs);
             else tail_smooth_n<WARP, 1>(M, F, pairs);
+        } else if (F.S.slots() <= 4 * Gr::N) {
+            if (many && F.S.thin()) tail_solve_plain<4>(M, lv + l, pairs);
+            else tail_smooth_n<WARP, 4>(M, F, pairs);
+        } else {
+            if (many) tail_solve_plain<8>(M, lv + l, pairs);
+            else tail_smooth_thin(M, lv + l, pairs);
         }
-        else if (F.S.slots() <= 4 * Gr::N) tail_smooth_n<WARP, 4>(M, F, pairs);
-        else tail_smooth_thin(M, lv + l, pairs);
         if (coarsest) {
             const float mean_e = tail_sum<WARP>(n, red, [&](int i) {
                 int x, y, z;

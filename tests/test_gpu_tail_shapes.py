@@ -137,3 +137,24 @@ def test_a_thin_coarsest_level_does_not_pay_for_its_walls():
     with env(AEROFLUX_FIXED_REFINEMENT_PASSES=1, AEROFLUX_MG_VCYCLES=1):
         thin, wide = New(mixed_cfg((2, 2, 97))), New(mixed_cfg((7, 7, 23)))
     assert step_ms(thin) < 0.62 * step_ms(wide)
+
+
+# Coarsest levels of many pairs with several cells of a colour a thread: more
+# than four (2048 slots and next to it), every cell at a wall, neither.
+@pytest.mark.parametrize("n", [(7, 23, 25), (1, 45, 45), (45, 45, 1), (3, 33, 31), (5, 21, 39), (2, 25, 27), (27, 2, 25), (25, 27, 2),
+                               (5, 15, 41), (1, 2047, 1), (1, 63, 65), (9, 3, 151)])
+def test_large_coarsest_levels_bit_exact(n):
+    e, o = make_mixed_pair(n, env_kw={"AEROFLUX_FIXED_REFINEMENT_PASSES": 1, "AEROFLUX_MG_VCYCLES": 1},
+                           orc_kw={"fixed_passes": 1, "vcycles": 1}, DT=0.256 / max(n))
+    e.project()
+    o.project()
+    assert_same(e.download, o, ("P", "U", "V", "W", "Div"), f"{n} one V-cycle")
+    e.Close()
+
+
+def test_a_large_coarsest_level_costs_by_its_slots():
+    # 1000 pairs each; 7x23x25 has 2300 slots a colour, 7x21x23 has 1932, within
+    # four a thread: 1.1 of the time (with ghosts written in every pair 2.05).
+    with env(AEROFLUX_FIXED_REFINEMENT_PASSES=1, AEROFLUX_MG_VCYCLES=1):
+        large, small = New(mixed_cfg((7, 23, 25))), New(mixed_cfg((7, 21, 23)))
+    assert step_ms(large, 5) < 1.6 * step_ms(small, 5)
