@@ -781,11 +781,15 @@ __global__ void __launch_bounds__(kDiagThreads) k_max_abs3(const double* __restr
 // is bit-identical run to run (it differs from the serial sum by rounding).
 constexpr int kKeThreads = 256;
 // Partial sums at most, and the rows of a block: enough blocks to fill the
-// GPU, as the grid alone decides.
+// GPU, as the grid alone decides.  Short rows, and planes of fewer rows than
+// half of a block's warps, are dealt out cell by cell instead of a row a warp,
+// 1024 cells or more to a block.  us a call, a row a warp / so: 1x1000x1000
+// 414 / 40, 8x512x512 163 / 52, 16x512x512 188 / 81, 1000x1x1000 77 / 40.
 constexpr int kKeMaxPartials = 16384;
-__host__ __device__ inline int ke_rows(int NY, int NZ) {
-    int per = kKeThreads / 32;  // a row a warp
-    while ((long long)NZ * ((NY + per - 1) / per) > kKeMaxPartials && per < NY) per *= 2;
+inline bool ke_dense(const Geom& g) { return g.NX < 32 || g.NY < kKeThreads / 64; }
+inline int ke_rows(const Geom& g) {
+    int per = ke_dense(g) ? (1024 + g.NX - 1) / g.NX : kKeThreads / 32;  // a row a warp
+    while ((long long)g.NZ * ((g.NY + per - 1) / per) > kKeMaxPartials && per < g.NY) per *= 2;
     return per;
 }
 
@@ -805,7 +809,8 @@ __device__ __forceinline__ double block_sum_fixed(double s) {
 
 // Per cell three additions of face pairs (one of them on the integer pipe),
 // three exact halvings (exponent) and three fused multiply-adds.
-__global__ void __launch_bounds__(kKeThreads) k_ke_planes(const __grid_constant__ Geom g,
+template <bool DENSE>
+__global__ void __launch_bounds__(kKeThreads) k_ke_planes(const __grid_constant__ Geom g, const FastDiv fx,
                                                           const double* __restrict__ u_,
                                                           const double* __restrict__ v_,
                                                           const double* __restrict__ w_, int rows,
@@ -817,16 +822,26 @@ __global__ void __launch_bounds__(kKeThreads) k_ke_planes(const __grid_constant_
     AF_PTR(double) partials = view(partials_, (long long)gridDim.x * gridDim.y, DK_F64_KE, 0);
     const int z = G + (int)blockIdx.x, y0 = (int)blockIdx.y * rows;
     double s = 0.0;
-    for (int r = (int)threadIdx.x >> 5; r < rows && y0 + r < g.NY; r += kKeThreads / 32) {
-        const int y = G + y0 + r;
-        const long long iu = y * g.u.sy + z * g.u.sz, iv = y * g.v.sy + z * g.v.sz, iw = y * g.w.sy + z * g.w.sz;
-        for (int x = G + ((int)threadIdx.x & 31); x < G + g.NX; x += 32) {
-            const double uc = half(dadd_int(u[iu + x], u[iu + x + 1]));
-            const double vc = half(dadd(v[iv + x], v[iv + x + g.v.sy]));
-            const double wc = half(dadd(w[iw + x], w[iw + x + g.w.sz]));
-            s = __fma_rn(uc, uc, s);
-            s = __fma_rn(vc, vc, s);
-            s = __fma_rn(wc, wc, s);
+    auto cell = [&](long long iu, long long iv, long long iw) {
+        const double uc = half(dadd_int(u[iu], u[iu + 1]));
+        const double vc = half(dadd(v[iv], v[iv + g.v.sy]));
+        const double wc = half(dadd(w[iw], w[iw + g.w.sz]));
+        s = __fma_rn(uc, uc, s);
+        s = __fma_rn(vc, vc, s);
+        s = __fma_rn(wc, wc, s);
+    };
+    if (DENSE) {
+        const unsigned n = (unsigned)min(rows, g.NY - y0) * (unsigned)g.NX;
+        for (unsigned k = threadIdx.x; k < n; k += kKeThreads) {
+            const unsigned r = fx.div(k);
+            const int x = G + (int)(k - r * fx.d), y = G + y0 + (int)r;
+            cell(x + y * g.u.sy + z * g.u.sz, x + y * g.v.sy + z * g.v.sz, x + y * g.w.sy + z * g.w.sz);
+        }
+    } else {
+        for (int r = (int)threadIdx.x >> 5; r < rows && y0 + r < g.NY; r += kKeThreads / 32) {
+            const int y = G + y0 + r;
+            const long long iu = y * g.u.sy + z * g.u.sz, iv = y * g.v.sy + z * g.v.sz, iw = y * g.w.sy + z * g.w.sz;
+            for (int x = G + ((int)threadIdx.x & 31); x < G + g.NX; x += 32) cell(iu + x, iv + x, iw + x);
         }
     }
     s = block_sum_fixed(s);
@@ -1164,13 +1179,14 @@ bool fp64_debug_bounds(unsigned long long* first, unsigned* count, bool reset) {
     return true;
 }
 
-int kinetic_energy_partials(const Geom& g) { return g.NZ * (int)cdiv(g.NY, ke_rows(g.NY, g.NZ)); }
+int kinetic_energy_partials(const Geom& g) { return g.NZ * (int)cdiv(g.NY, ke_rows(g)); }
 
 void launch_kinetic_energy(const Geom& g, const double* u, const double* v, const double* w, double* partials,
                            double* out, cudaStream_t s) {
-    const int rows = ke_rows(g.NY, g.NZ);
+    const int rows = ke_rows(g);
     const dim3 grid(g.NZ, cdiv(g.NY, rows));
-    k_ke_planes<<<grid, kKeThreads, 0, s>>>(g, u, v, w, rows, partials);
+    const auto k = ke_dense(g) ? k_ke_planes<true> : k_ke_planes<false>;
+    k<<<grid, kKeThreads, 0, s>>>(g, FastDiv((unsigned)g.NX), u, v, w, rows, partials);
     k_ke_final<<<1, kKeThreads, 0, s>>>(partials, (int)(grid.x * grid.y), out);
 }
 
