@@ -56,7 +56,8 @@ cudaError_t batch_project(Batch* b, std::string* err);
 // (returns the kernel launches it added); after capture, check the error the
 // enqueue may have recorded.  Faults go to batch_status(b, slot).
 cudaError_t batch_prepare_capture(Batch* b);
-int64_t batch_enqueue_project(Batch* b, int parity, int gate, cudaStream_t s);
+// once: the capture is launched once only.
+int64_t batch_enqueue_project(Batch* b, int parity, int gate, cudaStream_t s, bool once);
 cudaError_t batch_capture_error(Batch* b);
 Status* batch_status(Batch* b, int slot);
 // applyVelocityBC of every active slot.

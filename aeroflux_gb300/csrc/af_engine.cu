@@ -342,13 +342,13 @@ void enqueue_project_fp64(af_engine* e, const Fields& f, int gate) {
 
 // `parity` is the U/V/W slot parity at this point of the step (the
 // multigrid projection addresses fields through the batch's slot table).
-void enqueue_project(af_engine* e, const Fields& f, int gate, int parity) {
+void enqueue_project(af_engine* e, const Fields& f, int gate, int parity, bool once = false) {
     if (!e->mg) {
         enqueue_project_fp64(e, f, gate);
         return;
     }
     rec(e, kEvRb + (gate == 3 ? 0 : 2));
-    e->launches_per_step += af::batch_enqueue_project(e->mg, parity, gate, e->stream);
+    e->launches_per_step += af::batch_enqueue_project(e->mg, parity, gate, e->stream, once);
     rec(e, kEvRb + (gate == 3 ? 1 : 3));
 }
 
@@ -778,7 +778,7 @@ int af_project(af_engine* e) {
         // The multigrid projection's refinement loop is a conditional graph
         // node, so even a single projection runs as a captured graph.
         cudaGraphExec_t g = nullptr;
-        if (int rc = capture_step(e, [&] { enqueue_project(e, e->fields(), 0, e->parity); }, &g)) return rc;
+        if (int rc = capture_step(e, [&] { enqueue_project(e, e->fields(), 0, e->parity, true); }, &g)) return rc;
         const cudaError_t lr = cudaGraphLaunch(g, e->stream);
         cudaStreamSynchronize(e->stream);
         cudaGraphExecDestroy(g);

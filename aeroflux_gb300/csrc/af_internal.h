@@ -116,8 +116,9 @@ struct Fields {
 // 2.79, 128^3 11.5 -> 11.0, 256^3 79.1 -> 77.8; with the trigger at the
 // kernel's start, where the early blocks take residency from the running
 // ones, 64^3 3.54.
+// overlap = false launches it in the usual way.
 template <class... P, class... A>
-void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+void launch_maybe_pdl(bool overlap, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -127,8 +128,12 @@ void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaSt
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = overlap ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+template <class... P, class... A>
+void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+    launch_maybe_pdl(true, kernel, grid, block, smem, s, args...);
 }
 #if defined(__CUDACC__)
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
