@@ -2367,6 +2367,7 @@ struct Batch {
     bool tmaps_dirty = true;
     unsigned march = ~0u;              // levels whose fused pairs march where a slot's level allows it
     int force_pair_var = -1;           // AEROFLUX_PAIR_VARIANT: every fused pair stage's variant (-1: tuned)
+    int force_march = -1;              // AEROFLUX_MARCH_SHAPE: every marching pair's shape (-1: tuned)
     bool pair_chosen = false;          // the fused pairs' tile variants are set (tuned or by level size)
     unsigned march_polls = kMarchPolls;  // AEROFLUX_MARCH_POLLS: march_wait's first polls (0: every wait gives up)
     unsigned* d_diag = nullptr;        // nonzero: a kernel gave up a bounded wait; lies behind the statuses
@@ -2827,7 +2828,8 @@ void default_pair_variants(Batch* b) {
         for (const auto& S : b->slots)
             if (S.used && l < S.d.nlev) most = std::max(most, lvl_cells(S.d.lev[l]));
         int var = most >= (4ll << 20) ? 0 : (most >= (256ll << 10) ? 1 : 2);
-        b->shape[S_MARCH + l] = march_shape(most >= (4ll << 20) ? 7 : (most >= (256ll << 10) ? 1 : 0));
+        b->shape[S_MARCH + l] = march_shape(b->force_march >= 0 ? b->force_march
+                                                                : (most >= (4ll << 20) ? 7 : (most >= (256ll << 10) ? 1 : 0)));
         if (b->force_pair_var >= 0 && b->force_pair_var != 3) var = b->force_pair_var;
         b->shape[S_PAIR + l] = pair_shape(true, var);
         b->shape[S_PAIRN + l] = pair_shape(false, var);
@@ -3015,6 +3017,10 @@ Batch* batch_create(int capacity, size_t pool_bytes, std::string* err) {
     cudaMemsetAsync(b->d_diag, 0, sizeof(unsigned), b->stream);
     b->h_tmaps.assign(12 * (size_t)capacity, CUtensorMap{});
     b->h_tails.assign(kMaxLev * (size_t)capacity, TailLvl{});
+    // With variant 3, which is not tuned: an index into kMarchShapes, so that
+    // small grids run the shapes of large ones.
+    if (const char* ms = getenv("AEROFLUX_MARCH_SHAPE"))
+        b->force_march = std::min(kMarchShapeCount - 1, std::max(0, atoi(ms)));
     // 0: every wait of the marching pair gives up (how that is reported).
     if (const char* mp = getenv("AEROFLUX_MARCH_POLLS")) b->march_polls = (unsigned)std::min(4096, std::max(0, atoi(mp)));
     // The fused pairs' tile variant for every level (0-2 and 4; 3: marching
