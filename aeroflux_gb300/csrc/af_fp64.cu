@@ -14,7 +14,6 @@
 
 #include <math.h>
 #include <stdio.h>
-#include <stdlib.h>
 
 #include <algorithm>
 #include <cmath>
@@ -1061,27 +1060,12 @@ void launch_split_from_div(const Geom& g, const double* div, const Split& split,
 // the first and the last (the subtraction, which feeds the division unpacked)
 // run there: at 256^3 a launch takes 101 us with none, 86 with either, 77
 // with both -- both pipes then about 70 % busy -- 88 with a third and 140
-// with all six (the logic pipe bounds).  AEROFLUX_RBGS_EMU picks another mask
-// for measurements.
-static int rbgs_emu_mask() {
-    static const int m = [] {
-        const char* v = getenv("AEROFLUX_RBGS_EMU");
-        return v ? atoi(v) : 0x21;
-    }();
-    return m;
-}
+// with all six (the logic pipe bounds).
+constexpr int kRbEmu = 0x21;
 
 void launch_rbgs_fp64(const Split& split, int color, cudaStream_t s) {
     const dim3 grid(cdiv((long long)split.hx * split.NY, 128), split.NZ);
-    void (*k)(const Split, int) = k_rbgs_fp64<0x3F>;
-    switch (rbgs_emu_mask()) {
-    case 0x00: k = k_rbgs_fp64<0x00>; break;
-    case 0x01: k = k_rbgs_fp64<0x01>; break;
-    case 0x20: k = k_rbgs_fp64<0x20>; break;
-    case 0x21: k = k_rbgs_fp64<0x21>; break;
-    case 0x23: k = k_rbgs_fp64<0x23>; break;
-    }
-    launch_pdl(k, grid, dim3(128), 0, s, split, color);
+    launch_pdl(k_rbgs_fp64<kRbEmu>, grid, dim3(128), 0, s, split, color);
 }
 
 // The cluster kernel for this grid, its cells a thread in *nc; null where the
