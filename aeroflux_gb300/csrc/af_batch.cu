@@ -1729,7 +1729,7 @@ __global__ void __launch_bounds__(kMarchT[K], kMarchBlocks[K])
 // shared memory is indexed as such: the chain otherwise waits on instruction
 // fetches and generic loads.  Measured per Step with index decoding, wall
 // tests and block barriers in every sweep / so: 16^3 (a tail alone, 14
-// V-cycles) 0.72 / 0.59 ms, 48x32x64 1.44 / 1.38 ms, 256^3 10.40 / 10.27 ms.
+// V-cycles) 0.72 / 0.59 ms, 48x32x64 1.44 / 1.35 ms, 256^3 10.40 / 10.27 ms.
 constexpr int kWarpSlots = 32;  // at most the lanes of a warp
 // The most dynamic shared memory a tail takes (plan_tail): ghost cells on
 // every side make the thinnest hierarchy, 2 x 2 x 1024 cells, the largest.  The

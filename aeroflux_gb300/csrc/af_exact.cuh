@@ -145,13 +145,14 @@ struct Weights {
 
 // Splits the foot p, already inside the axis, into its cell a0 = trunc(p)
 // and the weights of the taps a0 (o) and a0 + 1 (t); t = 0 for a foot on a
-// face.  lim is the high word of binary64(n - 1), n < 2^20 the axis's extent.
+// face.  lim is the high word of binary64(n - 1), n the axis's padded extent:
+// n - 1 < 2^21, so that the word holds it whole and p's cell has at most 21 bits.
 // False -- nothing decided -- for NaN, p >= n - 1 and p < 2^-11.
 AF_HD bool foot_split(double p, unsigned lim, int* a0, Weights* w) {
     const u64 b = bits_of(p);
     const unsigned hi = (unsigned)(b >> 32);
     if (hi - 0x3FF00000u < lim - 0x3FF00000u) {  // 1 <= p < n - 1
-        const int e = (int)(hi >> 20) - 1023;    // 0 .. 19
+        const int e = (int)(hi >> 20) - 1023;    // 0 .. 20
         const u64 m = significand(b);
         *a0 = (int)((unsigned)(m >> 32) >> (20 - e));
         // t in units of 2^-52 (p >= 1 has no finer bits), so 1 - t is exact.

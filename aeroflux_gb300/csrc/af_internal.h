@@ -1,5 +1,5 @@
 // af_internal.h -- types shared by the engine (af_engine.cu) and the kernels
-// (af_fp64.cu, af_mixed.cu).  Not part of the public ABI.
+// (af_fp64.cu, af_batch.cu).  Not part of the public ABI.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -11,8 +11,8 @@
 namespace af {
 
 // Field geometry on the device: padded extents and strides of grid.go:12-21.
-// Indices inside one field fit in int32 up to ~1280^3; row bases are formed
-// in 64 bits so larger grids stay correct.
+// A field holds fewer than 2^31 elements (af_create and batch_config_fits
+// refuse larger grids), so most kernels index it in int.
 struct Dims {
     int nx, ny, nz;
     long long sy, sz, count;
