@@ -757,8 +757,10 @@ int af_step(af_engine* e, int64_t nsteps) {
         for (const int64_t end = std::min(nsteps, i + chunk); i < end; ++i)
             AF_CUDA(e, cudaGraphLaunch(e->graph[e->parity], e->stream));
         if (i == nsteps) break;
-        AF_CUDA(e, cudaMemcpyAsync(&e->seen[k & 1], e->st, sizeof(Status), cudaMemcpyDeviceToHost, e->stream));
-        AF_CUDA(e, cudaEventRecord(e->seen_ev[k & 1], e->stream));
+        if (nsteps - i > chunk) {  // looked at before the chunk after the next goes out
+            AF_CUDA(e, cudaMemcpyAsync(&e->seen[k & 1], e->st, sizeof(Status), cudaMemcpyDeviceToHost, e->stream));
+            AF_CUDA(e, cudaEventRecord(e->seen_ev[k & 1], e->stream));
+        }
         if (k == 0) continue;
         AF_CUDA(e, cudaEventSynchronize(e->seen_ev[(k - 1) & 1]));
         if (e->seen[(k - 1) & 1].fault_gate != af::kNoFault) break;
